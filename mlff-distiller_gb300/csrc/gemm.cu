@@ -1,0 +1,376 @@
+// FP32 GEMMs on the CUDA cores.
+//
+// They serve what has to stay FP32: the per-op path, the per-block entry
+// points and the weight gradients.  Bound by the FP32 pipes at large row
+// counts (8 x 8 outputs per thread: 4 shared-memory loads per 64 fused
+// multiply-adds) and by the number of tiles at small ones.  The A^T B sums
+// have few output tiles (12 of 64 x 64 for a 384 x 128 gradient) over many
+// rows, so the rows are split until every SM has four blocks; without the
+// split the message block of width 128 on 106,000 edges spent 75 of its
+// 102 ms there and 28 ms in column sums, which now ride along with the tiles
+// of output column 0 (forward + backward 2.9 ms; the width-64 update block on
+// 5,001 atoms 2.33 -> 0.42 ms).  Activations times weights: 64 x 64 tiles of
+// 4 x 4 outputs without load prefetch took 5.10 ms per call of the FP32 path
+// on 37 molecules, these tiles 3.45 ms.
+#include <algorithm>
+#include "gemm.cuh"
+#include "profile.h"
+
+namespace mlff {
+
+namespace {
+
+constexpr int BK = 16;
+
+// One BK-row step of the product: acc += As[k][rows of ty] Bs[k][cols of tx].
+// A thread's TM rows are TM / CM chunks of CM consecutive ones, the chunks
+// BM / (TM / CM) apart (columns alike), so that every fragment is one 8- or
+// 16-byte shared load and a warp's loads fall into different banks.
+template <int BM, int BN, int TM, int TN>
+struct Tile {
+    static constexpr int CM = TM < 4 ? TM : 4, CN = TN < 4 ? TN : 4;
+    static constexpr int RM = TM / CM, RN = TN / CN;
+    static constexpr int NTX = BN / TN, NTY = BM / TM, NT = NTX * NTY;
+    static constexpr int LDA = BM + 4, LDB = BN + 4;
+    static __device__ __forceinline__ int row(int ty, int i) { return (i / CM) * (BM / RM) + ty * CM + i % CM; }
+    static __device__ __forceinline__ int col(int tx, int j) { return (j / CN) * (BN / RN) + tx * CN + j % CN; }
+    template <int C, int R, int SPAN>
+    static __device__ __forceinline__ void frag(const float* s, int t, float* v) {
+#pragma unroll
+        for (int q = 0; q < R; ++q) {
+            const float* p = s + q * SPAN + t * C;
+            if constexpr (C == 4) *reinterpret_cast<float4*>(v + 4 * q) = *reinterpret_cast<const float4*>(p);
+            else if constexpr (C == 2) *reinterpret_cast<float2*>(v + 2 * q) = *reinterpret_cast<const float2*>(p);
+            else v[q] = *p;
+        }
+    }
+    static __device__ __forceinline__ void step(const float* As, const float* Bs, int ty, int tx,
+                                                float (&acc)[TM][TN], float* asum) {
+#pragma unroll 4
+        for (int k = 0; k < BK; ++k) {
+            float a[TM], b[TN];
+            frag<CM, RM, BM / RM>(As + k * LDA, ty, a);
+            frag<CN, RN, BN / RN>(Bs + k * LDB, tx, b);
+#pragma unroll
+            for (int i = 0; i < TM; ++i)
+#pragma unroll
+                for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
+            if (asum) {
+#pragma unroll
+                for (int i = 0; i < TM; ++i) asum[i] += a[i];
+            }
+        }
+    }
+};
+
+__host__ __device__ inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
+
+// (two blocks per SM for 8 x 8 outputs per thread, four for 4 x 4)
+template <int MODE, int BM, int BN, int TM, int TN>
+__global__ void __launch_bounds__(256, TM == 8 ? 2 : 4) gemm_nn_kernel(const float* __restrict__ A, const float* __restrict__ B,
+                                                      const float* __restrict__ bias, float* __restrict__ C,
+                                                      float* __restrict__ C2, const float* __restrict__ Z,
+                                                      int64_t M_static, const int32_t* __restrict__ m_dev, int N,
+                                                      int K, const Status* st) {
+    using T = Tile<BM, BN, TM, TN>;
+    static_assert(T::NT == 256, "256 threads");
+    __shared__ __align__(16) float As[2][BK * T::LDA];
+    __shared__ __align__(16) float Bs[2][BK * T::LDB];
+    if (st->code != 0) return;
+    const int64_t M = m_dev ? (int64_t)(*m_dev) : M_static;
+    const int t = threadIdx.x, tx = t % T::NTX, ty = t / T::NTX;
+    const int n_tiles = (N + BN - 1) / BN;
+    const int64_t m_tiles = (M + BM - 1) / BM;
+    // 16-byte loads and stores need rows that are multiples of 4 floats on a
+    // 16-byte aligned base
+    const bool va = (K & 3) == 0 && aligned16(A), vb = (N & 3) == 0 && aligned16(B);
+    const bool vc = T::CN == 4 && (N & 3) == 0 && aligned16(C) && (MODE != 1 || aligned16(C2)) &&
+                    (MODE != 2 || aligned16(Z));
+    constexpr int LA = BM * BK / 256, LB = BN * BK / 256;   // floats per thread and step
+    static_assert(LA % 4 == 0 || LA == 2, "A loads");
+    for (int64_t tile = blockIdx.x; tile < m_tiles * n_tiles; tile += gridDim.x) {
+        const int64_t m0 = (tile / n_tiles) * BM;
+        const int n0 = (int)(tile % n_tiles) * BN;
+        float acc[TM][TN];
+#pragma unroll
+        for (int i = 0; i < TM; ++i)
+#pragma unroll
+            for (int j = 0; j < TN; ++j) acc[i][j] = 0.f;
+        float ra[LA], rb[LB];
+        auto fetch = [&](int k0) {
+            if (va && LA >= 4) {
+#pragma unroll
+                for (int q = 0; q < LA / 4; ++q) {
+                    const int i = t + 256 * q, r = i / (BK / 4), k = k0 + 4 * (i % (BK / 4));
+                    const float4 x = (m0 + r < M && k < K) ? *reinterpret_cast<const float4*>(A + (m0 + r) * K + k)
+                                                           : make_float4(0.f, 0.f, 0.f, 0.f);
+                    ra[4 * q] = x.x; ra[4 * q + 1] = x.y; ra[4 * q + 2] = x.z; ra[4 * q + 3] = x.w;
+                }
+            } else {
+#pragma unroll
+                for (int q = 0; q < LA; ++q) {
+                    const int i = t + 256 * q, r = i / BK, k = k0 + i % BK;
+                    ra[q] = (m0 + r < M && k < K) ? A[(m0 + r) * K + k] : 0.f;
+                }
+            }
+            if (vb && LB >= 4) {
+#pragma unroll
+                for (int q = 0; q < LB / 4; ++q) {
+                    const int i = t + 256 * q, k = k0 + i / (BN / 4), n = n0 + 4 * (i % (BN / 4));
+                    const float4 x = (k < K && n < N) ? *reinterpret_cast<const float4*>(B + (int64_t)k * N + n)
+                                                      : make_float4(0.f, 0.f, 0.f, 0.f);
+                    rb[4 * q] = x.x; rb[4 * q + 1] = x.y; rb[4 * q + 2] = x.z; rb[4 * q + 3] = x.w;
+                }
+            } else {
+#pragma unroll
+                for (int q = 0; q < LB; ++q) {
+                    const int i = t + 256 * q, k = k0 + i / BN, n = n0 + i % BN;
+                    rb[q] = (k < K && n < N) ? B[(int64_t)k * N + n] : 0.f;
+                }
+            }
+        };
+        auto put = [&](int b) {
+            if (va && LA >= 4) {
+#pragma unroll
+                for (int q = 0; q < LA / 4; ++q) {
+                    const int i = t + 256 * q, r = i / (BK / 4), k = 4 * (i % (BK / 4));
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) As[b][(k + j) * T::LDA + r] = ra[4 * q + j];
+                }
+            } else {
+#pragma unroll
+                for (int q = 0; q < LA; ++q) {
+                    const int i = t + 256 * q;
+                    As[b][(i % BK) * T::LDA + i / BK] = ra[q];
+                }
+            }
+            if (vb && LB >= 4) {
+#pragma unroll
+                for (int q = 0; q < LB / 4; ++q) {
+                    const int i = t + 256 * q;
+                    *reinterpret_cast<float4*>(&Bs[b][(i / (BN / 4)) * T::LDB + 4 * (i % (BN / 4))]) =
+                        make_float4(rb[4 * q], rb[4 * q + 1], rb[4 * q + 2], rb[4 * q + 3]);
+                }
+            } else {
+#pragma unroll
+                for (int q = 0; q < LB; ++q) {
+                    const int i = t + 256 * q;
+                    Bs[b][(i / BN) * T::LDB + i % BN] = rb[q];
+                }
+            }
+        };
+        fetch(0);
+        put(0);
+        __syncthreads();
+        int b = 0;
+        for (int k0 = 0; k0 < K; k0 += BK, b ^= 1) {
+            const bool more = k0 + BK < K;
+            if (more) fetch(k0 + BK);   // in flight during this step's arithmetic
+            T::step(As[b], Bs[b], ty, tx, acc, nullptr);
+            if (more) put(b ^ 1);
+            __syncthreads();
+        }
+#pragma unroll
+        for (int i = 0; i < TM; ++i) {
+            const int64_t gm = m0 + T::row(ty, i);
+            if (gm >= M) continue;
+#pragma unroll
+            for (int j0 = 0; j0 < TN; j0 += T::CN) {
+                const int gn = n0 + T::col(tx, j0);
+                const int64_t idx = gm * N + gn;
+                if (vc && gn < N) {
+                    float v[4];
+#pragma unroll
+                    for (int j = 0; j < T::CN; ++j) v[j] = acc[i][j0 + j];
+                    if (MODE != 2 && bias) {
+#pragma unroll
+                        for (int j = 0; j < T::CN; ++j) v[j] += bias[gn + j];
+                    }
+                    if (MODE == 2) {
+                        const float4 z = *reinterpret_cast<const float4*>(Z + idx);
+                        v[0] *= dsilu_f(z.x); v[1] *= dsilu_f(z.y); v[2] *= dsilu_f(z.z); v[3] *= dsilu_f(z.w);
+                    }
+                    *reinterpret_cast<float4*>(C + idx) = make_float4(v[0], v[1], v[2], v[3]);
+                    if (MODE == 1)
+                        *reinterpret_cast<float4*>(C2 + idx) =
+                            make_float4(silu_f(v[0]), silu_f(v[1]), silu_f(v[2]), silu_f(v[3]));
+                } else {
+#pragma unroll
+                    for (int j = 0; j < T::CN; ++j) {
+                        if (gn + j >= N) continue;
+                        float v = acc[i][j0 + j];
+                        if (MODE != 2 && bias) v += bias[gn + j];
+                        if (MODE == 2) v *= dsilu_f(Z[idx + j]);
+                        C[idx + j] = v;
+                        if (MODE == 1) C2[idx + j] = silu_f(v);
+                    }
+                }
+            }
+        }
+    }
+}
+
+// partial[split][m][n] over the split's rows, partial column sums behind the
+// splits' matrices
+constexpr int TNB = 64;           // output tile 64 x 64, 4 x 4 per thread
+constexpr int TN_MAX_SPLIT = 256;
+constexpr int TN_TARGET_BLOCKS = 152 * 4;
+constexpr int TN_MIN_ROWS = 64;   // rows per split
+
+inline int tn_tiles(int64_t n) { return (int)std::max<int64_t>(1, (n + TNB - 1) / TNB); }
+inline int tn_splits(int64_t M, int64_t N) {
+    const int tiles = tn_tiles(M) * tn_tiles(N);
+    return std::max(1, std::min(TN_MAX_SPLIT, (TN_TARGET_BLOCKS + tiles - 1) / tiles));
+}
+
+__global__ void __launch_bounds__(256, 4) gemm_tn_kernel(const float* __restrict__ A, int lda,
+                                                      const float* __restrict__ B, int ldb, int M, int N,
+                                                      int64_t rows_static, const int32_t* __restrict__ n_dev,
+                                                      int nsplit, int want_sum, float* __restrict__ part,
+                                                      const Status* st) {
+    using T = Tile<TNB, TNB, 4, 4>;
+    __shared__ __align__(16) float As[2][BK * T::LDA];
+    __shared__ __align__(16) float Bs[2][BK * T::LDB];
+    if (st->code != 0) return;
+    const int64_t rows = n_dev ? (int64_t)(*n_dev) : rows_static;
+    const int tiles_n = max(1, (N + TNB - 1) / TNB);
+    const int m0 = (blockIdx.x / tiles_n) * TNB, n0 = (blockIdx.x % tiles_n) * TNB;
+    int64_t per = (rows + nsplit - 1) / nsplit;
+    if (per < TN_MIN_ROWS) per = TN_MIN_ROWS;
+    const int64_t r0 = (int64_t)blockIdx.y * per, r1 = min(rows, r0 + per);
+    const int t = threadIdx.x, tx = t % T::NTX, ty = t / T::NTX;
+    const bool va = (lda & 3) == 0 && (M & 3) == 0 && aligned16(A);
+    const bool vb = (ldb & 3) == 0 && (N & 3) == 0 && aligned16(B);
+    const bool sums = want_sum && n0 == 0;
+    float acc[4][4] = {}, asum[4] = {};
+    float ra[4], rb[4];
+    auto fetch1 = [&](const float* S, int ld, int c0, int ncol, bool vec, int64_t r, float (&v)[4]) {
+        if (vec) {
+            const int c = c0 + 4 * (t % (TNB / 4));
+            const int64_t row = r + t / (TNB / 4);
+            const float4 x = (row < r1 && c < ncol) ? *reinterpret_cast<const float4*>(S + row * ld + c)
+                                                    : make_float4(0.f, 0.f, 0.f, 0.f);
+            v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w;
+        } else {
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const int i = t + 256 * q, c = c0 + i % TNB;
+                const int64_t row = r + i / TNB;
+                v[q] = (row < r1 && c < ncol) ? S[row * ld + c] : 0.f;
+            }
+        }
+    };
+    auto put1 = [&](float* D, int ldd, bool vec, const float (&v)[4]) {
+        if (vec)
+            *reinterpret_cast<float4*>(D + (t / (TNB / 4)) * ldd + 4 * (t % (TNB / 4))) =
+                make_float4(v[0], v[1], v[2], v[3]);
+        else {
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const int i = t + 256 * q;
+                D[(i / TNB) * ldd + i % TNB] = v[q];
+            }
+        }
+    };
+    if (r0 < r1) {
+        fetch1(A, lda, m0, M, va, r0, ra);
+        fetch1(B, ldb, n0, N, vb, r0, rb);
+        put1(As[0], T::LDA, va, ra);
+        put1(Bs[0], T::LDB, vb, rb);
+        __syncthreads();
+        int b = 0;
+        for (int64_t r = r0; r < r1; r += BK, b ^= 1) {
+            const bool more = r + BK < r1;
+            if (more) {
+                fetch1(A, lda, m0, M, va, r + BK, ra);
+                fetch1(B, ldb, n0, N, vb, r + BK, rb);
+            }
+            T::step(As[b], Bs[b], ty, tx, acc, sums ? asum : nullptr);
+            if (more) {
+                put1(As[b ^ 1], T::LDA, va, ra);
+                put1(Bs[b ^ 1], T::LDB, vb, rb);
+            }
+            __syncthreads();
+        }
+    }
+    float* out = part + (int64_t)blockIdx.y * M * N;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int m = m0 + 4 * ty + i;
+        if (m >= M) continue;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int n = n0 + 4 * tx + j;
+            if (n < N) out[(int64_t)m * N + n] = acc[i][j];
+        }
+        if (sums && tx == 0) part[(int64_t)nsplit * M * N + (int64_t)blockIdx.y * M + m] = asum[i];
+    }
+}
+
+// sums over the splits, in split order: four interleaved chains per output
+__global__ void __launch_bounds__(256) gemm_tn_sum_kernel(const float* __restrict__ part, int64_t MN, int M,
+                                                          int nsplit, float* __restrict__ C,
+                                                          float* __restrict__ colsum, const Status* st) {
+    if (st->code != 0) return;
+    const int64_t total = (C ? MN : 0) + (colsum ? M : 0);
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
+        const bool col = !C || i >= MN;
+        const int64_t j = col ? i - (C ? MN : 0) : i;
+        const float* p = col ? part + (int64_t)nsplit * MN + j : part + j;
+        const int64_t stride = col ? M : MN;
+        float s[4] = {0.f, 0.f, 0.f, 0.f};
+        int sp = 0;
+        for (; sp + 4 <= nsplit; sp += 4)
+#pragma unroll
+            for (int q = 0; q < 4; ++q) s[q] += p[(int64_t)(sp + q) * stride];
+        for (; sp < nsplit; ++sp) s[0] += p[(int64_t)sp * stride];
+        (col ? colsum : C)[j] = (s[0] + s[1]) + (s[2] + s[3]);
+    }
+}
+
+template <int BM, int BN, int TM, int TN>
+int launch_nn(int mode, const float* A, const float* B, const float* bias, float* C, float* C2, const float* Z,
+              int64_t M, const int32_t* m_dev, int N, int K, const Status* st, cudaStream_t s, int per_sm) {
+    const int64_t tiles = ((M + BM - 1) / BM) * ((N + BN - 1) / BN);
+    const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>(tiles, (int64_t)num_sms() * per_sm));
+    if (mode == 0) gemm_nn_kernel<0, BM, BN, TM, TN><<<blocks, 256, 0, s>>>(A, B, bias, C, C2, Z, M, m_dev, N, K, st);
+    else if (mode == 1) gemm_nn_kernel<1, BM, BN, TM, TN><<<blocks, 256, 0, s>>>(A, B, bias, C, C2, Z, M, m_dev, N, K, st);
+    else gemm_nn_kernel<2, BM, BN, TM, TN><<<blocks, 256, 0, s>>>(A, B, bias, C, C2, Z, M, m_dev, N, K, st);
+    MLFF_LAUNCH_CHECK("gemm_nn");
+    return MLFF_OK;
+}
+
+}  // namespace
+
+int gemm_nn(int mode, const float* A, const float* B, const float* bias, float* C, float* C2, const float* Z,
+            int64_t M, const int32_t* m_dev, int N, int K, const Status* st, cudaStream_t s) {
+    ProfScope prof(PK_PLAIN_GEMM, s);
+    // The largest tile that still gives every SM two of them: 128 x 128 keeps
+    // the FP32 pipes busiest, small row counts need the tiles more.
+    auto tiles = [&](int bm, int bn) { return ((M + bm - 1) / bm) * ((N + bn - 1) / bn); };
+    const int64_t want = 2LL * num_sms();
+    if (N > 64 && tiles(128, 128) >= want)
+        return launch_nn<128, 128, 8, 8>(mode, A, B, bias, C, C2, Z, M, m_dev, N, K, st, s, 2);
+    if (tiles(64, 64) >= want) return launch_nn<64, 64, 4, 4>(mode, A, B, bias, C, C2, Z, M, m_dev, N, K, st, s, 6);
+    return launch_nn<32, 32, 2, 2>(mode, A, B, bias, C, C2, Z, M, m_dev, N, K, st, s, 8);
+}
+
+size_t gemm_tn_floats(int64_t M, int64_t N) { return (size_t)tn_splits(M, N) * (size_t)(M * N + M); }
+
+int gemm_tn(const float* A, int lda, const float* B, int ldb, int M, int N, int64_t rows, const int32_t* n_dev,
+            float* C, float* colsum, float* part, const Status* st, cudaStream_t s) {
+    ProfScope prof(PK_PLAIN_GEMM, s);
+    int ns = tn_splits(M, N);
+    // (a split holds at least TN_MIN_ROWS rows)
+    ns = (int)std::max<int64_t>(1, std::min<int64_t>(ns, (rows + TN_MIN_ROWS - 1) / TN_MIN_ROWS));
+    dim3 grid(tn_tiles(M) * tn_tiles(N), ns);
+    gemm_tn_kernel<<<grid, 256, 0, s>>>(A, lda, B, ldb, M, N, rows, n_dev, ns, colsum != nullptr, part, st);
+    MLFF_LAUNCH_CHECK("gemm_tn");
+    const int64_t out = (int64_t)M * N + M;
+    gemm_tn_sum_kernel<<<(int)std::min<int64_t>((out + 255) / 256, 152 * 8), 256, 0, s>>>(part, (int64_t)M * N, M, ns, C,
+                                                                                     colsum, st);
+    MLFF_LAUNCH_CHECK("gemm_tn_sum");
+    return MLFF_OK;
+}
+
+}  // namespace mlff

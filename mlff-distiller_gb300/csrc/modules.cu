@@ -6,21 +6,26 @@
 // These serve callers that use the blocks outside StudentForceField (the
 // reference's unit tests build a PaiNNInteraction of width 64 and call it
 // directly).  They follow the reference's per-op graph in FP32 -- filter
-// GEMMs on the plain path's SGEMM, messages scattered with float atomics as
+// GEMMs in FP32 (gemm.cu), messages scattered with float atomics as
 // index_add_ does on a GPU -- and are not the fused hot path.  Edge indices
 // come from the caller: an out-of-range index is reported through the
 // status word (MLFF_ERR_INVALID, the edge's position) and every later kernel
 // of the call returns without work, so nothing is read or written out of
 // bounds (the outputs then hold the residual copies only).
+#include <algorithm>
 #include "common.cuh"
+#include "gemm.cuh"
 #include "workspace.h"
 
 namespace mlff {
 
-int plain_sgemm(int mode, const float* A, const float* B, const float* bias, float* C, float* C2, const float* Z,
-                int64_t M, int N, int K, const Status* st, cudaStream_t s);
-
 namespace {
+
+int plain_sgemm(int mode, const float* A, const float* B, const float* bias, float* C, float* C2, const float* Z,
+                int64_t M, int N, int K, const Status* st, cudaStream_t s) {
+    return gemm_nn(mode, A, B, bias, C, C2, Z, M, nullptr, N, K, st, s);
+}
+
 
 constexpr int MOD_BLOCKS_MAX = 152 * 8;
 
@@ -49,19 +54,21 @@ inline ModLayout mod_layout(const int64_t* sizes, int n) {
 }
 
 // message workspace: w1t [R][H], w2t [H][3H], z, h [E][H], f [E][3H];
-// reverse pass: gf [E][3H], gz [E][H], gfT [3H][E], gzT [H][E]
+// reverse pass: gf [E][3H], gz [E][H], scratch of the weight-gradient sums
 inline ModLayout msg_layout(int64_t H, int64_t R, int64_t E, bool bwd) {
-    const int64_t s[9] = {R * H, H * 3 * H, E * H, E * H, E * 3 * H, E * 3 * H, E * H, 3 * H * E, H * E};
-    return mod_layout(s, bwd ? 9 : 5);
+    const int64_t part = (int64_t)std::max(gemm_tn_floats(3 * H, H), gemm_tn_floats(H, R));
+    const int64_t s[8] = {R * H, H * 3 * H, E * H, E * H, E * 3 * H, E * 3 * H, E * H, part};
+    return mod_layout(s, bwd ? 8 : 5);
 }
 // update workspace: u1t [2H][H], u2t [H][3H], comb [N][2H], z, h [N][H],
-// a [N][3H]; reverse pass: ga [N][3H], gz [N][H], gcomb [N][2H], gaT [3H][N],
-// gzT [H][N], gmix [MIX_BLOCKS][9]
+// a [N][3H]; reverse pass: ga [N][3H], gz [N][H], gcomb [N][2H], scratch of
+// the weight-gradient sums, gmix [MIX_BLOCKS][9]
 constexpr int MIX_BLOCKS = 256;
 inline ModLayout upd_layout(int64_t H, int64_t N, bool bwd) {
-    const int64_t s[12] = {2 * H * H, H * 3 * H, N * 2 * H, N * H, N * H, N * 3 * H,
-                           N * 3 * H, N * H, N * 2 * H, 3 * H * N, H * N, MIX_BLOCKS * 9};
-    return mod_layout(s, bwd ? 12 : 6);
+    const int64_t part = (int64_t)std::max(gemm_tn_floats(3 * H, H), gemm_tn_floats(H, 2 * H));
+    const int64_t s[11] = {2 * H * H, H * 3 * H, N * 2 * H, N * H, N * H, N * 3 * H,
+                           N * 3 * H, N * H, N * 2 * H, part, MIX_BLOCKS * 9};
+    return mod_layout(s, bwd ? 11 : 6);
 }
 
 template <typename T>
@@ -80,17 +87,6 @@ __global__ void mod_transpose_kernel(const float* __restrict__ in, float* __rest
     }
 }
 
-// sums over rows: out[c] = sum_r in[r][c] (fixed order)
-__global__ void mod_colsum_kernel(const float* __restrict__ in, float* __restrict__ out, int64_t rows, int cols,
-                                  const Status* st) {
-    if (st->code != 0) return;
-    for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < cols; c += gridDim.x * blockDim.x) {
-        float s = 0.f;
-        for (int64_t r = 0; r < rows; ++r) s += in[r * cols + c];
-        out[c] = s;
-    }
-}
-
 __global__ void mod_check_edges_kernel(const int64_t* __restrict__ ei, int64_t E, int32_t N, Status* st) {
     for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < E; e += (int64_t)gridDim.x * blockDim.x) {
         const int64_t s = ei[e], d = ei[E + e];
@@ -98,73 +94,128 @@ __global__ void mod_check_edges_kernel(const int64_t* __restrict__ ei, int64_t E
     }
 }
 
-// scalar_out[dst] += s[src] * phi_s;  vector_out[dst][i] += v[src][i] * phi_v1
-// + u[i] * phi_v2   (index_add_, student_model.py:359-385), thread per (edge, channel)
-__global__ void msg_scatter_kernel(const float* __restrict__ s, const float* __restrict__ v,
-                                   const int64_t* __restrict__ ei, const float* __restrict__ evec,
-                                   const float* __restrict__ f, int64_t E, int H, float* __restrict__ s_out,
-                                   float* __restrict__ v_out, const Status* st) {
-    if (st->code != 0) return;
-    const int64_t n = E * H;
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t e = i / H;
-        const int k = (int)(i % H);
-        const int64_t b = ei[e], a = ei[E + e];
-        const float* fe = f + e * 3 * H;
-        const float fs = fe[k], f1 = fe[H + k], f2 = fe[2 * H + k];
-        atomicAdd(s_out + a * H + k, s[b * H + k] * fs);
-#pragma unroll
-        for (int q = 0; q < 3; ++q)
-            atomicAdd(v_out + (a * 3 + q) * H + k, v[(b * 3 + q) * H + k] * f1 + evec[e * 3 + q] * f2);
+// V consecutive floats of a row: one 16-byte access and one 16-byte atomic
+// when the rows allow it (V = 4: H a multiple of 4, every base 16-byte
+// aligned), single floats otherwise.
+template <int V>
+struct Vec;
+template <>
+struct Vec<1> {
+    float x[1];
+    static __device__ __forceinline__ Vec load(const float* p) { return {{*p}}; }
+    __device__ __forceinline__ void store(float* p) const { *p = x[0]; }
+    __device__ __forceinline__ void add_to(float* p) const { atomicAdd(p, x[0]); }
+};
+template <>
+struct Vec<4> {
+    float x[4];
+    static __device__ __forceinline__ Vec load(const float* p) {
+        const float4 v = *reinterpret_cast<const float4*>(p);
+        return {{v.x, v.y, v.z, v.w}};
     }
-}
+    __device__ __forceinline__ void store(float* p) const {
+        *reinterpret_cast<float4*>(p) = make_float4(x[0], x[1], x[2], x[3]);
+    }
+    __device__ __forceinline__ void add_to(float* p) const {
+        atomicAdd(reinterpret_cast<float4*>(p), make_float4(x[0], x[1], x[2], x[3]));
+    }
+};
 
-// reverse of the scatter: filter adjoint gf [E][3H], and the gathered
-// adjoints of the sender features (grad_s, grad_v hold the residual part)
-__global__ void msg_scatter_bwd_kernel(const float* __restrict__ s, const float* __restrict__ v,
-                                       const int64_t* __restrict__ ei, const float* __restrict__ evec,
-                                       const float* __restrict__ f, const float* __restrict__ gs,
-                                       const float* __restrict__ gv, int64_t E, int H, float* __restrict__ gf,
-                                       float* __restrict__ grad_s, float* __restrict__ grad_v, const Status* st) {
+// scalar_out[dst] += s[src] * phi_s;  vector_out[dst][i] += v[src][i] * phi_v1
+// + u[i] * phi_v2   (index_add_, student_model.py:359-385), thread per (edge,
+// V channels).  Bound by the atomics: 16-byte ones issue a quarter as many.
+template <int V>
+__global__ void __launch_bounds__(256) msg_scatter_kernel(const float* __restrict__ s, const float* __restrict__ v,
+                                                          const int64_t* __restrict__ ei,
+                                                          const float* __restrict__ evec, const float* __restrict__ f,
+                                                          int64_t E, int H, float* __restrict__ s_out,
+                                                          float* __restrict__ v_out, const Status* st) {
     if (st->code != 0) return;
-    const int64_t n = E * H;
+    using W = Vec<V>;
+    const int per = H / V;
+    const int64_t n = E * per;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t e = i / H;
-        const int k = (int)(i % H);
+        const int64_t e = i / per;
+        const int k = (int)(i % per) * V;
         const int64_t b = ei[e], a = ei[E + e];
-        const float* fe = f + e * 3 * H;
-        const float gsa = gs[a * H + k];
-        float g1 = 0.f, g2 = 0.f;
+        const float* fe = f + e * 3 * H + k;
+        const W fs = W::load(fe), f1 = W::load(fe + H), f2 = W::load(fe + 2 * H);
+        W m = W::load(s + b * H + k);
+#pragma unroll
+        for (int j = 0; j < V; ++j) m.x[j] *= fs.x[j];
+        m.add_to(s_out + a * H + k);
 #pragma unroll
         for (int q = 0; q < 3; ++q) {
-            const float gva = gv[(a * 3 + q) * H + k];
-            g1 = fmaf(gva, v[(b * 3 + q) * H + k], g1);
-            g2 = fmaf(gva, evec[e * 3 + q], g2);
-            atomicAdd(grad_v + (b * 3 + q) * H + k, gva * fe[H + k]);
+            W x = W::load(v + (b * 3 + q) * H + k);
+            const float u = evec[e * 3 + q];
+#pragma unroll
+            for (int j = 0; j < V; ++j) x.x[j] = x.x[j] * f1.x[j] + u * f2.x[j];
+            x.add_to(v_out + (a * 3 + q) * H + k);
         }
-        float* g = gf + e * 3 * H;
-        g[k] = gsa * s[b * H + k];
-        g[H + k] = g1;
-        g[2 * H + k] = g2;
-        atomicAdd(grad_s + b * H + k, gsa * fe[k]);
     }
 }
 
-// grad_u[e][q] = sum_k gv[dst][q][k] phi_v2[e][k]
-__global__ void msg_evec_bwd_kernel(const int64_t* __restrict__ ei, const float* __restrict__ f,
-                                    const float* __restrict__ gv, int64_t E, int H, float* __restrict__ gu,
-                                    const Status* st) {
+// reverse of the scatter: filter adjoint gf [E][3H], the gathered adjoints
+// of the sender features (grad_s, grad_v hold the residual part) and
+// grad_u[e][q] = sum_k gv[dst][q][k] phi_v2[e][k].  One warp per edge, V
+// channels per lane and turn, so the channel sums stay in the warp and every
+// row is read once.
+template <int V>
+__global__ void __launch_bounds__(256) msg_scatter_bwd_kernel(
+    const float* __restrict__ s, const float* __restrict__ v, const int64_t* __restrict__ ei,
+    const float* __restrict__ evec, const float* __restrict__ f, const float* __restrict__ gs,
+    const float* __restrict__ gv, int64_t E, int H, float* __restrict__ gf, float* __restrict__ grad_s,
+    float* __restrict__ grad_v, float* __restrict__ gu, const Status* st) {
     if (st->code != 0) return;
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < E * 3; i += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t e = i / 3;
-        const int q = (int)(i % 3);
-        const int64_t a = ei[E + e];
-        const float* f2 = f + e * 3 * H + 2 * H;
-        const float* g = gv + (a * 3 + q) * H;
-        float acc = 0.f;
-        for (int k = 0; k < H; ++k) acc = fmaf(g[k], f2[k], acc);
-        gu[i] = acc;
+    using W = Vec<V>;
+    const int lane = threadIdx.x & 31;
+    const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
+    for (int64_t e = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; e < E; e += nw) {
+        const int64_t b = ei[e], a = ei[E + e];
+        const float u[3] = {evec[e * 3], evec[e * 3 + 1], evec[e * 3 + 2]};
+        float du[3] = {0.f, 0.f, 0.f};
+        for (int k = lane * V; k < H; k += 32 * V) {
+            const float* fe = f + e * 3 * H + k;
+            const W fs = W::load(fe), f1 = W::load(fe + H), f2 = W::load(fe + 2 * H);
+            const W ga = W::load(gs + a * H + k), sb = W::load(s + b * H + k);
+            W t0, t1, g1{}, g2{};
+#pragma unroll
+            for (int j = 0; j < V; ++j) {
+                t0.x[j] = ga.x[j] * sb.x[j];
+                t1.x[j] = ga.x[j] * fs.x[j];
+            }
+            float* g = gf + e * 3 * H + k;
+            t0.store(g);
+            t1.add_to(grad_s + b * H + k);
+#pragma unroll
+            for (int q = 0; q < 3; ++q) {
+                const W gva = W::load(gv + (a * 3 + q) * H + k), vb = W::load(v + (b * 3 + q) * H + k);
+                W d;
+#pragma unroll
+                for (int j = 0; j < V; ++j) {
+                    g1.x[j] = fmaf(gva.x[j], vb.x[j], g1.x[j]);
+                    g2.x[j] = fmaf(gva.x[j], u[q], g2.x[j]);
+                    d.x[j] = gva.x[j] * f1.x[j];
+                    du[q] = fmaf(gva.x[j], f2.x[j], du[q]);
+                }
+                d.add_to(grad_v + (b * 3 + q) * H + k);
+            }
+            g1.store(g + H);
+            g2.store(g + 2 * H);
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+            for (int q = 0; q < 3; ++q) du[q] += __shfl_xor_sync(0xffffffffu, du[q], o);
+        if (lane < 3) gu[e * 3 + lane] = lane == 0 ? du[0] : lane == 1 ? du[1] : du[2];
     }
+}
+
+inline bool rows16(int64_t H, std::initializer_list<const void*> ps) {
+    if (H % 4) return false;
+    for (const void* p : ps)
+        if (reinterpret_cast<uintptr_t>(p) & 15) return false;
+    return true;
 }
 
 // comb = [s, |v|] (norm over xyz, student_model.py:437-440)
@@ -360,8 +411,12 @@ int mlff_painn_message(int32_t hidden, int32_t n_rbf, int32_t n_atoms, int64_t n
         // filter = Linear(R, H) - SiLU - Linear(H, 3H)  (:318-322, :350)
         if ((r = plain_sgemm(1, edge_rbf, w1t, b1, z, h, nullptr, E, (int)H, (int)R, sw, st))) return r;
         if ((r = plain_sgemm(0, h, w2t, b2, f, nullptr, nullptr, E, (int)(3 * H), (int)H, sw, st))) return r;
-        MOD_LAUNCH(msg_scatter_kernel, E * H, st, scalar, vector, edge_index, edge_vector, f, E, (int)H, scalar_out,
-                   vector_out, sw);
+        if (rows16(H, {scalar, vector, scalar_out, vector_out}))
+            MOD_LAUNCH(msg_scatter_kernel<4>, E * H / 4, st, scalar, vector, edge_index, edge_vector, f, E, (int)H,
+                       scalar_out, vector_out, sw);
+        else
+            MOD_LAUNCH(msg_scatter_kernel<1>, E * H, st, scalar, vector, edge_index, edge_vector, f, E, (int)H,
+                       scalar_out, vector_out, sw);
     }
     MLFF_CUDA(cudaMemcpyAsync(status, sw, 4 * sizeof(int32_t), cudaMemcpyDeviceToDevice, st));
     return MLFF_OK;
@@ -405,7 +460,7 @@ int mlff_painn_message_backward(int32_t hidden, int32_t n_rbf, int32_t n_atoms, 
     float *w1t = at<float>(workspace, L.a[0]), *w2t = at<float>(workspace, L.a[1]);
     float *z = at<float>(workspace, L.a[2]), *h = at<float>(workspace, L.a[3]), *f = at<float>(workspace, L.a[4]);
     float *gf = at<float>(workspace, L.a[5]), *gz = at<float>(workspace, L.a[6]);
-    float *gfT = at<float>(workspace, L.a[7]), *gzT = at<float>(workspace, L.a[8]);
+    float* part = at<float>(workspace, L.a[7]);
     MOD_LAUNCH(mod_check_edges_kernel, E, st, edge_index, E, n_atoms, sw);
     // the filter of the forward pass, recomputed (no activation is kept between the calls)
     MOD_LAUNCH(mod_transpose_kernel, H * R, st, w1, w1t, H, R, sw);
@@ -413,19 +468,20 @@ int mlff_painn_message_backward(int32_t hidden, int32_t n_rbf, int32_t n_atoms, 
     if ((r = plain_sgemm(1, edge_rbf, w1t, b1, z, h, nullptr, E, (int)H, (int)R, sw, st))) return r;
     if ((r = plain_sgemm(0, h, w2t, b2, f, nullptr, nullptr, E, (int)(3 * H), (int)H, sw, st))) return r;
     // filter adjoint and the gathered feature adjoints; unit-vector adjoint
-    MOD_LAUNCH(msg_scatter_bwd_kernel, E * H, st, scalar, vector, edge_index, edge_vector, f, grad_scalar_out,
-               grad_vector_out, E, (int)H, gf, grad_scalar, grad_vector, sw);
-    MOD_LAUNCH(msg_evec_bwd_kernel, E * 3, st, edge_index, f, grad_vector_out, E, (int)H, grad_edge_vector, sw);
+    if (rows16(H, {scalar, vector, grad_scalar_out, grad_vector_out, grad_scalar, grad_vector}))
+        MOD_LAUNCH(msg_scatter_bwd_kernel<4>, E * 32, st, scalar, vector, edge_index, edge_vector, f, grad_scalar_out,
+                   grad_vector_out, E, (int)H, gf, grad_scalar, grad_vector, grad_edge_vector, sw);
+    else
+        MOD_LAUNCH(msg_scatter_bwd_kernel<1>, E * 32, st, scalar, vector, edge_index, edge_vector, f, grad_scalar_out,
+                   grad_vector_out, E, (int)H, gf, grad_scalar, grad_vector, grad_edge_vector, sw);
     // through the filter MLP: gz = (gf W2) silu'(z), grad_rbf = gz W1
     if ((r = plain_sgemm(2, gf, w2, nullptr, gz, nullptr, z, E, (int)H, (int)(3 * H), sw, st))) return r;
     if ((r = plain_sgemm(0, gz, w1, nullptr, grad_rbf, nullptr, nullptr, E, (int)R, (int)H, sw, st))) return r;
     // parameter gradients: W2 = gf^T h, W1 = gz^T rbf, biases = column sums
-    MOD_LAUNCH(mod_transpose_kernel, E * 3 * H, st, gf, gfT, E, 3 * H, sw);
-    MOD_LAUNCH(mod_transpose_kernel, E * H, st, gz, gzT, E, H, sw);
-    if ((r = plain_sgemm(0, gfT, h, nullptr, grad_w2, nullptr, nullptr, 3 * H, (int)H, (int)E, sw, st))) return r;
-    if ((r = plain_sgemm(0, gzT, edge_rbf, nullptr, grad_w1, nullptr, nullptr, H, (int)R, (int)E, sw, st))) return r;
-    MOD_LAUNCH(mod_colsum_kernel, 3 * H, st, gf, grad_b2, E, (int)(3 * H), sw);
-    MOD_LAUNCH(mod_colsum_kernel, H, st, gz, grad_b1, E, (int)H, sw);
+    if ((r = gemm_tn(gf, (int)(3 * H), h, (int)H, (int)(3 * H), (int)H, E, nullptr, grad_w2, grad_b2, part, sw, st)))
+        return r;
+    if ((r = gemm_tn(gz, (int)H, edge_rbf, (int)R, (int)H, (int)R, E, nullptr, grad_w1, grad_b1, part, sw, st)))
+        return r;
     MLFF_CUDA(cudaMemcpyAsync(status, sw, 4 * sizeof(int32_t), cudaMemcpyDeviceToDevice, st));
     return MLFF_OK;
 }
@@ -494,8 +550,8 @@ int mlff_painn_update_backward(int32_t hidden, int32_t n_atoms, const float* sca
     float *comb = at<float>(workspace, L.a[2]), *z = at<float>(workspace, L.a[3]);
     float *h = at<float>(workspace, L.a[4]), *a = at<float>(workspace, L.a[5]);
     float *ga = at<float>(workspace, L.a[6]), *gz = at<float>(workspace, L.a[7]);
-    float *gcomb = at<float>(workspace, L.a[8]), *gaT = at<float>(workspace, L.a[9]);
-    float *gzT = at<float>(workspace, L.a[10]), *gmix = at<float>(workspace, L.a[11]);
+    float *gcomb = at<float>(workspace, L.a[8]), *part = at<float>(workspace, L.a[9]);
+    float* gmix = at<float>(workspace, L.a[10]);
     // the forward pass, recomputed
     MOD_LAUNCH(mod_transpose_kernel, 2 * H * H, st, w1, u1t, H, 2 * H, sw);
     MOD_LAUNCH(mod_transpose_kernel, 3 * H * H, st, w2, u2t, 3 * H, H, sw);
@@ -513,12 +569,10 @@ int mlff_painn_update_backward(int32_t hidden, int32_t n_atoms, const float* sca
     if ((r = plain_sgemm(0, gz, w1, nullptr, gcomb, nullptr, nullptr, N, (int)(2 * H), (int)H, sw, st))) return r;
     MOD_LAUNCH(upd_comb_bwd_kernel, N * H, st, vector, comb, gcomb, N, (int)H, grad_scalar, grad_vector, sw);
     // parameter gradients
-    MOD_LAUNCH(mod_transpose_kernel, N * 3 * H, st, ga, gaT, N, 3 * H, sw);
-    MOD_LAUNCH(mod_transpose_kernel, N * H, st, gz, gzT, N, H, sw);
-    if ((r = plain_sgemm(0, gaT, h, nullptr, grad_w2, nullptr, nullptr, 3 * H, (int)H, (int)N, sw, st))) return r;
-    if ((r = plain_sgemm(0, gzT, comb, nullptr, grad_w1, nullptr, nullptr, H, (int)(2 * H), (int)N, sw, st))) return r;
-    MOD_LAUNCH(mod_colsum_kernel, 3 * H, st, ga, grad_b2, N, (int)(3 * H), sw);
-    MOD_LAUNCH(mod_colsum_kernel, H, st, gz, grad_b1, N, (int)H, sw);
+    if ((r = gemm_tn(ga, (int)(3 * H), h, (int)H, (int)(3 * H), (int)H, N, nullptr, grad_w2, grad_b2, part, sw, st)))
+        return r;
+    if ((r = gemm_tn(gz, (int)H, comb, (int)(2 * H), (int)H, (int)(2 * H), N, nullptr, grad_w1, grad_b1, part, sw, st)))
+        return r;
     return MLFF_OK;
 }
 

@@ -11,6 +11,7 @@
 // derivative along a direction G of the atom positions.
 #include "common.cuh"
 #include "dual.cuh"
+#include "gemm.cuh"
 #include "workspace.h"
 #include "profile.h"
 
@@ -166,6 +167,7 @@ __global__ void __launch_bounds__(256) sgemm_kernel(const T* __restrict__ A, con
 template <int MODE, class T>
 static int sgemm(const T* A, const float* B, const float* bias, T* C, T* C2, const T* Z,
                  int64_t M, const int32_t* m_dev, int N, int K, const Status* st, cudaStream_t s) {
+    if constexpr (!is_dual_v<T>) return gemm_nn(MODE, A, B, bias, C, C2, Z, M, m_dev, N, K, st, s);
     const int64_t tiles = ((M + SG_BM - 1) / SG_BM) * ((N + SG_BN - 1) / SG_BN);
     const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>(tiles, 152 * 8));
     ProfScope prof(PK_PLAIN_GEMM, s);
@@ -608,16 +610,6 @@ static int run_plain_t(const mlff_dims& d, const float* P, const PackedOffsets& 
     if constexpr (DUAL) return MLFF_OK;
     if (!out.forces && !out.virial) return MLFF_OK;
     return launch_forces(d, sys, L, ws, out, st, vf);
-}
-
-// Float32 C[M][N] = A[M][K] B[K][N] (+ bias) for the per-module entry points
-// (modules.cu): mode 0 C = acc + bias; 1 also C2 = silu(C); 2 C = acc *
-// silu'(Z).
-int plain_sgemm(int mode, const float* A, const float* B, const float* bias, float* C, float* C2, const float* Z,
-                int64_t M, int N, int K, const Status* st, cudaStream_t s) {
-    if (mode == 0) return sgemm<0, float>(A, B, bias, C, C2, Z, M, nullptr, N, K, st, s);
-    if (mode == 1) return sgemm<1, float>(A, B, bias, C, C2, Z, M, nullptr, N, K, st, s);
-    return sgemm<2, float>(A, B, bias, C, C2, Z, M, nullptr, N, K, st, s);
 }
 
 int run_plain(const mlff_dims& d, const float* P, const PackedOffsets& po, const mlff_system& sys,
