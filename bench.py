@@ -16,9 +16,11 @@ Beside the headline the line carries, measured in the same run:
     paths timed the same way (CUDA-graph replays of one step, L2 flushed);
   * ``accuracy``: energy and force errors of the timed path against the
     float64 oracle (a checker, run after the timed regions);
-  * ``roofline``: the dominant kernel's algorithmic filter-MLP FLOPs over its
-    CUDA-event launch time against the measured bf16 burst peak, and the
-    whole step's GEMM FLOPs over the step time.
+  * ``roofline``: the dominant kernel's work over its CUDA-event launch time
+    against the measured peak -- filter-MLP FLOPs against the bf16 burst for a
+    network-evaluating edge kernel, compulsory bytes against the HBM copy for
+    the tabulated reverse kernel -- and the whole step's GEMM FLOPs (as if
+    every filter were evaluated by its network) over the step time.
 
   python bench.py [--gpus N --steps K --warmup W] [--workload batch256]
                   [--path fp16x3|tuned_fp32|fp32] [--impl ours|reference]
@@ -440,7 +442,7 @@ def graph_step(model, sysm, warmup):
     batch = make_batch(sysm.Z, sysm.pos, sysm.mol_ptr, sysm.box if sysm.pbc.any() else None,
                        sysm.pbc if sysm.pbc.any() else None)
     eng.energy_forces(batch, model.path, graph=False)
-    if model.path == _lib.PATH_TUNED_TC:
+    if model.path in (_lib.PATH_TUNED_TC, _lib.PATH_TABLE):
         eng.autotune(batch, model.path)
     _, n_edges, _ = eng.status()
     step, E, F = eng.capture(batch, model.path)
@@ -503,7 +505,7 @@ def main():
     batch = make_batch(sysm.Z, sysm.pos, sysm.mol_ptr, sysm.box if sysm.pbc.any() else None,
                        sysm.pbc if sysm.pbc.any() else None)
     eng.energy_forces(batch, path, graph=False)   # sizes the edge capacity, checks status
-    tune = eng.autotune(batch, path) if path == _lib.PATH_TUNED_TC else None
+    tune = eng.autotune(batch, path) if path in (_lib.PATH_TUNED_TC, _lib.PATH_TABLE) else None
     _, n_edges, _ = eng.status()
     flush = torch.empty(L2_FLUSH_BYTES // 4, dtype=torch.float32, device="cuda")
     for _ in range(max(3, args.warmup)):
@@ -564,23 +566,34 @@ def main():
     launches = prof.launches[dom]
     avg_ms = prof.ms[dom] / max(1, launches)
     peak_tf, hbm, peak_src = measured_peaks()
+    table_reverse = path == _lib.PATH_TABLE and dom == "edge_bwd"
     if dom == "edge_fwd":
         flop = n_edges * GEMM_FLOP_PER_EDGE
-    elif dom == "edge_bwd":
+    elif dom == "edge_bwd" and not table_reverse:
         flop = 2 * n_edges * GEMM_FLOP_PER_EDGE
     else:
         flop = None
     step_flop = step_gemm_flop(sysm.n_atoms, n_edges, L)
     step_tf = step_flop / (ms_per_step * 1e-3) / 1e12
     roof = None
-    if flop is not None:
+    if table_reverse:
+        # the reverse edge kernel reads tabulated filters: per edge its record and the four
+        # channel slices' (dE/dd, dE/du) read and written, per atom three rows of 2 KB
+        nbytes = n_edges * (32 + 2 * 4 * 16) + sysm.n_atoms * 3 * 2048
+        ach = nbytes / (avg_ms * 1e-3) / 1e9
+        roof = {"bound": "issue", "kernel": dom, "achieved": round(ach, 1), "peak": hbm, "unit": "GB/s",
+                "frac": round(ach / hbm, 4), "peak_source": f"{peak_src} HBM copy",
+                "avg_launch_ms": round(avg_ms, 4), "launches_per_step": launches / args.steps,
+                "bytes_per_launch": nbytes,
+                "step": {"gemm_flop_per_step_untabulated": step_flop, "achieved": round(step_tf, 2)}}
+    elif flop is not None:
         ach = flop / (avg_ms * 1e-3) / 1e12
         roof = {"bound": "tensor", "kernel": dom, "achieved": round(ach, 2), "peak": peak_tf, "unit": "TFLOP/s",
                 "frac": round(ach / peak_tf, 4), "peak_source": f"{peak_src} bf16 burst",
                 "traffic": read_traffic(dom, args.workload), "avg_launch_ms": round(avg_ms, 4),
                 "launches_per_step": launches / args.steps, "flop_per_launch": flop,
                 "mma_work_factor": (3.0 * (2 * (32 * 128 + 128 * 384)) / GEMM_FLOP_PER_EDGE
-                                    if path == _lib.PATH_TUNED_TC else None),
+                                    if path in (_lib.PATH_TUNED_TC, _lib.PATH_TABLE) else None),
                 "step": {"gemm_flop_per_step": step_flop, "achieved": round(step_tf, 2),
                          "frac": round(step_tf / peak_tf, 4)}}
         if dom == "edge_bwd" and prof.launches.get("edge_bwd_q", 0) > 0:

@@ -49,6 +49,13 @@ typedef struct CUstream_st *mlff_stream_t; /* same type as cudaStream_t */
 #define MLFF_PATH_TUNED_FP32 2    /* fused edge kernels, FP32 CUDA cores */
 #define MLFF_PATH_TRAIN 3         /* plain FP32 path plus parameter gradients (workspace sizing) */
 #define MLFF_PATH_TRAIN_FORCES 4  /* plus the force-loss term (workspace sizing; runs as path 0) */
+/* The fused paths with tabulated filters: the edge filter of a layer is a
+ * function of the distance alone, evaluated in FP32 from the piecewise
+ * polynomials that mlff_pack_weights builds.  A call whose weights' tables
+ * miss the path's accuracy class ends with MLFF_ERR_UNSUPPORTED in the status
+ * word; mlff_filter_table_class tells beforehand. */
+#define MLFF_PATH_TABLE 5         /* path 1's forward pass, reverse pass from the tables (class 1 or 2) */
+#define MLFF_PATH_TABLE_FP32 6    /* path 2 from the tables, both passes (class 2) */
 
 #define MLFF_MAX_LAYERS 8
 
@@ -138,6 +145,12 @@ size_t mlff_packed_weights_size(const mlff_dims *dims);
  * StudentForceField.load / load_state_dict (student_model.py:1101-1176). */
 int mlff_pack_weights(const mlff_dims *dims, const mlff_params *params, void *packed,
                       size_t packed_bytes, mlff_stream_t stream);
+
+/* Accuracy class of the filter tables in a packed blob: 0 not usable (the
+ * radial functions are sharper than the table resolves: use paths 1 and 2),
+ * 1 path 5, 2 paths 5 and 6.  Synchronises the stream.  accuracy: host. */
+int mlff_filter_table_class(const mlff_dims *dims, const void *packed, int32_t *accuracy,
+                            mlff_stream_t stream);
 
 /* Workspace bytes for a batch of n_atoms atoms in n_mol structures with
  * room for edge_capacity directed edges, for the given path. */

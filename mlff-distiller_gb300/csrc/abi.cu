@@ -11,6 +11,7 @@
 #include <tuple>
 #include <atomic>
 #include "common.cuh"
+#include "tab.cuh"
 #include "workspace.h"
 
 namespace mlff {
@@ -49,13 +50,16 @@ int num_sms() {
     return sms;
 }
 
+// paths that run the tensor-core edge kernels (the table path: forward only)
+static bool has_tc_edges(int32_t path) { return path == MLFF_PATH_TUNED_TC || path == MLFF_PATH_TABLE; }
+
 int persistent_ctas(int32_t path) {
     // Receiver partitions: the CUDA-core fused kernels run 4 CTAs of 128
     // threads per SM; the tensor-core kernels run one CTA per SM with two
     // partitions each (the reverse kernel's two pipelines take one each,
     // the forward kernel walks both as one receiver range), times the
     // partition factor the autotuner chose for the call's size.
-    return path == MLFF_PATH_TUNED_TC ? 2 * num_sms() : num_sms() * 4;
+    return has_tc_edges(path) ? 2 * num_sms() : num_sms() * 4;
 }
 
 // ----------------------------------------------------------- autotuning
@@ -93,7 +97,7 @@ std::tuple<int, int, int> tune_key(int32_t path, int32_t n_atoms, int32_t n_mol)
 }  // namespace
 
 TunedShape tuned_shape(int32_t path, int32_t n_atoms, int32_t n_mol) {
-    if (path != MLFF_PATH_TUNED_TC) return DEFAULT_SHAPE;
+    if (!has_tc_edges(path)) return DEFAULT_SHAPE;
     if (g_tune_override.factor) return g_tune_override;
     std::lock_guard<std::mutex> lk(g_tune_mu);
     auto it = g_tune.find(tune_key(path, n_atoms, n_mol));
@@ -105,11 +109,15 @@ WsLayout ws_layout(const mlff_dims& d, int32_t n_atoms, int32_t n_mol, int64_t c
     L.N = n_atoms;
     L.B = n_mol;
     L.L = d.n_layers;
+    const bool tc = has_tc_edges(path);
+    const bool table = path == MLFF_PATH_TABLE || path == MLFF_PATH_TABLE_FP32;
     // arrays sized for the largest partition factor, so that tuning never changes the size
-    const int64_t P_max = (int64_t)persistent_ctas(path) * (path == MLFF_PATH_TUNED_TC ? TUNE_FACTOR_MAX : 1);
+    const int64_t P_max = (int64_t)persistent_ctas(path) * (tc ? TUNE_FACTOR_MAX : 1);
     const TunedShape shape = tuned_shape(path, n_atoms, n_mol);
     L.P = persistent_ctas(path) * shape.factor;
     L.UT = shape.update_atoms;
+    L.gather = tc ? GATHER_PAIRS : table ? GATHER_QUADS : GATHER_ROWS;
+    L.gather_bar = table ? GATHER_QUADS : L.gather;
     L.cap = cap;
     // Morton code spaces of the cell grids: under 8 x max(n_atoms, 27) per structure
     L.ncell_cap = 8LL * ((int64_t)n_atoms + 27LL * n_mol);
@@ -150,14 +158,26 @@ WsLayout ws_layout(const mlff_dims& d, int32_t n_atoms, int32_t n_mol, int64_t c
     L.e_atom = take(sizeof(float) * N);
     L.md_pos32 = take(sizeof(float) * 3 * N);
     L.md_noise = take(sizeof(double) * 6 * N);
-    if (path == MLFF_PATH_TUNED_TC) {
+    if (tc) {
         L.geo = take(sizeof(float4) * cap);
         // at most cap / 32 + one partial tile per partition: sum over partitions of ceil(E_p / 32)
         L.n_etile = cap / 32 + P_max + 1;
         L.etile_base = take(4 * ((size_t)P_max + 1));
         L.etile = take((size_t)L.n_etile * 8192);
-        L.qs = take((size_t)N * 3 * 2 * H * 2);
-        L.qb = take(sizeof(float) * 3 * N);
+        if (!table) {
+            L.qs = take((size_t)N * 3 * 2 * H * 2);
+            L.qb = take(sizeof(float) * 3 * N);
+        }
+    }
+    if (table) {
+        // after a tensor-core forward pass the table's reverse pass reuses the
+        // E tiles' space (256 bytes per edge against 100)
+        const size_t keep = p;
+        if (tc) p = L.etile;
+        L.trec = take(32 * ((size_t)cap + TREC_PAD));
+        L.tperm = take(4 * cap);
+        L.tpart = take(sizeof(float4) * 4 * cap);
+        p = std::max(p, keep);
     }
     if (path == MLFF_PATH_PLAIN_FP32 || path == MLFF_PATH_TRAIN || dual) {
         L.geo = take(4 * fs * cap);
@@ -211,7 +231,8 @@ static int check_sys(const mlff_system* s, int64_t cap) {
 
 static int check_path(int32_t path) {
     if (path != MLFF_PATH_PLAIN_FP32 && path != MLFF_PATH_TUNED_TC && path != MLFF_PATH_TUNED_FP32 &&
-        path != MLFF_PATH_TRAIN && path != MLFF_PATH_TRAIN_FORCES) {
+        path != MLFF_PATH_TRAIN && path != MLFF_PATH_TRAIN_FORCES && path != MLFF_PATH_TABLE &&
+        path != MLFF_PATH_TABLE_FP32) {
         set_error("unknown path %d", path);
         return MLFF_ERR_INVALID;
     }
@@ -236,6 +257,7 @@ int energy_forces_impl(const mlff_dims& d, const void* packed, const mlff_system
     const float* P = static_cast<const float*>(packed);
     if (path == MLFF_PATH_PLAIN_FP32 || path == MLFF_PATH_TRAIN || path == MLFF_PATH_TRAIN_FORCES)
         return run_plain(d, P, po, sys, L, ws, out, st, nullptr, vf);
+    if (path == MLFF_PATH_TABLE_FP32) return run_table(d, P, po, sys, L, ws, out, path, st, vf);
     return run_tuned(d, P, po, sys, L, ws, out, path, st, vf);
 }
 int md_kick_drift(const WsLayout& L, void* ws, mlff_md_state* s, double dt, cudaStream_t st);
@@ -292,7 +314,16 @@ int mlff_pack_weights(const mlff_dims* dims, const mlff_params* params, void* pa
     }
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
     if ((r = pack_fp32(*dims, *params, static_cast<float*>(packed), o, st))) return r;
-    return pack_bf16(*dims, static_cast<float*>(packed), o, st);
+    if ((r = pack_bf16(*dims, static_cast<float*>(packed), o, st))) return r;
+    return build_tables(*dims, static_cast<float*>(packed), o, st);
+}
+
+int mlff_filter_table_class(const mlff_dims* dims, const void* packed, int32_t* accuracy, mlff_stream_t stream) {
+    int r = check_dims(dims);
+    if (r) return r;
+    if (!packed || !accuracy) { set_error("packed weights and accuracy are required"); return MLFF_ERR_INVALID; }
+    return read_table_flag(static_cast<const float*>(packed), packed_offsets(*dims), accuracy,
+                           reinterpret_cast<cudaStream_t>(stream));
 }
 
 size_t mlff_workspace_size(const mlff_dims* dims, int32_t n_atoms, int32_t n_mol, int64_t edge_capacity,
@@ -356,7 +387,7 @@ int mlff_energy_forces(const mlff_dims* dims, const void* packed, const mlff_sys
 int mlff_autotune(const mlff_dims* dims, const void* packed, const mlff_system* sys, int64_t edge_capacity,
                   int32_t path, const mlff_outputs* out, void* workspace, size_t workspace_bytes, mlff_stream_t stream,
                   int32_t repeats, int32_t* chosen, double* ms_per_candidate) {
-    if (path != MLFF_PATH_TUNED_TC) {
+    if (!has_tc_edges(path)) {
         if (chosen) *chosen = 1;
         return MLFF_OK;   // the other paths have no tunable shape
     }
@@ -440,7 +471,7 @@ int mlff_autotune_set(int32_t path, int32_t n_atoms, int32_t n_mol, int32_t fact
         set_error("partition factor %d: use 1, 2 or 4 (0 removes the entry)", factor);
         return MLFF_ERR_INVALID;
     }
-    if (path != MLFF_PATH_TUNED_TC) { set_error("only the tensor-core path has a tunable shape"); return MLFF_ERR_INVALID; }
+    if (!has_tc_edges(path)) { set_error("only the tensor-core paths have a tunable shape"); return MLFF_ERR_INVALID; }
     std::lock_guard<std::mutex> lk(g_tune_mu);
     const auto key = tune_key(path, n_atoms, n_mol);
     if (factor == 0) {
@@ -461,7 +492,7 @@ int mlff_autotune_set_shape(int32_t path, int32_t n_atoms, int32_t n_mol, int32_
         set_error("update tile %d atoms: use 32 or 64", update_atoms);
         return MLFF_ERR_INVALID;
     }
-    if (path != MLFF_PATH_TUNED_TC) { set_error("only the tensor-core path has a tunable shape"); return MLFF_ERR_INVALID; }
+    if (!has_tc_edges(path)) { set_error("only the tensor-core paths have a tunable shape"); return MLFF_ERR_INVALID; }
     std::lock_guard<std::mutex> lk(g_tune_mu);
     if (factor == 0) g_tune.erase(tune_key(path, n_atoms, n_mol));
     else g_tune[tune_key(path, n_atoms, n_mol)] = TunedShape{factor, update_atoms};

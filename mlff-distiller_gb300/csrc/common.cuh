@@ -144,6 +144,9 @@ struct PackedOffsets {
     int64_t head_b2;   // [32]
     int64_t head_w3;   // [32]
     int64_t head_b3;   // [1]
+    int64_t tab;       // [L] filter tables (tab.cuh)
+    int64_t tab_err;   // [L][intervals][4] doubles: the tables' measured errors
+    int64_t tab_flag;  // int32: accuracy class of the tables
     LayerOffsets layer[MAXL];
     int64_t total;     // floats
 };

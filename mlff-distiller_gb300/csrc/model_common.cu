@@ -12,6 +12,7 @@
 #include <cstdio>
 #include <mutex>
 #include "common.cuh"
+#include "tab.cuh"
 #include "workspace.h"
 #include "profile.h"
 
@@ -64,6 +65,9 @@ PackedOffsets packed_offsets(const mlff_dims& d) {
         L.u1t_tc = take(2 * H * 2 * H / 2);
         L.w2q_tc = take(2 * H * H / 2);
     }
+    o.tab = take(d.n_layers * TAB_LAYER);
+    o.tab_err = take((int64_t)d.n_layers * TAB_NI * 4 * 2);
+    o.tab_flag = take(1);
     o.total = p;
     return o;
 }
@@ -143,10 +147,24 @@ int pack_fp32(const mlff_dims& d, const mlff_params& p, float* out, const Packed
 
 // ------------------------------------------------------------- embedding
 __global__ void embed_kernel(const float* __restrict__ emb, const int64_t* __restrict__ Z, int32_t n_atoms,
-                             int32_t n_species, float* __restrict__ X, int pairs, Status* st) {
+                             int32_t n_species, float* __restrict__ X, int layout, Status* st) {
     pdl_wait();
     pdl_trigger();
+    if (layout == GATHER_QUADS) {   // the s rows alone: v is zero
+        const int64_t total = (int64_t)n_atoms * H;
+        for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total;
+             i += (int64_t)gridDim.x * blockDim.x) {
+            int64_t z = Z[i / H];
+            if (z < 0 || z >= n_species) {
+                set_status(st, MLFF_ERR_INVALID, (int)(i / H));
+                z = 0;
+            }
+            X[i] = emb[z * H + i % H];
+        }
+        return;
+    }
     // X[a] = (emb[Z[a]], 0, 0, 0), component-major or in the pair layout
+    const bool pairs = layout == GATHER_PAIRS;
     const int64_t total = (int64_t)n_atoms * 4 * H;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
         int64_t a = i / (4 * H);
@@ -167,10 +185,10 @@ __global__ void embed_kernel(const float* __restrict__ emb, const int64_t* __res
 }
 
 int launch_embed(const mlff_dims& d, const float* packed, const PackedOffsets& po, const mlff_system& sys,
-                 const WsLayout& L, void* ws, cudaStream_t st, bool pairs) {
+                 const WsLayout& L, void* ws, cudaStream_t st) {
     ProfScope prof(PK_OTHER, st);
     MLFF_LAUNCH_PDL("embed", embed_kernel, 152 * 8, 256, 0, st, packed + po.emb, sys.Z, sys.n_atoms, d.n_species,
-                    ws_ptr<float>(ws, L.X), pairs ? 1 : 0, ws_ptr<Status>(ws, L.status));
+                    ws_ptr<float>(ws, L.X), L.gather, ws_ptr<Status>(ws, L.status));
     return MLFF_OK;
 }
 
@@ -530,8 +548,9 @@ constexpr int UPD_ATOMS = 16;
 
 __global__ void __launch_bounds__(128) update_fwd_kernel(const float* __restrict__ P, LayerOffsets lo,
                                                          const float* __restrict__ Xt, int32_t n_atoms,
-                                                         float* __restrict__ Xout, float* __restrict__ uz,
-                                                         float* __restrict__ ua, const Status* st) {
+                                                         float* __restrict__ Xout, int out_quads,
+                                                         float* __restrict__ uz, float* __restrict__ ua,
+                                                         const Status* st) {
     __shared__ float comb[UPD_ATOMS][2 * H];
     __shared__ float hsm[UPD_ATOMS][H];
     __shared__ float mix[9];
@@ -616,11 +635,18 @@ __global__ void __launch_bounds__(128) update_fwd_kernel(const float* __restrict
             // s' = s + ds ; v' = v g1 + (M v) g2  (student_model.py:452-468)
             const float v3[3] = {vx[q], vy[q], vz[q]};
             float* xo = Xout + (int64_t)a * 4 * H;
-            xo[c] = sv[q] + o[0][q];
+            float vo[3];
 #pragma unroll
             for (int i = 0; i < 3; ++i) {
                 float mv = mix[3 * i] * v3[0] + mix[3 * i + 1] * v3[1] + mix[3 * i + 2] * v3[2];
-                xo[(1 + i) * H + c] = v3[i] * o[1][q] + mv * o[2][q];
+                vo[i] = v3[i] * o[1][q] + mv * o[2][q];
+            }
+            if (out_quads) {
+                reinterpret_cast<float4*>(xo)[c] = make_float4(sv[q] + o[0][q], vo[0], vo[1], vo[2]);
+            } else {
+                xo[c] = sv[q] + o[0][q];
+#pragma unroll
+                for (int i = 0; i < 3; ++i) xo[(1 + i) * H + c] = vo[i];
             }
         }
         __syncthreads();
@@ -632,7 +658,7 @@ __global__ void __launch_bounds__(128) update_bwd_kernel(const float* __restrict
                                                          const float* __restrict__ Xt, const float* __restrict__ uz,
                                                          const float* __restrict__ ua,
                                                          const float* __restrict__ xbar_out, int32_t n_atoms,
-                                                         float* __restrict__ xtbar, const Status* st) {
+                                                         float* __restrict__ xtbar, int out_quads, const Status* st) {
     __shared__ float abar[UPD_ATOMS][H3];
     __shared__ float zbar[UPD_ATOMS][H];
     __shared__ float mix[9];
@@ -723,9 +749,14 @@ __global__ void __launch_bounds__(128) update_bwd_kernel(const float* __restrict
             float n = pair_distance(vt[0][q], vt[1][q], vt[2][q]);
             float sc = n > 0.0f ? cn[q] / n : 0.0f;     // d|v|/dv = v/|v|, 0 at v = 0
             float* o = xtbar + (int64_t)a * 4 * H;
-            o[c] = sb[q] + cs[q];
+            if (out_quads) {
+                reinterpret_cast<float4*>(o)[c] = make_float4(sb[q] + cs[q], vb[0][q] + sc * vt[0][q],
+                                                              vb[1][q] + sc * vt[1][q], vb[2][q] + sc * vt[2][q]);
+            } else {
+                o[c] = sb[q] + cs[q];
 #pragma unroll
-            for (int i = 0; i < 3; ++i) o[(1 + i) * H + c] = vb[i][q] + sc * vt[i][q];
+                for (int i = 0; i < 3; ++i) o[(1 + i) * H + c] = vb[i][q] + sc * vt[i][q];
+            }
         }
         __syncthreads();
     }
@@ -741,7 +772,8 @@ int launch_update_fwd(const mlff_dims& d, const float* packed, const LayerOffset
     float* uz = ws_ptr<float>(ws, L.uz) + (int64_t)layer * L.N * H;
     float* ua = ws_ptr<float>(ws, L.ua) + (int64_t)layer * L.N * H3;
     int blocks = (int)std::min<int64_t>((L.N + UPD_ATOMS - 1) / UPD_ATOMS, 152 * 4);
-    update_fwd_kernel<<<std::max(blocks, 1), 128, 0, st>>>(packed, lo, Xt, L.N, Xout, uz, ua,
+    update_fwd_kernel<<<std::max(blocks, 1), 128, 0, st>>>(packed, lo, Xt, L.N, Xout,
+                                                           L.gather == GATHER_QUADS && layer + 1 < L.L, uz, ua,
                                                            ws_ptr<Status>(ws, L.status));
     MLFF_LAUNCH_CHECK("update_fwd");
     return MLFF_OK;
@@ -757,7 +789,7 @@ int launch_update_bwd(const mlff_dims& d, const float* packed, const LayerOffset
     const float* ua = ws_ptr<float>(ws, L.ua) + (int64_t)layer * L.N * H3;
     int blocks = (int)std::min<int64_t>((L.N + UPD_ATOMS - 1) / UPD_ATOMS, 152 * 4);
     update_bwd_kernel<<<std::max(blocks, 1), 128, 0, st>>>(packed, lo, Xt, uz, ua, xbar_out, L.N, xtbar,
-                                                           ws_ptr<Status>(ws, L.status));
+                                                           L.gather_bar == GATHER_QUADS, ws_ptr<Status>(ws, L.status));
     MLFF_LAUNCH_CHECK("update_bwd");
     return MLFF_OK;
 }

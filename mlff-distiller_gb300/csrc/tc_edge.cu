@@ -230,6 +230,8 @@ __global__ void __launch_bounds__(1024) etile_index_kernel(const int32_t* __rest
     if (t == 0) base[P] = carry;
 }
 
+// (DERIV false: the E rows alone, for calls whose reverse pass reads tables)
+template <bool DERIV>
 __global__ void __launch_bounds__(256) etile_fill_kernel(EdgeArgs a, const int32_t* __restrict__ base,
                                                          unsigned char* __restrict__ out) {
     pdl_wait();
@@ -242,7 +244,7 @@ __global__ void __launch_bounds__(256) etile_fill_kernel(EdgeArgs a, const int32
     __syncthreads();
     if (a.st->code != 0) return;
     constexpr int TE = 32;                              // edges per tile
-    constexpr int ROWS = ET_ROWS;
+    constexpr int ROWS = DERIV ? ET_ROWS : ET_ROWS / 2;
     constexpr int PER = 2 * ROWS;                       // threads per tile: (row, K-step)
     constexpr int TPI = 256 / PER;                      // tiles per block iteration
     const int t = threadIdx.x, sub = t / PER, loc = t % PER;
@@ -272,10 +274,11 @@ __global__ void __launch_bounds__(256) etile_fill_kernel(EdgeArgs a, const int32
     }
 }
 
-int launch_etiles(const EdgeArgs& a, int32_t* base, unsigned char* tiles, cudaStream_t st) {
+int launch_etiles(const EdgeArgs& a, int32_t* base, unsigned char* tiles, bool deriv, cudaStream_t st) {
     MLFF_LAUNCH_PDL("etile_index", etile_index_kernel, 1, 1024, 0, st, a.row_ptr, a.part, a.nparts, base);
     // tiles of a partition spread over gridDim.y blocks
-    MLFF_LAUNCH_PDL("etile_fill", etile_fill_kernel, dim3(a.nparts, 16), 256, 0, st, a, base, tiles);
+    if (deriv) MLFF_LAUNCH_PDL("etile_fill", etile_fill_kernel<true>, dim3(a.nparts, 16), 256, 0, st, a, base, tiles);
+    else MLFF_LAUNCH_PDL("etile_fill", etile_fill_kernel<false>, dim3(a.nparts, 8), 256, 0, st, a, base, tiles);
     return MLFF_OK;
 }
 

@@ -155,12 +155,17 @@ __device__ __forceinline__ void store_row4(unsigned char* tile, uint32_t half_by
 }
 
 // One atom's row of a [N][4][H] array (lane: channels 4 lane .. 4 lane + 3
-// of each component) in the component-major layout or, with pairs, in the
-// pair layout of the edge kernels' gathers (pair_off).
+// of each component) component-major or in a layout of the edge kernels'
+// gathers (GATHER_*).
 __device__ __forceinline__ void store_atom_row(float* row, int lane, float4 s, float4 x, float4 y, float4 z,
-                                               bool pairs) {
+                                               int layout) {
     float4* o = reinterpret_cast<float4*>(row);
-    if (pairs) {
+    if (layout == GATHER_QUADS) {
+        o[4 * lane] = make_float4(s.x, x.x, y.x, z.x);
+        o[4 * lane + 1] = make_float4(s.y, x.y, y.y, z.y);
+        o[4 * lane + 2] = make_float4(s.z, x.z, y.z, z.z);
+        o[4 * lane + 3] = make_float4(s.w, x.w, y.w, z.w);
+    } else if (layout == GATHER_PAIRS) {
         o[2 * lane] = make_float4(s.x, x.x, s.y, x.y);
         o[2 * lane + 1] = make_float4(s.z, x.z, s.w, x.w);
         o[64 + 2 * lane] = make_float4(y.x, z.x, y.y, z.y);
@@ -224,7 +229,7 @@ struct UFwd {
 template <int UN>
 __global__ void __launch_bounds__(UNT, 2) update_fwd_tc_kernel(const float* __restrict__ P, LayerOffsets lo,
                                                                const float* __restrict__ Xt, int32_t n_atoms,
-                                                               float* __restrict__ Xout, int out_pairs,
+                                                               float* __restrict__ Xout, int out_layout,
                                                                float* __restrict__ uz, float* __restrict__ ua,
                                                                Status* st) {
     using LF = UFwd<UN>;
@@ -413,7 +418,7 @@ __global__ void __launch_bounds__(UNT, 2) update_fwd_tc_kernel(const float* __re
                         oz.w = vnew(vx.w, vy.w, vz.w, vz.w, g1.w, g2.w, 2);
                         store_atom_row(Xout + (int64_t)a * 4 * H, lane,
                                        make_float4(sv.x + ds.x, sv.y + ds.y, sv.z + ds.z, sv.w + ds.w), ox, oy, oz,
-                                       out_pairs != 0);
+                                       out_layout);
                     }
                 }
                 __syncthreads();
@@ -460,11 +465,11 @@ static int launch_update_fwd_tc_t(const float* packed, const LayerOffsets& lo, c
     float* ua = ws_ptr<float>(ws, L.ua) + (int64_t)layer * L.N * H3;
     const int ntiles = (L.N + UN - 1) / UN;
     const int grid = std::max(1, std::min(ntiles, 2 * num_sms()));
-    // the next layer's input in the pair layout of the edge kernels' gathers;
-    // the last layer's output (read by the readout) component-major
-    const int out_pairs = layer + 1 < L.L ? 1 : 0;
+    // the next layer's input in the layout of the edge kernels' gathers; the
+    // last layer's output (read by the readout) component-major
+    const int out_layout = layer + 1 < L.L ? L.gather : GATHER_ROWS;
     MLFF_LAUNCH_PDL("update_fwd_tc", update_fwd_tc_kernel<UN>, grid, UNT, UFwd<UN>::SMEM, st, packed, lo, Xt, L.N,
-                    Xout, out_pairs, uz, ua, ws_ptr<Status>(ws, L.status));
+                    Xout, out_layout, uz, ua, ws_ptr<Status>(ws, L.status));
     return MLFF_OK;
 }
 
@@ -501,7 +506,7 @@ __global__ void __launch_bounds__(UNT, 2) update_bwd_tc_kernel(const float* __re
                                                                const float* __restrict__ Xt, const float* __restrict__ uz,
                                                                const float* __restrict__ ua,
                                                                const float* __restrict__ xbo, int32_t n_atoms,
-                                                               float* __restrict__ xtbar, Status* st) {
+                                                               float* __restrict__ xtbar, int out_layout, Status* st) {
     using LB = UBwd<UN>;
     extern __shared__ __align__(1024) unsigned char smem[];
     unsigned char* Bs = smem + LB::OFF_B;
@@ -686,9 +691,9 @@ __global__ void __launch_bounds__(UNT, 2) update_bwd_tc_kernel(const float* __re
                     one(bx.y, by.y, bz.y, vx.y, vy.y, vz.y, g1.y, g2.y, cn.y, ox.y, oy.y, oz.y);
                     one(bx.z, by.z, bz.z, vx.z, vy.z, vz.z, g1.z, g2.z, cn.z, ox.z, oy.z, oz.z);
                     one(bx.w, by.w, bz.w, vx.w, vy.w, vz.w, g1.w, g2.w, cn.w, ox.w, oy.w, oz.w);
-                    // dE/dXt in the pair layout the reverse edge kernel gathers from
+                    // dE/dXt in the layout the reverse edge kernel gathers from
                     store_atom_row(xtbar + (int64_t)a * 4 * H, lane,
-                                   make_float4(sb.x + cs.x, sb.y + cs.y, sb.z + cs.z, sb.w + cs.w), ox, oy, oz, true);
+                                   make_float4(sb.x + cs.x, sb.y + cs.y, sb.z + cs.z, sb.w + cs.w), ox, oy, oz, out_layout);
                 }
             }
         }
@@ -730,7 +735,7 @@ static int launch_update_bwd_tc_t(const float* packed, const LayerOffsets& lo, c
     const int ntiles = (L.N + UN - 1) / UN;
     const int grid = std::max(1, std::min(ntiles, 2 * num_sms()));
     MLFF_LAUNCH_PDL("update_bwd_tc", update_bwd_tc_kernel<UN>, grid, UNT, UBwd<UN>::SMEM, st, packed, lo, Xt, uz, ua,
-                    xbar_out, L.N, xtbar, ws_ptr<Status>(ws, L.status));
+                    xbar_out, L.N, xtbar, L.gather_bar, ws_ptr<Status>(ws, L.status));
     return MLFF_OK;
 }
 

@@ -300,7 +300,7 @@ int launch_edge_fwd_tc(const EdgeArgs& a, int layer, cudaStream_t st);
 int launch_edge_bwd_tc(const EdgeArgs& a, int layer, cudaStream_t st);
 int launch_vq(const float* P, const LayerOffsets& lo, const float* xtbar, int n_atoms, unsigned char* qs, float* qb,
               Status* st_word, cudaStream_t st);
-int launch_etiles(const EdgeArgs& a, int32_t* base, unsigned char* tiles, cudaStream_t st);
+int launch_etiles(const EdgeArgs& a, int32_t* base, unsigned char* tiles, bool deriv, cudaStream_t st);
 
 
 __global__ void edge_geom_kernel(EdgeArgs a, float4* __restrict__ geo) {
@@ -317,18 +317,16 @@ __global__ void edge_geom_kernel(EdgeArgs a, float4* __restrict__ geo) {
     }
 }
 
-// dst += src over n4 float4 elements (the reverse tensor-core edge kernel
-// writes the gathered part of dE/dX only)
 int run_tuned(const mlff_dims& d, const float* P, const PackedOffsets& po, const mlff_system& sys,
               const WsLayout& L, void* ws, const mlff_outputs& out, int path, cudaStream_t st,
               const VerletFuse* vf) {
     const int N = sys.n_atoms;
     const int64_t NX = (int64_t)N * 4 * H;
     int r;
-    const bool tc = path == MLFF_PATH_TUNED_TC;
-    // the tensor-core path keeps the layer inputs X[0..L-1] and dE/dXt in the
-    // pair layout of its edge kernels' gathers
-    if ((r = launch_embed(d, P, po, sys, L, ws, st, tc))) return r;
+    // MLFF_PATH_TABLE: the tensor-core forward pass, then run_table's reverse pass
+    const bool table = path == MLFF_PATH_TABLE;
+    const bool tc = path == MLFF_PATH_TUNED_TC || table;
+    if ((r = launch_embed(d, P, po, sys, L, ws, st))) return r;
     if ((r = launch_partition(L, ws, st))) return r;
     EdgeArgs a{};
     a.pos4 = ws_ptr<float4>(ws, L.pos4);
@@ -360,7 +358,8 @@ int run_tuned(const mlff_dims& d, const float* P, const PackedOffsets& po, const
         // [E; E'] tiles (RBF x cutoff and its d-derivative) of every 32 edges,
         // for every layer: the forward kernel reads their E rows, the reverse
         // kernel both
-        if ((r = launch_etiles(a, ws_ptr<int32_t>(ws, L.etile_base), ws_ptr<unsigned char>(ws, L.etile), st)))
+        if ((r = launch_etiles(a, ws_ptr<int32_t>(ws, L.etile_base), ws_ptr<unsigned char>(ws, L.etile), !table,
+                               st)))
             return r;
         a.etile = ws_ptr<unsigned char>(ws, L.etile);
         a.etile_base = ws_ptr<int32_t>(ws, L.etile_base);
@@ -385,6 +384,7 @@ int run_tuned(const mlff_dims& d, const float* P, const PackedOffsets& po, const
     const bool want_grad = out.forces != nullptr || out.virial != nullptr;
     if ((r = launch_readout(d, P, po, sys, L, ws, out, want_grad ? 1 : 0, st))) return r;
     if (!want_grad) return MLFF_OK;
+    if (table) return run_table_reverse(d, P, po, sys, L, ws, out, path, st, vf);
     float* xbo = ws_ptr<float>(ws, L.xbar);
     float* xtb = xbo + NX;
     for (int l = d.n_layers - 1; l >= 0; --l) {

@@ -10,9 +10,17 @@ namespace mlff {
 constexpr int GRAD_SPLIT = 64;        // row splits of the weight-gradient reductions
 constexpr int GRAD_MIX_BLOCKS = 304;  // blocks of the mixing-matrix gradient
 
+// Layout of the layer inputs X[0..L-1] and of dE/dXt that the path's edge
+// kernels gather: component-major rows, the tensor-core path's component
+// pairs (pair_off) or the table path's quads (quad_off; X[0] holds the s rows
+// alone).
+enum { GATHER_ROWS = 0, GATHER_PAIRS = 1, GATHER_QUADS = 2 };
+
 struct WsLayout {
     int32_t N, B, L, P;        // atoms, structures, layers, persistent CTAs
     int32_t UT;                // atoms per tile of the tensor-core update kernels (64 or 32)
+    int32_t gather;            // GATHER_* of the layer inputs
+    int32_t gather_bar;        // GATHER_* of dE/dXt
     int64_t cap;               // edge capacity
     int64_t ncell_cap;         // cell-code capacity, 8 (N + 27 B) (Morton code spaces of the cell grids)
     size_t status;             // Status
@@ -46,6 +54,10 @@ struct WsLayout {
     size_t qs;                 // reverse: per-atom Q rows [N][3][hi, lo][H] fp16 (W2's third chunk^T dE/dXt_v)
     size_t qb;                 // reverse: per-atom b2 . dE/dXt_v [N][3] float
     int64_t n_etile;
+    // table path: edges of each receiver group sorted by table interval
+    size_t trec;               // TabRec [cap + TREC_PAD], 32 bytes each
+    size_t tperm;              // int32 [cap] sorted position -> edge
+    size_t tpart;              // float4 [4][cap] (dE/dd, dE/du) of each 32-channel slice
     size_t erbf;               // float [cap][RMAX]
     size_t erbf_d;             // float [cap][RMAX]
     size_t fz;                 // float [L][cap][H]
@@ -98,9 +110,9 @@ struct NbrBuffers {
 int launch_neighbors_into(const mlff_dims& d, const mlff_system& sys, const NbrBuffers& b, cudaStream_t st);
 int launch_neighbors(const mlff_dims& d, const mlff_system& sys, const WsLayout& L, void* ws,
                      cudaStream_t st);
-// X[0] component-major or (pairs: the tensor-core path) in the pair layout
+// X[0] in the path's gather layout (L.gather)
 int launch_embed(const mlff_dims& d, const float* packed, const PackedOffsets& po,
-                 const mlff_system& sys, const WsLayout& L, void* ws, cudaStream_t st, bool pairs = false);
+                 const mlff_system& sys, const WsLayout& L, void* ws, cudaStream_t st);
 int launch_readout(const mlff_dims& d, const float* packed, const PackedOffsets& po,
                    const mlff_system& sys, const WsLayout& L, void* ws, const mlff_outputs& out,
                    int want_grad, cudaStream_t st);
@@ -158,6 +170,13 @@ int grad_embedding(const mlff_dims& d, const mlff_system& sys, const WsLayout& L
 int run_tuned(const mlff_dims& d, const float* packed, const PackedOffsets& po,
               const mlff_system& sys, const WsLayout& L, void* ws, const mlff_outputs& out,
               int path, cudaStream_t st, const VerletFuse* vf = nullptr);
+int run_table(const mlff_dims& d, const float* packed, const PackedOffsets& po,
+              const mlff_system& sys, const WsLayout& L, void* ws, const mlff_outputs& out,
+              int path, cudaStream_t st, const VerletFuse* vf = nullptr);
+// reverse pass, forces and virial from the tables after either forward pass
+int run_table_reverse(const mlff_dims& d, const float* packed, const PackedOffsets& po,
+                      const mlff_system& sys, const WsLayout& L, void* ws, const mlff_outputs& out,
+                      int path, cudaStream_t st, const VerletFuse* vf);
 int launch_partition(const WsLayout& L, void* ws, cudaStream_t st);
 int launch_scan(int32_t* data, int64_t n, int32_t* tmp, cudaStream_t st);
 int launch_update_fwd(const mlff_dims& d, const float* packed, const LayerOffsets& lo,
@@ -166,6 +185,11 @@ int launch_update_fwd_tc(const float* packed, const LayerOffsets& lo, const WsLa
                          cudaStream_t st);
 int launch_update_bwd_tc(const float* packed, const LayerOffsets& lo, const WsLayout& L, void* ws, int layer,
                          const float* xbar_out, float* xtbar, cudaStream_t st);
+// the same in FP32 for the table path (upd32.cu)
+int launch_upd32_fwd(const float* packed, const LayerOffsets& lo, const WsLayout& L, void* ws, int layer,
+                     cudaStream_t st);
+int launch_upd32_bwd(const float* packed, const LayerOffsets& lo, const WsLayout& L, void* ws, int layer,
+                     const float* xbar_out, float* xtbar, cudaStream_t st);
 int launch_update_bwd(const mlff_dims& d, const float* packed, const LayerOffsets& lo,
                       const WsLayout& L, void* ws, int layer, const float* xbar_out,
                       float* xtbar, cudaStream_t st);

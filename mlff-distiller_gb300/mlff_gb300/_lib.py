@@ -29,6 +29,8 @@ PATH_TUNED_TC = 1
 PATH_TUNED_FP32 = 2
 PATH_TRAIN = 3
 PATH_TRAIN_FORCES = 4
+PATH_TABLE = 5
+PATH_TABLE_FP32 = 6
 
 PATHS = {"plain": PATH_PLAIN_FP32, "fp32": PATH_PLAIN_FP32, "plain_fp32": PATH_PLAIN_FP32,
          "fp16x3": PATH_TUNED_TC, "tc": PATH_TUNED_TC, "tuned": PATH_TUNED_TC,
@@ -50,7 +52,7 @@ EXPORTS = ["mlff_version", "mlff_last_error_string", "mlff_packed_weights_size",
            "mlff_painn_message_backward", "mlff_painn_update_workspace_size", "mlff_painn_update",
            "mlff_painn_update_backward", "mlff_force_stats_workspace_size", "mlff_force_stats",
            "mlff_autotune", "mlff_autotune_query", "mlff_autotune_set", "mlff_autotune_query_shape",
-           "mlff_autotune_set_shape", "mlff_autotune_reset"]
+           "mlff_autotune_set_shape", "mlff_autotune_reset", "mlff_filter_table_class"]
 
 PROFILE_KINDS = ["neighbors", "edge_fwd", "edge_bwd", "update_fwd", "update_bwd", "readout", "forces",
                  "plain_gemm", "plain_edge", "other", "md", "edge_bwd_q"]
@@ -135,6 +137,8 @@ def load(build_if_missing: bool = True):
         lib.mlff_packed_weights_size.argtypes = [ctypes.POINTER(Dims)]
         lib.mlff_pack_weights.restype = ctypes.c_int
         lib.mlff_pack_weights.argtypes = [ctypes.POINTER(Dims), ctypes.POINTER(Params), _P, sz, _P]
+        lib.mlff_filter_table_class.restype = ctypes.c_int
+        lib.mlff_filter_table_class.argtypes = [ctypes.POINTER(Dims), _P, ctypes.POINTER(i32), _P]
         lib.mlff_workspace_size.restype = sz
         lib.mlff_workspace_size.argtypes = [ctypes.POINTER(Dims), i32, i32, i64, i32]
         lib.mlff_build_neighbors.restype = ctypes.c_int

@@ -105,6 +105,7 @@ class Engine:
         self.workspace: Optional[torch.Tensor] = None
         self.edge_capacity: Dict[int, int] = {}
         self._param_version = None
+        self.table_class = 0            # accuracy class of the packed weights' filter tables
         self.use_graphs = True          # replay cached CUDA graphs for repeated shapes
         self.auto_tune = True           # tune the tensor-core path's partition factor once per size bucket
         self._graphs: Dict[tuple, dict] = {}
@@ -136,8 +137,28 @@ class Engine:
         _lib.check(self.lib.mlff_pack_weights(ctypes.byref(self.dims), ctypes.byref(p),
                                               self.packed.data_ptr(), self.packed.numel() * 4,
                                               _stream_handle()))
-        torch.cuda.current_stream().synchronize()
+        cls = ctypes.c_int32(0)   # (synchronises)
+        _lib.check(self.lib.mlff_filter_table_class(ctypes.byref(self.dims), self.packed.data_ptr(),
+                                                    ctypes.byref(cls), _stream_handle()))
+        self.table_class = cls.value
         del self._keep
+
+    def route(self, path: int) -> int:
+        """The library path that evaluates ``path`` with the packed weights:
+        the tabulated-filter form of the fused paths when the tables are as
+        accurate as the network evaluation they replace, else the network
+        form."""
+        tc, fp32 = self.table_class >= 1, self.table_class >= 2
+        if path in (_lib.PATH_TUNED_TC, _lib.PATH_TABLE):
+            return _lib.PATH_TABLE if tc else _lib.PATH_TUNED_TC
+        if path in (_lib.PATH_TUNED_FP32, _lib.PATH_TABLE_FP32):
+            return _lib.PATH_TABLE_FP32 if fp32 else _lib.PATH_TUNED_FP32
+        return path
+
+    def _checked_path(self, path: int) -> int:
+        """A table path chosen for earlier weights falls back when the
+        tables of the present weights do not serve it."""
+        return self.route(path) if path in (_lib.PATH_TABLE, _lib.PATH_TABLE_FP32) else path
 
     # ------------------------------------------------------------ workspace
     def workspace_for(self, n_atoms: int, n_mol: int, cap: int, path: int) -> torch.Tensor:
@@ -174,6 +195,7 @@ class Engine:
         immutable: passing the same tensor object again skips its copy.
         ``to_host``: the batch's Z and positions may live in host memory and
         the results are returned in host memory."""
+        path = self._checked_path(path)
         use_graph = self.use_graphs if graph is None else graph
         if use_graph and check and not torch.cuda.is_current_stream_capturing():
             res = self._graph_call(batch, path, forces, virial, atom_energy, to_host)
@@ -235,7 +257,7 @@ class Engine:
             del self._graphs[key]
             ent = None
         if ent is None:
-            if self.auto_tune and path == _lib.PATH_TUNED_TC and _bucket(path, N, B) not in _tuned_buckets:
+            if self.auto_tune and path in (_lib.PATH_TUNED_TC, _lib.PATH_TABLE) and _bucket(path, N, B) not in _tuned_buckets:
                 db = batch if not to_host else Batch(batch.Z.to(self.device), batch.pos.to(self.device),
                                                      batch.mol_ptr, batch.box, batch.pbc)
                 self.autotune(db, path)
@@ -318,6 +340,7 @@ class Engine:
         cached by the library for every call of the bucket).  Returns the
         choices and the milliseconds per call of each partition factor.
         Synchronises the stream; not for use during stream capture."""
+        path = self._checked_path(path)
         self.energy_forces(batch, path, graph=False)       # sizes the edge capacity and workspace
         N, B = batch.n_atoms, batch.n_mol
         cap = self.capacity(N, path)

@@ -248,6 +248,7 @@ class VelocityVerletGPU:
 
     # one library call of n steps on the current stream
     def _call(self, n_steps: int, cap: int, e_trace: Optional[torch.Tensor], k_trace: Optional[torch.Tensor]):
+        self.path = self.engine._checked_path(self.path)
         ws = self.engine.workspace_for(self.N, self.B, cap, self.path)
         st = _lib.MDState()
         st.pos, st.vel = self.pos.data_ptr(), self.vel.data_ptr()

@@ -281,7 +281,8 @@ class _EnergyTrain(torch.autograd.Function):
     @staticmethod
     def forward(ctx, positions, model, batch, mol_index, *params):
         from . import _lib
-        E, F, _ = model.engine().energy_forces(batch, _lib.PATH_TUNED_FP32, forces=True)
+        eng = model.engine()
+        E, F, _ = eng.energy_forces(batch, eng.route(_lib.PATH_TUNED_FP32), forces=True)
         ctx.model, ctx.batch = model, batch
         ctx.save_for_backward(F, mol_index, *params)
         return E.to(positions.dtype)
@@ -461,10 +462,12 @@ class StudentForceField(nn.Module):
     # ------------------------------------------------------------- engine
     @property
     def path(self) -> int:
+        """Library path of ``precision`` for the weights packed last."""
         try:
-            return _lib.PATHS[self.precision]
+            base = _lib.PATHS[self.precision]
         except KeyError:
             raise ValueError(f"unknown precision {self.precision!r}; use one of {sorted(_lib.PATHS)}")
+        return base if self._engine is None else self._engine.route(base)
 
     def _weights_version(self):
         """(address, in-place version) of every parameter and buffer: changes
@@ -493,7 +496,8 @@ class StudentForceField(nn.Module):
         return self._engine
 
     def _engine_call(self, batch: Batch, forces: bool = True, virial: bool = False, to_host: bool = False):
-        return self.engine().energy_forces(batch, self.path, forces=forces, virial=virial, to_host=to_host)
+        eng = self.engine()   # packs changed weights, which decides the path
+        return eng.energy_forces(batch, self.path, forces=forces, virial=virial, to_host=to_host)
 
     def _make_batch(self, atomic_numbers, positions, cell, pbc, batch, need_index: bool = True,
                     host_inputs: bool = False):
