@@ -57,6 +57,8 @@ typedef struct CUstream_st *mlff_stream_t; /* same type as cudaStream_t */
 #define MLFF_PATH_TABLE 5         /* path 1's forward pass, reverse pass from the tables (class 1 or 2) */
 #define MLFF_PATH_TABLE_FP32 6    /* path 2 from the tables, both passes (class 2) */
 
+#define MLFF_PATH_TRAIN_TABLE 7   /* mlff_param_grads_table and its force term (workspace sizing) */
+
 #define MLFF_MAX_LAYERS 8
 
 /* Model shape: StudentForceField(hidden_dim, num_interactions, num_rbf,
@@ -354,6 +356,21 @@ int mlff_param_grads_forces(const mlff_dims *dims, const void *packed, const mlf
                             int64_t edge_capacity, const float *force_weights, const double *virial_weights,
                             const mlff_grads *grads, void *workspace, size_t workspace_bytes,
                             mlff_stream_t stream);
+
+/* The same two with tabulated filters, for weights whose tables are of class
+ * 2 (mlff_filter_table_class; otherwise MLFF_ERR_UNSUPPORTED in the status
+ * word).  A filter value is linear in the network's values at the table's
+ * 576 nodes, so the filter's weight gradients need the network's reverse
+ * pass at those nodes only; everything else is evaluated as in path 6.
+ * energy: double [B].  Fixed-order sums: the same bits on every call.
+ * Workspace of both: mlff_workspace_size(..., MLFF_PATH_TRAIN_TABLE). */
+int mlff_param_grads_table(const mlff_dims *dims, const void *packed, const mlff_system *sys,
+                           int64_t edge_capacity, const double *energy_weights, const mlff_grads *grads,
+                           double *energy, void *workspace, size_t workspace_bytes, mlff_stream_t stream);
+int mlff_param_grads_forces_table(const mlff_dims *dims, const void *packed, const mlff_system *sys,
+                                  int64_t edge_capacity, const float *force_weights,
+                                  const double *virial_weights, const mlff_grads *grads, void *workspace,
+                                  size_t workspace_bytes, mlff_stream_t stream);
 
 /* Kernel timing for benchmarks (no counterpart in the reference, whose
  * timers wrap whole Python calls: cuda/benchmark_utils.py:147-194).

@@ -110,7 +110,8 @@ WsLayout ws_layout(const mlff_dims& d, int32_t n_atoms, int32_t n_mol, int64_t c
     L.B = n_mol;
     L.L = d.n_layers;
     const bool tc = has_tc_edges(path);
-    const bool table = path == MLFF_PATH_TABLE || path == MLFF_PATH_TABLE_FP32;
+    const bool train_table = path == MLFF_PATH_TRAIN_TABLE;
+    const bool table = path == MLFF_PATH_TABLE || path == MLFF_PATH_TABLE_FP32 || train_table;
     // arrays sized for the largest partition factor, so that tuning never changes the size
     const int64_t P_max = (int64_t)persistent_ctas(path) * (tc ? TUNE_FACTOR_MAX : 1);
     const TunedShape shape = tuned_shape(path, n_atoms, n_mol);
@@ -131,7 +132,8 @@ WsLayout ws_layout(const mlff_dims& d, int32_t n_atoms, int32_t n_mol, int64_t c
     // the tangent pass of the force-loss gradient keeps (value, tangent)
     // pairs in the plain path's float arrays
     const bool dual = path == MLFF_PATH_TRAIN_FORCES;
-    const size_t fs = dual ? 2 * sizeof(float) : sizeof(float);
+    // (the table path's training: value planes, then tangent planes)
+    const size_t fs = dual || train_table ? 2 * sizeof(float) : sizeof(float);
     const int64_t scan_n = std::max<int64_t>(N + 1, L.ncell_cap + 1);
     L.status = take(sizeof(Status));
     L.pos4 = take(sizeof(float4) * N);
@@ -197,6 +199,7 @@ WsLayout ws_layout(const mlff_dims& d, int32_t n_atoms, int32_t n_mol, int64_t c
         L.gpart = take(fs * GRAD_SPLIT * H3 * H);
         L.gmix = take(fs * GRAD_MIX_BLOCKS * 9);
     }
+    if (train_table) p = train_table_workspace(L, d, p);
     L.total = p;
     return L;
 }
@@ -232,7 +235,7 @@ static int check_sys(const mlff_system* s, int64_t cap) {
 static int check_path(int32_t path) {
     if (path != MLFF_PATH_PLAIN_FP32 && path != MLFF_PATH_TUNED_TC && path != MLFF_PATH_TUNED_FP32 &&
         path != MLFF_PATH_TRAIN && path != MLFF_PATH_TRAIN_FORCES && path != MLFF_PATH_TABLE &&
-        path != MLFF_PATH_TABLE_FP32) {
+        path != MLFF_PATH_TABLE_FP32 && path != MLFF_PATH_TRAIN_TABLE) {
         set_error("unknown path %d", path);
         return MLFF_ERR_INVALID;
     }
@@ -257,7 +260,7 @@ int energy_forces_impl(const mlff_dims& d, const void* packed, const mlff_system
     const float* P = static_cast<const float*>(packed);
     if (path == MLFF_PATH_PLAIN_FP32 || path == MLFF_PATH_TRAIN || path == MLFF_PATH_TRAIN_FORCES)
         return run_plain(d, P, po, sys, L, ws, out, st, nullptr, vf);
-    if (path == MLFF_PATH_TABLE_FP32) return run_table(d, P, po, sys, L, ws, out, path, st, vf);
+    if (path == MLFF_PATH_TABLE_FP32 || path == MLFF_PATH_TRAIN_TABLE) return run_table(d, P, po, sys, L, ws, out, path, st, vf);
     return run_tuned(d, P, po, sys, L, ws, out, path, st, vf);
 }
 int md_kick_drift(const WsLayout& L, void* ws, mlff_md_state* s, double dt, cudaStream_t st);
@@ -704,6 +707,43 @@ int mlff_param_grads_forces(const mlff_dims* dims, const void* packed, const mlf
     GradCtx g{nullptr, *grads};
     return run_plain_tangent(*dims, static_cast<const float*>(packed), po, *sys, L, workspace, st, g, force_weights,
                              virial_weights);
+}
+
+int mlff_param_grads_table(const mlff_dims* dims, const void* packed, const mlff_system* sys, int64_t edge_capacity,
+                           const double* energy_weights, const mlff_grads* grads, double* energy, void* workspace,
+                           size_t workspace_bytes, mlff_stream_t stream) {
+    WsLayout L;
+    int r = prepare(dims, sys, edge_capacity, MLFF_PATH_TRAIN_TABLE, workspace, workspace_bytes, L);
+    if (r) return r;
+    if (!packed || !energy_weights || !grads || !energy) {
+        set_error("packed weights, energy_weights, grads and energy are required");
+        return MLFF_ERR_INVALID;
+    }
+    cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+    MLFF_CUDA(cudaMemsetAsync(ws_ptr<Status>(workspace, L.status), 0, sizeof(Status), st));
+    if ((r = launch_neighbors(*dims, *sys, L, workspace, st))) return r;
+    const GradCtx g{energy_weights, *grads};
+    return run_train_table(*dims, static_cast<const float*>(packed), packed_offsets(*dims), *sys, L, workspace, energy,
+                           st, g);
+}
+
+int mlff_param_grads_forces_table(const mlff_dims* dims, const void* packed, const mlff_system* sys,
+                                  int64_t edge_capacity, const float* force_weights, const double* virial_weights,
+                                  const mlff_grads* grads, void* workspace, size_t workspace_bytes,
+                                  mlff_stream_t stream) {
+    WsLayout L;
+    int r = prepare(dims, sys, edge_capacity, MLFF_PATH_TRAIN_TABLE, workspace, workspace_bytes, L);
+    if (r) return r;
+    if (!packed || (!force_weights && !virial_weights) || !grads) {
+        set_error("packed weights, grads and force_weights and / or virial_weights are required");
+        return MLFF_ERR_INVALID;
+    }
+    cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+    MLFF_CUDA(cudaMemsetAsync(ws_ptr<Status>(workspace, L.status), 0, sizeof(Status), st));
+    if ((r = launch_neighbors(*dims, *sys, L, workspace, st))) return r;
+    const GradCtx g{nullptr, *grads};
+    return run_train_table_tangent(*dims, static_cast<const float*>(packed), packed_offsets(*dims), *sys, L, workspace,
+                                   st, g, force_weights, virial_weights);
 }
 
 int mlff_read_status(const void* workspace, int32_t* code, int64_t* n_edges, int32_t* where, mlff_stream_t stream) {

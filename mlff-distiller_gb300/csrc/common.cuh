@@ -145,6 +145,7 @@ struct PackedOffsets {
     int64_t head_w3;   // [32]
     int64_t head_b3;   // [1]
     int64_t tab;       // [L] filter tables (tab.cuh)
+    int64_t tab_node;  // [L] network values at the tables' nodes
     int64_t tab_err;   // [L][intervals][4] doubles: the tables' measured errors
     int64_t tab_flag;  // int32: accuracy class of the tables
     LayerOffsets layer[MAXL];

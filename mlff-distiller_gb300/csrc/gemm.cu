@@ -71,7 +71,7 @@ __global__ void __launch_bounds__(256, TM == 8 ? 2 : 4) gemm_nn_kernel(const flo
                                                       const float* __restrict__ bias, float* __restrict__ C,
                                                       float* __restrict__ C2, const float* __restrict__ Z,
                                                       int64_t M_static, const int32_t* __restrict__ m_dev, int N,
-                                                      int K, const Status* st) {
+                                                      int K, int lda, const Status* st) {
     using T = Tile<BM, BN, TM, TN>;
     static_assert(T::NT == 256, "256 threads");
     __shared__ __align__(16) float As[2][BK * T::LDA];
@@ -83,7 +83,7 @@ __global__ void __launch_bounds__(256, TM == 8 ? 2 : 4) gemm_nn_kernel(const flo
     const int64_t m_tiles = (M + BM - 1) / BM;
     // 16-byte loads and stores need rows that are multiples of 4 floats on a
     // 16-byte aligned base
-    const bool va = (K & 3) == 0 && aligned16(A), vb = (N & 3) == 0 && aligned16(B);
+    const bool va = (K & 3) == 0 && (lda & 3) == 0 && aligned16(A), vb = (N & 3) == 0 && aligned16(B);
     const bool vc = T::CN == 4 && (N & 3) == 0 && aligned16(C) && (MODE != 1 || aligned16(C2)) &&
                     (MODE != 2 || aligned16(Z));
     constexpr int LA = BM * BK / 256, LB = BN * BK / 256;   // floats per thread and step
@@ -102,7 +102,7 @@ __global__ void __launch_bounds__(256, TM == 8 ? 2 : 4) gemm_nn_kernel(const flo
 #pragma unroll
                 for (int q = 0; q < LA / 4; ++q) {
                     const int i = t + 256 * q, r = i / (BK / 4), k = k0 + 4 * (i % (BK / 4));
-                    const float4 x = (m0 + r < M && k < K) ? *reinterpret_cast<const float4*>(A + (m0 + r) * K + k)
+                    const float4 x = (m0 + r < M && k < K) ? *reinterpret_cast<const float4*>(A + (m0 + r) * lda + k)
                                                            : make_float4(0.f, 0.f, 0.f, 0.f);
                     ra[4 * q] = x.x; ra[4 * q + 1] = x.y; ra[4 * q + 2] = x.z; ra[4 * q + 3] = x.w;
                 }
@@ -110,7 +110,7 @@ __global__ void __launch_bounds__(256, TM == 8 ? 2 : 4) gemm_nn_kernel(const flo
 #pragma unroll
                 for (int q = 0; q < LA; ++q) {
                     const int i = t + 256 * q, r = i / BK, k = k0 + i % BK;
-                    ra[q] = (m0 + r < M && k < K) ? A[(m0 + r) * K + k] : 0.f;
+                    ra[q] = (m0 + r < M && k < K) ? A[(m0 + r) * lda + k] : 0.f;
                 }
             }
             if (vb && LB >= 4) {
@@ -220,28 +220,29 @@ constexpr int TN_MIN_ROWS = 64;   // rows per split
 inline int tn_tiles(int64_t n) { return (int)std::max<int64_t>(1, (n + TNB - 1) / TNB); }
 inline int tn_splits(int64_t M, int64_t N) {
     const int tiles = tn_tiles(M) * tn_tiles(N);
-    return std::max(1, std::min(TN_MAX_SPLIT, (TN_TARGET_BLOCKS + tiles - 1) / tiles));
+    return std::max(2, std::min(TN_MAX_SPLIT, (TN_TARGET_BLOCKS + tiles - 1) / tiles));
 }
 
-__global__ void __launch_bounds__(256, 4) gemm_tn_kernel(const float* __restrict__ A, int lda,
-                                                      const float* __restrict__ B, int ldb, int M, int N,
-                                                      int64_t rows_static, const int32_t* __restrict__ n_dev,
-                                                      int nsplit, int want_sum, float* __restrict__ part,
-                                                      const Status* st) {
+// splits [0, nsplit / segments) cover the first set of rows, the rest the second
+__global__ void __launch_bounds__(256, 4) gemm_tn_kernel(GemmRows x, int lda, int ldb, int M, int N, int64_t rows,
+                                                         int nsplit, int want_sum, float* __restrict__ part,
+                                                         const Status* st) {
     using T = Tile<TNB, TNB, 4, 4>;
     __shared__ __align__(16) float As[2][BK * T::LDA];
     __shared__ __align__(16) float Bs[2][BK * T::LDB];
     if (st->code != 0) return;
-    const int64_t rows = n_dev ? (int64_t)(*n_dev) : rows_static;
     const int tiles_n = max(1, (N + TNB - 1) / TNB);
     const int m0 = (blockIdx.x / tiles_n) * TNB, n0 = (blockIdx.x % tiles_n) * TNB;
-    int64_t per = (rows + nsplit - 1) / nsplit;
+    const int seg_splits = x.A1 ? nsplit / 2 : nsplit, seg = blockIdx.y / seg_splits;
+    const float* A = seg ? x.A1 : x.A;
+    const float* B = seg ? x.B1 : x.B;
+    int64_t per = (rows + seg_splits - 1) / seg_splits;
     if (per < TN_MIN_ROWS) per = TN_MIN_ROWS;
-    const int64_t r0 = (int64_t)blockIdx.y * per, r1 = min(rows, r0 + per);
+    const int64_t r0 = (int64_t)(blockIdx.y - seg * seg_splits) * per, r1 = min(rows, r0 + per);
     const int t = threadIdx.x, tx = t % T::NTX, ty = t / T::NTX;
     const bool va = (lda & 3) == 0 && (M & 3) == 0 && aligned16(A);
     const bool vb = (ldb & 3) == 0 && (N & 3) == 0 && aligned16(B);
-    const bool sums = want_sum && n0 == 0;
+    const bool sums = want_sum && n0 == 0 && seg == 0;
     float acc[4][4] = {}, asum[4] = {};
     float ra[4], rb[4];
     auto fetch1 = [&](const float* S, int ld, int c0, int ncol, bool vec, int64_t r, float (&v)[4]) {
@@ -303,13 +304,13 @@ __global__ void __launch_bounds__(256, 4) gemm_tn_kernel(const float* __restrict
             const int n = n0 + 4 * tx + j;
             if (n < N) out[(int64_t)m * N + n] = acc[i][j];
         }
-        if (sums && tx == 0) part[(int64_t)nsplit * M * N + (int64_t)blockIdx.y * M + m] = asum[i];
+        if (want_sum && n0 == 0 && tx == 0) part[(int64_t)nsplit * M * N + (int64_t)blockIdx.y * M + m] = asum[i];
     }
 }
 
 // sums over the splits, in split order: four interleaved chains per output
 __global__ void __launch_bounds__(256) gemm_tn_sum_kernel(const float* __restrict__ part, int64_t MN, int M,
-                                                          int nsplit, float* __restrict__ C,
+                                                          int nsplit, int acc, float* __restrict__ C,
                                                           float* __restrict__ colsum, const Status* st) {
     if (st->code != 0) return;
     const int64_t total = (C ? MN : 0) + (colsum ? M : 0);
@@ -324,18 +325,20 @@ __global__ void __launch_bounds__(256) gemm_tn_sum_kernel(const float* __restric
 #pragma unroll
             for (int q = 0; q < 4; ++q) s[q] += p[(int64_t)(sp + q) * stride];
         for (; sp < nsplit; ++sp) s[0] += p[(int64_t)sp * stride];
-        (col ? colsum : C)[j] = (s[0] + s[1]) + (s[2] + s[3]);
+        const float v = (s[0] + s[1]) + (s[2] + s[3]);
+        float* o = (col ? colsum : C) + j;
+        *o = acc ? *o + v : v;
     }
 }
 
 template <int BM, int BN, int TM, int TN>
 int launch_nn(int mode, const float* A, const float* B, const float* bias, float* C, float* C2, const float* Z,
-              int64_t M, const int32_t* m_dev, int N, int K, const Status* st, cudaStream_t s, int per_sm) {
+              int64_t M, const int32_t* m_dev, int N, int K, int lda, const Status* st, cudaStream_t s, int per_sm) {
     const int64_t tiles = ((M + BM - 1) / BM) * ((N + BN - 1) / BN);
     const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>(tiles, (int64_t)num_sms() * per_sm));
-    if (mode == 0) gemm_nn_kernel<0, BM, BN, TM, TN><<<blocks, 256, 0, s>>>(A, B, bias, C, C2, Z, M, m_dev, N, K, st);
-    else if (mode == 1) gemm_nn_kernel<1, BM, BN, TM, TN><<<blocks, 256, 0, s>>>(A, B, bias, C, C2, Z, M, m_dev, N, K, st);
-    else gemm_nn_kernel<2, BM, BN, TM, TN><<<blocks, 256, 0, s>>>(A, B, bias, C, C2, Z, M, m_dev, N, K, st);
+    if (mode == 0) gemm_nn_kernel<0, BM, BN, TM, TN><<<blocks, 256, 0, s>>>(A, B, bias, C, C2, Z, M, m_dev, N, K, lda, st);
+    else if (mode == 1) gemm_nn_kernel<1, BM, BN, TM, TN><<<blocks, 256, 0, s>>>(A, B, bias, C, C2, Z, M, m_dev, N, K, lda, st);
+    else gemm_nn_kernel<2, BM, BN, TM, TN><<<blocks, 256, 0, s>>>(A, B, bias, C, C2, Z, M, m_dev, N, K, lda, st);
     MLFF_LAUNCH_CHECK("gemm_nn");
     return MLFF_OK;
 }
@@ -343,32 +346,34 @@ int launch_nn(int mode, const float* A, const float* B, const float* bias, float
 }  // namespace
 
 int gemm_nn(int mode, const float* A, const float* B, const float* bias, float* C, float* C2, const float* Z,
-            int64_t M, const int32_t* m_dev, int N, int K, const Status* st, cudaStream_t s) {
+            int64_t M, const int32_t* m_dev, int N, int K, const Status* st, cudaStream_t s, int lda) {
     ProfScope prof(PK_PLAIN_GEMM, s);
-    // The largest tile that still gives every SM two of them: 128 x 128 keeps
-    // the FP32 pipes busiest, small row counts need the tiles more.
+    if (lda == 0) lda = K;
+    // The largest tile that still gives every SM two of them (64 x 64: one):
+    // 128 x 128 keeps the FP32 pipes busiest, small row counts need the tiles
+    // more.
     auto tiles = [&](int bm, int bn) { return ((M + bm - 1) / bm) * ((N + bn - 1) / bn); };
     const int64_t want = 2LL * num_sms();
     if (N > 64 && tiles(128, 128) >= want)
-        return launch_nn<128, 128, 8, 8>(mode, A, B, bias, C, C2, Z, M, m_dev, N, K, st, s, 2);
-    if (tiles(64, 64) >= want) return launch_nn<64, 64, 4, 4>(mode, A, B, bias, C, C2, Z, M, m_dev, N, K, st, s, 6);
-    return launch_nn<32, 32, 2, 2>(mode, A, B, bias, C, C2, Z, M, m_dev, N, K, st, s, 8);
+        return launch_nn<128, 128, 8, 8>(mode, A, B, bias, C, C2, Z, M, m_dev, N, K, lda, st, s, 2);
+    if (2 * tiles(64, 64) >= want) return launch_nn<64, 64, 4, 4>(mode, A, B, bias, C, C2, Z, M, m_dev, N, K, lda, st, s, 6);
+    return launch_nn<32, 32, 2, 2>(mode, A, B, bias, C, C2, Z, M, m_dev, N, K, lda, st, s, 8);
 }
 
 size_t gemm_tn_floats(int64_t M, int64_t N) { return (size_t)tn_splits(M, N) * (size_t)(M * N + M); }
 
-int gemm_tn(const float* A, int lda, const float* B, int ldb, int M, int N, int64_t rows, const int32_t* n_dev,
-            float* C, float* colsum, float* part, const Status* st, cudaStream_t s) {
+int gemm_tn(const GemmRows& x, int lda, int ldb, int M, int N, int64_t rows, float* C, float* colsum,
+            bool accumulate, float* part, const Status* st, cudaStream_t s) {
     ProfScope prof(PK_PLAIN_GEMM, s);
-    int ns = tn_splits(M, N);
-    // (a split holds at least TN_MIN_ROWS rows)
-    ns = (int)std::max<int64_t>(1, std::min<int64_t>(ns, (rows + TN_MIN_ROWS - 1) / TN_MIN_ROWS));
+    // a split holds at least TN_MIN_ROWS rows; two sets of rows take half of the splits each
+    int ns = (int)std::max<int64_t>(1, std::min<int64_t>(tn_splits(M, N), (rows + TN_MIN_ROWS - 1) / TN_MIN_ROWS));
+    if (x.A1) ns = 2 * std::max(1, ns / 2);
     dim3 grid(tn_tiles(M) * tn_tiles(N), ns);
-    gemm_tn_kernel<<<grid, 256, 0, s>>>(A, lda, B, ldb, M, N, rows, n_dev, ns, colsum != nullptr, part, st);
+    gemm_tn_kernel<<<grid, 256, 0, s>>>(x, lda, ldb, M, N, rows, ns, colsum != nullptr, part, st);
     MLFF_LAUNCH_CHECK("gemm_tn");
     const int64_t out = (int64_t)M * N + M;
-    gemm_tn_sum_kernel<<<(int)std::min<int64_t>((out + 255) / 256, 152 * 8), 256, 0, s>>>(part, (int64_t)M * N, M, ns, C,
-                                                                                     colsum, st);
+    gemm_tn_sum_kernel<<<(int)std::min<int64_t>((out + 255) / 256, 152 * 8), 256, 0, s>>>(
+        part, (int64_t)M * N, M, ns, accumulate ? 1 : 0, C, colsum, st);
     MLFF_LAUNCH_CHECK("gemm_tn_sum");
     return MLFF_OK;
 }

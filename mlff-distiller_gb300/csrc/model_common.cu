@@ -66,6 +66,7 @@ PackedOffsets packed_offsets(const mlff_dims& d) {
         L.w2q_tc = take(2 * H * H / 2);
     }
     o.tab = take(d.n_layers * TAB_LAYER);
+    o.tab_node = take(d.n_layers * TAB_NODE_LAYER);
     o.tab_err = take((int64_t)d.n_layers * TAB_NI * 4 * 2);
     o.tab_flag = take(1);
     o.total = p;

@@ -478,9 +478,9 @@ int mlff_painn_message_backward(int32_t hidden, int32_t n_rbf, int32_t n_atoms, 
     if ((r = plain_sgemm(2, gf, w2, nullptr, gz, nullptr, z, E, (int)H, (int)(3 * H), sw, st))) return r;
     if ((r = plain_sgemm(0, gz, w1, nullptr, grad_rbf, nullptr, nullptr, E, (int)R, (int)H, sw, st))) return r;
     // parameter gradients: W2 = gf^T h, W1 = gz^T rbf, biases = column sums
-    if ((r = gemm_tn(gf, (int)(3 * H), h, (int)H, (int)(3 * H), (int)H, E, nullptr, grad_w2, grad_b2, part, sw, st)))
+    if ((r = gemm_tn({gf, h}, (int)(3 * H), (int)H, (int)(3 * H), (int)H, E, grad_w2, grad_b2, false, part, sw, st)))
         return r;
-    if ((r = gemm_tn(gz, (int)H, edge_rbf, (int)R, (int)H, (int)R, E, nullptr, grad_w1, grad_b1, part, sw, st)))
+    if ((r = gemm_tn({gz, edge_rbf}, (int)H, (int)R, (int)H, (int)R, E, grad_w1, grad_b1, false, part, sw, st)))
         return r;
     MLFF_CUDA(cudaMemcpyAsync(status, sw, 4 * sizeof(int32_t), cudaMemcpyDeviceToDevice, st));
     return MLFF_OK;
@@ -569,9 +569,9 @@ int mlff_painn_update_backward(int32_t hidden, int32_t n_atoms, const float* sca
     if ((r = plain_sgemm(0, gz, w1, nullptr, gcomb, nullptr, nullptr, N, (int)(2 * H), (int)H, sw, st))) return r;
     MOD_LAUNCH(upd_comb_bwd_kernel, N * H, st, vector, comb, gcomb, N, (int)H, grad_scalar, grad_vector, sw);
     // parameter gradients
-    if ((r = gemm_tn(ga, (int)(3 * H), h, (int)H, (int)(3 * H), (int)H, N, nullptr, grad_w2, grad_b2, part, sw, st)))
+    if ((r = gemm_tn({ga, h}, (int)(3 * H), (int)H, (int)(3 * H), (int)H, N, grad_w2, grad_b2, false, part, sw, st)))
         return r;
-    if ((r = gemm_tn(gz, (int)H, comb, (int)(2 * H), (int)H, (int)(2 * H), N, nullptr, grad_w1, grad_b1, part, sw, st)))
+    if ((r = gemm_tn({gz, comb}, (int)H, (int)(2 * H), (int)H, (int)(2 * H), N, grad_w1, grad_b1, false, part, sw, st)))
         return r;
     return MLFF_OK;
 }

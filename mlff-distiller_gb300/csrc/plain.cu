@@ -12,6 +12,7 @@
 #include "common.cuh"
 #include "dual.cuh"
 #include "gemm.cuh"
+#include "tab.cuh"
 #include "workspace.h"
 #include "profile.h"
 
@@ -76,10 +77,10 @@ __global__ void pl_geom_kernel(const float4* __restrict__ pos4, const float* __r
                 const T diff = d - centers[q];
                 const T g = texp(-gamma[q] * diff * diff);
                 e[q] = g * fc;
-                ed[q] = g * (dfc - 2.0f * gamma[q] * diff * fc);
+                if (erbf_d) ed[q] = g * (dfc - 2.0f * gamma[q] * diff * fc);
             } else {
                 e[q] = T{};
-                ed[q] = T{};
+                if (erbf_d) ed[q] = T{};
             }
         }
     }
@@ -610,6 +611,55 @@ static int run_plain_t(const mlff_dims& d, const float* P, const PackedOffsets& 
     if constexpr (DUAL) return MLFF_OK;
     if (!out.forces && !out.virial) return MLFF_OK;
     return launch_forces(d, sys, L, ws, out, st, vf);
+}
+
+// Forward pass alone, the same kernels in the same order: X [L + 1][N][4][H]
+// component-major, Xt, uz and ua of every layer in the workspace.
+int plain_forward(const mlff_dims& d, const float* P, const PackedOffsets& po, const mlff_system& sys,
+                  const WsLayout& L, void* ws, float* X, cudaStream_t st) {
+    const int N = sys.n_atoms;
+    const int64_t NX = (int64_t)N * 4 * H, cap = L.cap;
+    const Status* status = ws_ptr<Status>(ws, L.status);
+    const int32_t *row_ptr = ws_ptr<int32_t>(ws, L.row_ptr), *E_dev = row_ptr + N, *col = ws_ptr<int32_t>(ws, L.col);
+    float4* geo = ws_ptr<float4>(ws, L.pgeo);
+    float *erbf = ws_ptr<float>(ws, L.erbf), *fz = ws_ptr<float>(ws, L.fz), *fh = ws_ptr<float>(ws, L.fh);
+    float *ff = ws_ptr<float>(ws, L.ff), *Xt = ws_ptr<float>(ws, L.Xt), *comb = ws_ptr<float>(ws, L.comb);
+    float* uh = ws_ptr<float>(ws, L.uh);
+    const int nblocks = (int)std::max<int64_t>(1, std::min<int64_t>(((int64_t)N * H + 255) / 256, 152 * 8));
+    const int rblocks = std::max(1, std::min(N, 152 * 16));
+    const float* none = nullptr;
+    int r;
+    {
+        ProfScope prof(PK_PLAIN_EDGE, st);
+        pl_geom_kernel<float><<<152 * 8, 256, 0, st>>>(ws_ptr<float4>(ws, L.pos4), nullptr, nullptr,
+                                                       ws_ptr<int32_t>(ws, L.atom_mol), sys.box, sys.pbc, row_ptr, col,
+                                                       ws_ptr<int32_t>(ws, L.erecv), N, P + po.centers, P + po.gamma,
+                                                       d.n_rbf, d.cutoff, geo, erbf, nullptr, status);
+        MLFF_LAUNCH_CHECK("pl_geom");
+    }
+    WsLayout rows = L;
+    rows.gather = GATHER_ROWS;
+    rows.X = static_cast<size_t>(reinterpret_cast<char*>(X) - static_cast<char*>(ws));
+    if ((r = launch_embed(d, P, po, sys, rows, ws, st))) return r;
+    for (int l = 0; l < d.n_layers; ++l) {
+        const LayerOffsets& lo = po.layer[l];
+        if ((r = sgemm<1>((const float*)erbf, P + lo.w1t, P + lo.b1, fz, fh, none, cap, E_dev, H, RMAX, status, st)))
+            return r;
+        if ((r = sgemm<0>((const float*)fh, P + lo.w2t, P + lo.b2, ff, (float*)nullptr, none, cap, E_dev, H3, H, status,
+                          st))) return r;
+        pl_message_kernel<float><<<rblocks, 128, 0, st>>>(X + l * NX, ff, geo, col, row_ptr, N, Xt + l * NX, status);
+        MLFF_LAUNCH_CHECK("pl_message");
+        pl_update_pre_kernel<float><<<nblocks, 256, 0, st>>>(Xt + l * NX, N, comb, status);
+        MLFF_LAUNCH_CHECK("pl_update_pre");
+        float *uzl = ws_ptr<float>(ws, L.uz) + (int64_t)l * N * H, *ual = ws_ptr<float>(ws, L.ua) + (int64_t)l * N * H3;
+        if ((r = sgemm<1>((const float*)comb, P + lo.u1t, P + lo.c1, uzl, uh, none, N, nullptr, H, 2 * H, status, st)))
+            return r;
+        if ((r = sgemm<0>((const float*)uh, P + lo.u2t, P + lo.c2, ual, (float*)nullptr, none, N, nullptr, H3, H, status,
+                          st))) return r;
+        pl_update_post_kernel<float><<<nblocks, 256, 0, st>>>(Xt + l * NX, ual, P + lo.mix, N, X + (l + 1) * NX, status);
+        MLFF_LAUNCH_CHECK("pl_update_post");
+    }
+    return MLFF_OK;
 }
 
 int run_plain(const mlff_dims& d, const float* P, const PackedOffsets& po, const mlff_system& sys,

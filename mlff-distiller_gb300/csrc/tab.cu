@@ -85,8 +85,9 @@ constexpr int TB_P = TAB_NC + 1;   // nodes and the end point t = 1
 // derivative at the end, go through shared memory as (hi, lo) floats.
 __global__ void __launch_bounds__(H) tab_build_kernel(const float* __restrict__ P, PackedOffsets po, int R,
                                                       float cutoff, NodeInverse ni, float* __restrict__ tab,
-                                                      double* __restrict__ err) {
+                                                      float* __restrict__ node, double* __restrict__ err) {
     __shared__ double e[TB_P + 1][RMAX];   // basis x cutoff at the points; its derivative at the end
+    __shared__ float en[TAB_NC][RMAX];     // its derivative at the nodes
     __shared__ float hh[TB_P + 1][H], hl[TB_P + 1][H];
     __shared__ double red[4][4];
     const int t = threadIdx.x, i = blockIdx.x, l = blockIdx.y;
@@ -102,9 +103,15 @@ __global__ void __launch_bounds__(H) tab_build_kernel(const float* __restrict__ 
         const double gm = (double)P[po.gamma + r];
         const double g = r < R ? exp(-gm * diff * diff) : 0.0;
         e[pt][r] = g * fc;
+        const double dfc = d < rc ? -0.5 * (3.14159265358979323846 / rc) * sin(arg) : 0.0;
+        const double gd = g * (dfc - 2.0 * gm * diff * fc);
         if (pt == TAB_NC) {
-            const double dfc = d < rc ? -0.5 * (3.14159265358979323846 / rc) * sin(arg) : 0.0;
-            e[TB_P][r] = g * (dfc - 2.0 * gm * diff * fc);
+            e[TB_P][r] = gd;
+        } else {
+            en[pt][r] = (float)gd;
+            float* o = node + l * TAB_NODE_LAYER + TAB_NODES * 4 * H + (int64_t)(i * TAB_NC + pt) * RMAX + r;
+            o[0] = (float)(g * fc);
+            o[TAB_NODES * RMAX] = (float)gd;
         }
     }
     __syncthreads();
@@ -122,6 +129,15 @@ __global__ void __launch_bounds__(H) tab_build_kernel(const float* __restrict__ 
             const double h = z[pt] * s;
             hh[pt][t] = (float)h;
             hl[pt][t] = (float)(h - (double)(float)h);
+            if (pt < TAB_NC) {
+                float zd = 0.f;
+                for (int r = 0; r < R; ++r) zd = fmaf(P[lo.w1t + r * H + t], en[pt][r], zd);
+                float* o = node + l * TAB_NODE_LAYER + (int64_t)(i * TAB_NC + pt) * H + t;
+                o[0] = (float)z[pt];
+                o[TAB_NODES * H] = (float)h;
+                o[2 * TAB_NODES * H] = zd;
+                o[3 * TAB_NODES * H] = dsilu_f((float)z[pt]) * zd;
+            }
             if (pt == TAB_NC) {
                 const double hd = s * (1.0 + z[pt] * (1.0 - s)) * z[TB_P];
                 hh[TB_P][t] = (float)hd;
@@ -204,11 +220,21 @@ static_assert(TAB_NI <= 128, "one thread per interval");
 int build_tables(const mlff_dims& d, float* packed, const PackedOffsets& po, cudaStream_t st) {
     double* err = reinterpret_cast<double*>(packed + po.tab_err);
     tab_build_kernel<<<dim3(TAB_NI, d.n_layers), H, 0, st>>>(packed, po, d.n_rbf, d.cutoff, node_inverse(),
-                                                             packed + po.tab, err);
+                                                             packed + po.tab, packed + po.tab_node, err);
     MLFF_LAUNCH_CHECK("tab_build");
     tab_flag_kernel<<<1, 128, 0, st>>>(err, d.n_layers, reinterpret_cast<int32_t*>(packed + po.tab_flag));
     MLFF_LAUNCH_CHECK("tab_flag");
     return MLFF_OK;
+}
+
+void table_nodes(float* node, float* weight) {
+    for (int j = 0; j < TAB_NC; ++j) node[j] = (float)node_inverse().x[j];
+    for (int j = 0; j < TAB_NC; ++j) {
+        double w = 1.0;
+        for (int m = 0; m < TAB_NC; ++m)
+            if (m != j) w *= node_inverse().x[j] - node_inverse().x[m];
+        weight[j] = (float)(1.0 / w);
+    }
 }
 
 int read_table_flag(const float* packed, const PackedOffsets& po, int32_t* flag, cudaStream_t st) {
@@ -226,16 +252,6 @@ namespace {
 // order for every G, so results do not depend on it.  One warp per group,
 // a stable counting sort over the intervals in shared memory; a group of up
 // to 256 edges keeps its geometry in registers between the two passes.
-struct __align__(16) TabRec {
-    float t, t2;      // local coordinate, twice (an operand pair)
-    float uy, uz;
-    float ux;
-    int32_t sender;
-    int32_t off;      // byte offset of the interval's row in a table slice
-    int32_t r;        // receiver within the group
-};
-static_assert(sizeof(TabRec) == 32, "two 16-byte loads");
-
 constexpr int REC_WARPS = 4;
 constexpr int REC_REG = 8;    // chunks of 32 edges kept in registers
 
@@ -398,171 +414,6 @@ struct TabArgs {
     int eacc_init;         // reverse: 1 = part is written, 0 = added to
     Status* st;
 };
-
-// The 18 coefficients of one channel: pairs (phi_s, phi_v1) and phi_v2.
-struct Coef {
-    f32x2 sa[TAB_NC];
-    float b[TAB_NC];
-    template <bool SMEM>
-    __device__ __forceinline__ void load(const char* table, int off, int lane) {
-        const float4* q = reinterpret_cast<const float4*>(table + off) + lane;
-        const float2* q2 = reinterpret_cast<const float2*>(table + off + 2048) + lane;
-        float4 v[4];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) v[j] = SMEM ? q[32 * j] : __ldg(q + 32 * j);
-        const float2 w = SMEM ? *q2 : __ldg(q2);
-#pragma unroll
-        for (int j = 0; j < 3; ++j) {
-            sa[2 * j] = pack2(v[j].x, v[j].y);
-            sa[2 * j + 1] = pack2(v[j].z, v[j].w);
-        }
-        b[0] = v[3].x; b[1] = v[3].y; b[2] = v[3].z; b[3] = v[3].w;
-        b[4] = w.x; b[5] = w.y;
-    }
-};
-
-__device__ __forceinline__ float poly(const float (&c)[TAB_NC], float t) {
-    return fmaf(fmaf(fmaf(fmaf(fmaf(c[5], t, c[4]), t, c[3]), t, c[2]), t, c[1]), t, c[0]);
-}
-// value and d/dt
-__device__ __forceinline__ void poly_d(const float (&c)[TAB_NC], float t, float& f, float& fd) {
-    float p = c[5], q = c[5];
-    p = fmaf(p, t, c[4]);
-#pragma unroll
-    for (int k = 3; k >= 0; --k) {
-        q = fmaf(q, t, p);
-        p = fmaf(p, t, c[k]);
-    }
-    f = p;
-    fd = q;
-}
-__device__ __forceinline__ f32x2 poly(const f32x2 (&c)[TAB_NC], f32x2 t) {
-    f32x2 p = c[5];
-#pragma unroll
-    for (int k = 4; k >= 0; --k) p = fma2(p, t, c[k]);
-    return p;
-}
-__device__ __forceinline__ void poly_d(const f32x2 (&c)[TAB_NC], f32x2 t, f32x2& f, f32x2& fd) {
-    f32x2 p = c[5], q = c[5];
-    p = fma2(p, t, c[4]);
-#pragma unroll
-    for (int k = 3; k >= 0; --k) {
-        q = fma2(q, t, p);
-        p = fma2(p, t, c[k]);
-    }
-    f = p;
-    fd = q;
-}
-
-// Records of a warp's edges staged through shared memory: chunks of 4 (128
-// bytes), a ring of 4, two chunks ahead.
-constexpr int RING = 4;
-constexpr int RING_BYTES = RING * 4 * (int)sizeof(TabRec);
-struct RecRing {
-    unsigned char* buf;
-    const TabRec* src;      // the group's first record
-    int lane;
-    __device__ __forceinline__ void stage(int k) const {
-        if (lane < 8)
-            tc::cp_async16(buf + (k & (RING - 1)) * 128 + lane * 16,
-                           reinterpret_cast<const unsigned char*>(src + 4 * k) + lane * 16);
-        tc::cp_async_commit();
-    }
-    // all but the last staged chunk have landed, for every lane
-    __device__ __forceinline__ void ready() const {
-        asm volatile("cp.async.wait_group 1;" ::: "memory");
-        __syncwarp();
-    }
-    __device__ __forceinline__ const TabRec* at(int k, int u) const {
-        return reinterpret_cast<const TabRec*>(buf + (k & (RING - 1)) * 128) + u;
-    }
-};
-
-constexpr int FWD_NT = 640, BWD_NT = 512, SMALL_NT = 128;   // threads per CTA (small: table read from memory)
-constexpr uint32_t TAB_SLICE_BYTES = TAB_SLICE * 4;      // 221,184
-constexpr uint32_t TAB_RING = TAB_SLICE_BYTES + 64;       // behind the barrier, group range and counter
-__host__ __device__ constexpr uint32_t tab_smem(int nt) { return TAB_RING + nt / 32 * RING_BYTES; }
-static_assert(tab_smem(FWD_NT) <= 232448, "table slice and record rings in shared memory");
-
-// The CTA's table slice into shared memory (one bulk copy of packed weights,
-// before the wait for the previous kernel).
-__device__ __forceinline__ uint64_t* tab_stage(unsigned char* smem, const float* tab, int slice) {
-    uint64_t* bar = reinterpret_cast<uint64_t*>(smem + TAB_SLICE_BYTES);
-    if (threadIdx.x == 0) {
-        tc::mbar_init(bar, 1);
-        tc::fence_mbar_init();
-        tc::mbar_expect_tx(bar, TAB_SLICE_BYTES);
-        const char* src = reinterpret_cast<const char*>(tab + slice * TAB_SLICE);
-        constexpr uint32_t CH = TAB_SLICE_BYTES / 12;
-        static_assert(CH % 16 == 0 && CH * 12 == TAB_SLICE_BYTES, "copy chunks");
-#pragma unroll 1
-        for (int i = 0; i < 12; ++i) tc::bulk_g2s(smem + i * CH, src + i * CH, CH, bar);
-    }
-    return bar;
-}
-
-// first group whose edges start at or after share p of nparts
-__device__ __forceinline__ int group_bound(const int32_t* row_ptr, int n_atoms, int G, int ngroups, int p, int nparts) {
-    if (p <= 0) return 0;
-    if (p >= nparts) return ngroups;
-    const int64_t target = ((int64_t)row_ptr[n_atoms] * p + nparts - 1) / nparts;
-    int lo = 0, hi = ngroups;
-    while (lo < hi) {
-        const int mid = (lo + hi) >> 1;
-        if (row_ptr[min(mid * G, n_atoms)] >= target) hi = mid;
-        else lo = mid + 1;
-    }
-    return lo;
-}
-
-// Walks the groups of this CTA (SMEM: its share of the groups of slice
-// blockIdx.x % 4, handed to the warps one by one; otherwise one group and
-// slice per warp) and calls body(group, slice).
-template <bool SMEM, class F>
-__device__ __forceinline__ void for_groups(const TabArgs& a, int G, unsigned char* smem, F&& body) {
-    const int ngroups = (a.n_atoms + G - 1) / G;
-    const int lane = threadIdx.x & 31;
-    if constexpr (SMEM) {
-        const int slice = blockIdx.x & 3;
-        uint64_t* bar = tab_stage(smem, a.tab, slice);
-        int* range = reinterpret_cast<int*>(smem + TAB_SLICE_BYTES + 16);   // first, end, next
-        pdl_wait();
-        const bool dead = a.st->code != 0;
-        if (!dead) {
-            if ((threadIdx.x & 31) == 0 && threadIdx.x < 64) {
-                const int p = (blockIdx.x >> 2) + (threadIdx.x >> 5);
-                range[threadIdx.x >> 5] = group_bound(a.row_ptr, a.n_atoms, G, ngroups, p, gridDim.x >> 2);
-            }
-        }
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            range[2] = dead ? ngroups : range[0];
-            // (also before returning: the copy must have landed when the CTA exits)
-            if (!tc::mbar_wait(bar, 0, tc::WAIT_BUDGET)) {
-                set_status(a.st, MLFF_ERR_TIMEOUT, 50);
-                range[2] = ngroups;
-                tc::mbar_wait(bar, 0, tc::WAIT_BUDGET);   // no copy in flight past the CTA's end
-            }
-        }
-        __syncthreads();
-        pdl_trigger();
-        if (dead) return;
-        const int end = range[1];
-        while (true) {
-            int g = 0;
-            if (lane == 0) g = atomicAdd(range + 2, 1);
-            g = __shfl_sync(0xffffffffu, g, 0);
-            if (g >= end) break;
-            body(g, slice);
-        }
-    } else {
-        pdl_wait();
-        pdl_trigger();
-        if (a.st->code != 0) return;
-        const int nw = (gridDim.x * blockDim.x) >> 5;
-        for (int k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; k < 4 * ngroups; k += nw) body(k >> 2, k & 3);
-    }
-}
 
 template <int G, bool SMEM, bool L0, int NT>
 __global__ void __launch_bounds__(NT, SMEM ? 1 : 4) tab_fwd_kernel(TabArgs a) {
@@ -848,22 +699,6 @@ __global__ void __launch_bounds__(256) tab_combine_kernel(const float4* __restri
 }
 
 // ------------------------------------------------------------- launchers
-// Grid and dynamic shared memory of a table kernel: one CTA per SM and
-// slice share with the table staged, else a warp per group and slice.
-template <int G, bool SMEM, int NT>
-struct TabLaunch {
-    static constexpr uint32_t SM = SMEM ? tab_smem(NT) : NT / 32 * RING_BYTES;
-    static int grid(int n_atoms) {
-        return SMEM ? std::max(4, num_sms() & ~3) : (4 * ((n_atoms + G - 1) / G) + NT / 32 - 1) / (NT / 32);
-    }
-    template <class K>
-    static int prepare(K* kernel) {
-        if (!SMEM) return MLFF_OK;
-        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SM);
-        return e == cudaSuccess ? MLFF_OK : cuda_status(e, "table kernel smem attribute");
-    }
-};
-
 template <int G, bool SMEM, bool L0>
 int launch_fwd_t(const TabArgs& a, cudaStream_t st) {
     constexpr int NT = SMEM ? FWD_NT : SMALL_NT;
@@ -885,17 +720,6 @@ int launch_bwd_t(const TabArgs& a, float scale, cudaStream_t st) {
     if (err) return err;
     MLFF_LAUNCH_PDL("tab_bwd", (tab_bwd_kernel<G, SMEM, L0, PAIRS, NT>), TL::grid(a.n_atoms), NT, TL::SM, st, a, scale);
     return MLFF_OK;
-}
-
-// Receivers per group and where the table is read from.
-struct TabShape {
-    int G;
-    bool smem;
-};
-TabShape tab_shape(int n_atoms) {
-    if (n_atoms >= 4096) return {4, true};
-    if (n_atoms >= 1500) return {2, true};
-    return {1, false};
 }
 
 template <bool L0>
@@ -926,6 +750,8 @@ TabArgs tab_args(const WsLayout& L, void* ws) {
     return a;
 }
 
+}  // namespace
+
 int launch_records(const mlff_dims& d, const float* P, const PackedOffsets& po, const mlff_system& sys,
                    const WsLayout& L, void* ws, int path, cudaStream_t st) {
     ProfScope prof(PK_NEIGHBORS, st);
@@ -941,11 +767,8 @@ int launch_records(const mlff_dims& d, const float* P, const PackedOffsets& po, 
     return MLFF_OK;
 }
 
-}  // namespace
-
-// The FP32 path with tabulated filters (MLFF_PATH_TABLE_FP32).
-int run_table(const mlff_dims& d, const float* P, const PackedOffsets& po, const mlff_system& sys, const WsLayout& L,
-              void* ws, const mlff_outputs& out, int path, cudaStream_t st, const VerletFuse* vf) {
+int table_forward(const mlff_dims& d, const float* P, const PackedOffsets& po, const mlff_system& sys,
+                  const WsLayout& L, void* ws, int path, cudaStream_t st) {
     const int64_t NX = (int64_t)L.N * 4 * H;
     const TabShape shape = tab_shape(L.N);
     int r;
@@ -962,6 +785,14 @@ int run_table(const mlff_dims& d, const float* P, const PackedOffsets& po, const
         }
         if ((r = launch_upd32_fwd(P, po.layer[l], L, ws, l, st))) return r;
     }
+    return MLFF_OK;
+}
+
+// The FP32 path with tabulated filters (MLFF_PATH_TABLE_FP32).
+int run_table(const mlff_dims& d, const float* P, const PackedOffsets& po, const mlff_system& sys, const WsLayout& L,
+              void* ws, const mlff_outputs& out, int path, cudaStream_t st, const VerletFuse* vf) {
+    int r = table_forward(d, P, po, sys, L, ws, path, st);
+    if (r) return r;
     const bool want_grad = out.forces != nullptr || out.virial != nullptr;
     if ((r = launch_readout(d, P, po, sys, L, ws, out, want_grad ? 1 : 0, st))) return r;
     if (!want_grad) return MLFF_OK;

@@ -38,6 +38,15 @@ __host__ __device__ constexpr int tab_off(int lane, int g, int k) {
                                 : 512 + lane * 2 + (tab_index(g, k) - 16);
 }
 
+// The network at the intervals' nodes (row interval * TAB_NC + node), for the
+// weight gradients: per layer z = W1 e + b1, h = silu(z) and their
+// d-derivatives z', h' [nodes][H], the basis rows e and e' [nodes][RMAX].
+constexpr int64_t TAB_NODES = (int64_t)TAB_NI * TAB_NC;
+constexpr int64_t TAB_NODE_LAYER = TAB_NODES * (4 * H + 2 * RMAX);
+
+// training: edges per segment of the counting sort and per partial sum
+constexpr int TT_SEG = 256, TT_CHUNK = 64;
+
 // Edge records are read in chunks of 4, up to TREC_PAD past the last edge.
 constexpr int TREC_PAD = 16;
 
@@ -46,6 +55,23 @@ constexpr int TREC_PAD = 16;
 __host__ __device__ constexpr int quad_off(int comp, int c) { return 4 * c + comp; }
 
 int build_tables(const mlff_dims& d, float* packed, const PackedOffsets& po, cudaStream_t st);
+void table_nodes(float* node, float* weight);   // Chebyshev nodes, 1 / prod_{m != j} (node_j - node_m)
+int launch_records(const mlff_dims& d, const float* P, const PackedOffsets& po, const mlff_system& sys,
+                   const WsLayout& L, void* ws, int path, cudaStream_t st);
+// forward pass of the plain FP32 path; X [L + 1][N][4][H] component-major
+int plain_forward(const mlff_dims& d, const float* P, const PackedOffsets& po, const mlff_system& sys,
+                  const WsLayout& L, void* ws, float* X, cudaStream_t st);
+// forward pass with the tables: records, X, Xt, uz, ua of every layer
+int table_forward(const mlff_dims& d, const float* P, const PackedOffsets& po, const mlff_system& sys,
+                  const WsLayout& L, void* ws, int path, cudaStream_t st);
+// training (train_tab.cu): offsets of its arrays from p on; returns the end
+size_t train_table_workspace(WsLayout& L, const mlff_dims& d, size_t p);
+struct GradCtx;
+int run_train_table(const mlff_dims& d, const float* P, const PackedOffsets& po, const mlff_system& sys,
+                    const WsLayout& L, void* ws, double* energy, cudaStream_t st, const GradCtx& grad);
+int run_train_table_tangent(const mlff_dims& d, const float* P, const PackedOffsets& po, const mlff_system& sys,
+                            const WsLayout& L, void* ws, cudaStream_t st, const GradCtx& grad, const float* G,
+                            const double* S);
 int read_table_flag(const float* packed, const PackedOffsets& po, int32_t* flag, cudaStream_t st);
 
 }  // namespace mlff

@@ -58,6 +58,21 @@ struct WsLayout {
     size_t trec;               // TabRec [cap + TREC_PAD], 32 bytes each
     size_t tperm;              // int32 [cap] sorted position -> edge
     size_t tpart;              // float4 [4][cap] (dE/dd, dE/du) of each 32-channel slice
+    // training through the tables (train_tab.cu); planes: value, tangent
+    size_t txtbar;             // float4 [2][N][H] dE/dXt quads
+    size_t thb;                // float [2][N][H] adjoint of the update MLP's hidden layer
+    size_t tcb;                // float [2][N][2H] adjoint of its input
+    size_t tgeo_t;             // float4 [cap] (u', t')
+    size_t trec_t;             // float4 [cap + TREC_PAD] the same in the records' order
+    size_t tkey;               // int32 [cap] interval of each edge
+    size_t torder;             // int32 [cap] edges sorted by interval
+    size_t toffs, tscan;       // int32 [intervals][segments] offsets of the sort; scan scratch
+    size_t tcst;               // int32 [intervals + 1] first partial sum of each interval
+    size_t thead;              // float: activations and adjoints of the energy head
+    size_t tadj;               // float [partial sums][18][H]
+    size_t prows, pgeo;        // plain forward pass of the force term: X rows, geometry
+    size_t tnode;              // float [nodes][3H], [nodes][H]
+    size_t temb;               // float: partial embedding gradients
     size_t erbf;               // float [cap][RMAX]
     size_t erbf_d;             // float [cap][RMAX]
     size_t fz;                 // float [L][cap][H]
@@ -135,7 +150,7 @@ int launch_forces(const mlff_dims& d, const mlff_system& sys, const WsLayout& L,
                   const mlff_outputs& out, cudaStream_t st, const VerletFuse* vf = nullptr);
 // Training: per-structure loss weights dL/dE_b and the gradient outputs.
 struct GradCtx {
-    const double* w;
+    const double* w;     // NULL: unit weights
     mlff_grads g;
 };
 int run_plain(const mlff_dims& d, const float* packed, const PackedOffsets& po,

@@ -31,6 +31,7 @@ PATH_TRAIN = 3
 PATH_TRAIN_FORCES = 4
 PATH_TABLE = 5
 PATH_TABLE_FP32 = 6
+PATH_TRAIN_TABLE = 7
 
 PATHS = {"plain": PATH_PLAIN_FP32, "fp32": PATH_PLAIN_FP32, "plain_fp32": PATH_PLAIN_FP32,
          "fp16x3": PATH_TUNED_TC, "tc": PATH_TUNED_TC, "tuned": PATH_TUNED_TC,
@@ -52,7 +53,8 @@ EXPORTS = ["mlff_version", "mlff_last_error_string", "mlff_packed_weights_size",
            "mlff_painn_message_backward", "mlff_painn_update_workspace_size", "mlff_painn_update",
            "mlff_painn_update_backward", "mlff_force_stats_workspace_size", "mlff_force_stats",
            "mlff_autotune", "mlff_autotune_query", "mlff_autotune_set", "mlff_autotune_query_shape",
-           "mlff_autotune_set_shape", "mlff_autotune_reset", "mlff_filter_table_class"]
+           "mlff_autotune_set_shape", "mlff_autotune_reset", "mlff_filter_table_class",
+           "mlff_param_grads_table", "mlff_param_grads_forces_table"]
 
 PROFILE_KINDS = ["neighbors", "edge_fwd", "edge_bwd", "update_fwd", "update_bwd", "readout", "forces",
                  "plain_gemm", "plain_edge", "other", "md", "edge_bwd_q"]
@@ -179,6 +181,12 @@ def load(build_if_missing: bool = True):
         lib.mlff_param_grads_forces.restype = ctypes.c_int
         lib.mlff_param_grads_forces.argtypes = [ctypes.POINTER(Dims), _P, ctypes.POINTER(System), i64, _P, _P,
                                                 ctypes.POINTER(Grads), _P, sz, _P]
+        lib.mlff_param_grads_table.restype = ctypes.c_int
+        lib.mlff_param_grads_table.argtypes = [ctypes.POINTER(Dims), _P, ctypes.POINTER(System), i64, _P,
+                                               ctypes.POINTER(Grads), _P, _P, sz, _P]
+        lib.mlff_param_grads_forces_table.restype = ctypes.c_int
+        lib.mlff_param_grads_forces_table.argtypes = [ctypes.POINTER(Dims), _P, ctypes.POINTER(System), i64, _P, _P,
+                                                      ctypes.POINTER(Grads), _P, sz, _P]
         lib.mlff_painn_message_workspace_size.restype = sz
         lib.mlff_painn_message_workspace_size.argtypes = [i32, i32, i64, i32]
         lib.mlff_painn_message.restype = ctypes.c_int

@@ -59,6 +59,12 @@ def _grads_struct(model, grads: Dict[str, torch.Tensor]):
     return g
 
 
+def _use_table(eng) -> bool:
+    """The passes through the tabulated filters serve weights whose tables
+    are as accurate as the FP32 network evaluation."""
+    return eng.route(_lib.PATH_TUNED_FP32) == _lib.PATH_TABLE_FP32
+
+
 def param_grads(model, batch: Batch, weights: torch.Tensor, forces: bool = False,
                 force_weights: Optional[torch.Tensor] = None, virial_weights: Optional[torch.Tensor] = None
                 ) -> Tuple[torch.Tensor, Dict[str, torch.Tensor], Optional[torch.Tensor]]:
@@ -95,13 +101,19 @@ def param_grads(model, batch: Batch, weights: torch.Tensor, forces: bool = False
     sysd = batch.system()
     path = _lib.PATH_TRAIN
     second = G is not None or S is not None
-    ws_path = _lib.PATH_TRAIN_FORCES if second else _lib.PATH_TRAIN
+    table = _use_table(eng) and not forces
+    ws_path = _lib.PATH_TRAIN_TABLE if table else _lib.PATH_TRAIN_FORCES if second else _lib.PATH_TRAIN
     for _ in range(4):
         cap = eng.capacity(N, path)
         ws = eng.workspace_for(N, B, cap, ws_path)
-        _lib.check(eng.lib.mlff_param_grads(ctypes.byref(eng.dims), eng.packed.data_ptr(), ctypes.byref(sysd), cap,
-                                            w.data_ptr(), ctypes.byref(g), ctypes.byref(out), ws.data_ptr(),
-                                            ws.numel(), _stream_handle()))
+        if table:
+            _lib.check(eng.lib.mlff_param_grads_table(ctypes.byref(eng.dims), eng.packed.data_ptr(),
+                                                      ctypes.byref(sysd), cap, w.data_ptr(), ctypes.byref(g),
+                                                      E.data_ptr(), ws.data_ptr(), ws.numel(), _stream_handle()))
+        else:
+            _lib.check(eng.lib.mlff_param_grads(ctypes.byref(eng.dims), eng.packed.data_ptr(), ctypes.byref(sysd),
+                                                cap, w.data_ptr(), ctypes.byref(g), ctypes.byref(out), ws.data_ptr(),
+                                                ws.numel(), _stream_handle()))
         code, n_edges, where = eng.status()
         if code == _lib.ERR_CAPACITY:
             eng.edge_capacity[path] = int(n_edges * 1.25) + 1024
@@ -114,9 +126,9 @@ def param_grads(model, batch: Batch, weights: torch.Tensor, forces: bool = False
         raise _lib.MLFFError(_lib.ERR_CAPACITY, "edge capacity did not converge")
     if second:
         # same structures, same capacity: the edge list fits
-        _lib.check(eng.lib.mlff_param_grads_forces(ctypes.byref(eng.dims), eng.packed.data_ptr(), ctypes.byref(sysd),
-                                                   cap, _lib.ptr(G), _lib.ptr(S), ctypes.byref(g), ws.data_ptr(),
-                                                   ws.numel(), _stream_handle()))
+        fn = eng.lib.mlff_param_grads_forces_table if table else eng.lib.mlff_param_grads_forces
+        _lib.check(fn(ctypes.byref(eng.dims), eng.packed.data_ptr(), ctypes.byref(sysd), cap, _lib.ptr(G),
+                      _lib.ptr(S), ctypes.byref(g), ws.data_ptr(), ws.numel(), _stream_handle()))
         code, _, where = eng.status()
         if code != _lib.OK:
             raise _lib.MLFFError(code, f"device status {code} at index {where}")
@@ -146,12 +158,13 @@ def force_term_grads(model, batch: Batch, force_weights: torch.Tensor,
     g = _grads_struct(model, grads)
     sysd = batch.system()
     path = _lib.PATH_TRAIN
+    table = _use_table(eng)
+    fn = eng.lib.mlff_param_grads_forces_table if table else eng.lib.mlff_param_grads_forces
     for _ in range(4):
         cap = eng.capacity(N, path)
-        ws = eng.workspace_for(N, B, cap, _lib.PATH_TRAIN_FORCES)
-        _lib.check(eng.lib.mlff_param_grads_forces(ctypes.byref(eng.dims), eng.packed.data_ptr(), ctypes.byref(sysd),
-                                                   cap, _lib.ptr(G), _lib.ptr(S), ctypes.byref(g), ws.data_ptr(),
-                                                   ws.numel(), _stream_handle()))
+        ws = eng.workspace_for(N, B, cap, _lib.PATH_TRAIN_TABLE if table else _lib.PATH_TRAIN_FORCES)
+        _lib.check(fn(ctypes.byref(eng.dims), eng.packed.data_ptr(), ctypes.byref(sysd), cap, _lib.ptr(G),
+                      _lib.ptr(S), ctypes.byref(g), ws.data_ptr(), ws.numel(), _stream_handle()))
         code, n_edges, where = eng.status()
         if code == _lib.ERR_CAPACITY:
             eng.edge_capacity[path] = int(n_edges * 1.25) + 1024

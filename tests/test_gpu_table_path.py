@@ -124,3 +124,36 @@ def test_accuracy_class_and_fallback(weights_bias):
     E0, F0, _ = eng.energy_forces(b, _lib.PATH_TUNED_TC, graph=False)
     np.testing.assert_array_equal(E.cpu().numpy(), E0.cpu().numpy())
     np.testing.assert_array_equal(F.cpu().numpy(), F0.cpu().numpy())
+
+
+@pytest.mark.parametrize("name", ["isolated", "molecules1", "molecules7", "box1499", "box1503", "box4097"])
+def test_table_gradients_match_the_plain_path(weights_bias, name):
+    """Energy and force / stress gradient terms through the tables against
+    the plain FP32 path.  Both are FP32: against float64 the plain path's
+    energy term is off by up to 2e-6 and its force term by up to 2e-5
+    (2-norm per tensor); asked of the two together 1e-5 and 5e-5."""
+    from mlff_gb300.training import force_term_grads, param_grads
+    s = system(name)
+    m = model(weights_bias, "tuned_fp32")
+    b = batch_of(s)
+    g = torch.Generator(device="cuda").manual_seed(8)
+    w = torch.randn(b.n_mol, device="cuda", generator=g, dtype=torch.float64)
+    G = torch.randn(b.n_atoms, 3, device="cuda", generator=g)
+    S = torch.randn(b.n_mol, 3, 3, device="cuda", generator=g, dtype=torch.float64) if b.box is not None else None
+    eng = m.engine()
+    got = [param_grads(m, b, w)[:2], (None, force_term_grads(m, b, G, S))]
+    again = force_term_grads(m, b, G, S)
+    assert all(torch.equal(again[k], v) for k, v in got[1][1].items())
+    cls, eng.table_class = eng.table_class, 0
+    try:
+        want = [param_grads(m, b, w)[:2], (None, force_term_grads(m, b, G, S))]
+    finally:
+        eng.table_class = cls
+    assert float(((got[0][0] - want[0][0]).abs().cpu() / torch.tensor(np.diff(s.mol_ptr))).max()) < 2e-5
+    for (_, a), (_, e), tol in zip(got, want, (1e-5, 5e-5)):
+        for k in e:
+            n = float(e[k].double().norm())
+            d = float((a[k].double() - e[k].double()).norm())
+            # a tensor whose gradient cancels is held to the scale of the others
+            floor = 1e-3 * max(float(x.double().norm()) for x in e.values())
+            assert d <= tol * max(n, floor), (k, d, n)
