@@ -1,20 +1,27 @@
 // FP32 GEMMs on the CUDA cores.
 //
 // They serve what has to stay FP32: the per-op path, the per-block entry
-// points and the weight gradients.  Bound by the FP32 pipes at large row
-// counts (8 x 8 outputs per thread: 4 shared-memory loads per 64 fused
-// multiply-adds) and by the number of tiles at small ones.  The A^T B sums
-// have few output tiles (12 of 64 x 64 for a 384 x 128 gradient) over many
-// rows, so the rows are split until every SM has four blocks; without the
-// split the message block of width 128 on 106,000 edges spent 75 of its
-// 102 ms there and 28 ms in column sums, which now ride along with the tiles
-// of output column 0 (forward + backward 2.9 ms; the width-64 update block on
-// 5,001 atoms 2.33 -> 0.42 ms).  Activations times weights: 64 x 64 tiles of
-// 4 x 4 outputs without load prefetch took 5.10 ms per call of the FP32 path
-// on 37 molecules, these tiles 3.45 ms.
+// points and the weight gradients.
+//
+// Activations times weights on 16-byte aligned rows (gemm_nn_vec_kernel):
+// tiles streamed to shared memory by a three-stage cp.async ring, packed fused
+// multiply-adds (half the issue slots).  Bound by the FP32 pipes (50 of 74
+// TFLOP/s at 8 x 8 outputs per thread): a 145,000 x 128 x 384 product 354 ->
+// 277 us against tiles fetched through registers, the FP32 path on 37
+// molecules 3.45 -> 2.70 ms a call.  An output's products are summed in the
+// order of k in every kernel here, so the choice never changes a bit.
+// Other layouts keep the kernel with scalar fallbacks (gemm_nn_kernel).
+//
+// The A^T B sums have few output tiles (12 of 64 x 64 for a 384 x 128
+// gradient) over many rows, so the rows are split until every SM has four
+// blocks; without the split the message block of width 128 on 106,000 edges
+// spent 75 of its 102 ms there and 28 ms in column sums, which now ride along
+// with the tiles of output column 0.
 #include <algorithm>
+#include "f32x2.cuh"
 #include "gemm.cuh"
 #include "profile.h"
+#include "tc_ptx.cuh"
 
 namespace mlff {
 
@@ -65,15 +72,17 @@ struct Tile {
 
 __host__ __device__ inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
-// (two blocks per SM for 8 x 8 outputs per thread, four for 4 x 4)
+// Any layout: tiles fetched through registers, the next step's loads in flight
+// during this step's arithmetic.
 template <int MODE, int BM, int BN, int TM, int TN>
-__global__ void __launch_bounds__(256, TM == 8 ? 2 : 4) gemm_nn_kernel(const float* __restrict__ A, const float* __restrict__ B,
+__global__ void __launch_bounds__(Tile<BM, BN, TM, TN>::NT, 4)
+    gemm_nn_kernel(const float* __restrict__ A, const float* __restrict__ B,
                                                       const float* __restrict__ bias, float* __restrict__ C,
                                                       float* __restrict__ C2, const float* __restrict__ Z,
                                                       int64_t M_static, const int32_t* __restrict__ m_dev, int N,
                                                       int K, int lda, const Status* st) {
     using T = Tile<BM, BN, TM, TN>;
-    static_assert(T::NT == 256, "256 threads");
+    constexpr int NT = T::NT;
     __shared__ __align__(16) float As[2][BK * T::LDA];
     __shared__ __align__(16) float Bs[2][BK * T::LDB];
     if (st->code != 0) return;
@@ -86,7 +95,7 @@ __global__ void __launch_bounds__(256, TM == 8 ? 2 : 4) gemm_nn_kernel(const flo
     const bool va = (K & 3) == 0 && (lda & 3) == 0 && aligned16(A), vb = (N & 3) == 0 && aligned16(B);
     const bool vc = T::CN == 4 && (N & 3) == 0 && aligned16(C) && (MODE != 1 || aligned16(C2)) &&
                     (MODE != 2 || aligned16(Z));
-    constexpr int LA = BM * BK / 256, LB = BN * BK / 256;   // floats per thread and step
+    constexpr int LA = BM * BK / NT, LB = BN * BK / NT;   // floats per thread and step
     static_assert(LA % 4 == 0 || LA == 2, "A loads");
     for (int64_t tile = blockIdx.x; tile < m_tiles * n_tiles; tile += gridDim.x) {
         const int64_t m0 = (tile / n_tiles) * BM;
@@ -101,7 +110,7 @@ __global__ void __launch_bounds__(256, TM == 8 ? 2 : 4) gemm_nn_kernel(const flo
             if (va && LA >= 4) {
 #pragma unroll
                 for (int q = 0; q < LA / 4; ++q) {
-                    const int i = t + 256 * q, r = i / (BK / 4), k = k0 + 4 * (i % (BK / 4));
+                    const int i = t + NT * q, r = i / (BK / 4), k = k0 + 4 * (i % (BK / 4));
                     const float4 x = (m0 + r < M && k < K) ? *reinterpret_cast<const float4*>(A + (m0 + r) * lda + k)
                                                            : make_float4(0.f, 0.f, 0.f, 0.f);
                     ra[4 * q] = x.x; ra[4 * q + 1] = x.y; ra[4 * q + 2] = x.z; ra[4 * q + 3] = x.w;
@@ -109,14 +118,14 @@ __global__ void __launch_bounds__(256, TM == 8 ? 2 : 4) gemm_nn_kernel(const flo
             } else {
 #pragma unroll
                 for (int q = 0; q < LA; ++q) {
-                    const int i = t + 256 * q, r = i / BK, k = k0 + i % BK;
+                    const int i = t + NT * q, r = i / BK, k = k0 + i % BK;
                     ra[q] = (m0 + r < M && k < K) ? A[(m0 + r) * lda + k] : 0.f;
                 }
             }
             if (vb && LB >= 4) {
 #pragma unroll
                 for (int q = 0; q < LB / 4; ++q) {
-                    const int i = t + 256 * q, k = k0 + i / (BN / 4), n = n0 + 4 * (i % (BN / 4));
+                    const int i = t + NT * q, k = k0 + i / (BN / 4), n = n0 + 4 * (i % (BN / 4));
                     const float4 x = (k < K && n < N) ? *reinterpret_cast<const float4*>(B + (int64_t)k * N + n)
                                                       : make_float4(0.f, 0.f, 0.f, 0.f);
                     rb[4 * q] = x.x; rb[4 * q + 1] = x.y; rb[4 * q + 2] = x.z; rb[4 * q + 3] = x.w;
@@ -124,7 +133,7 @@ __global__ void __launch_bounds__(256, TM == 8 ? 2 : 4) gemm_nn_kernel(const flo
             } else {
 #pragma unroll
                 for (int q = 0; q < LB; ++q) {
-                    const int i = t + 256 * q, k = k0 + i / BN, n = n0 + i % BN;
+                    const int i = t + NT * q, k = k0 + i / BN, n = n0 + i % BN;
                     rb[q] = (k < K && n < N) ? B[(int64_t)k * N + n] : 0.f;
                 }
             }
@@ -133,28 +142,28 @@ __global__ void __launch_bounds__(256, TM == 8 ? 2 : 4) gemm_nn_kernel(const flo
             if (va && LA >= 4) {
 #pragma unroll
                 for (int q = 0; q < LA / 4; ++q) {
-                    const int i = t + 256 * q, r = i / (BK / 4), k = 4 * (i % (BK / 4));
+                    const int i = t + NT * q, r = i / (BK / 4), k = 4 * (i % (BK / 4));
 #pragma unroll
                     for (int j = 0; j < 4; ++j) As[b][(k + j) * T::LDA + r] = ra[4 * q + j];
                 }
             } else {
 #pragma unroll
                 for (int q = 0; q < LA; ++q) {
-                    const int i = t + 256 * q;
+                    const int i = t + NT * q;
                     As[b][(i % BK) * T::LDA + i / BK] = ra[q];
                 }
             }
             if (vb && LB >= 4) {
 #pragma unroll
                 for (int q = 0; q < LB / 4; ++q) {
-                    const int i = t + 256 * q;
+                    const int i = t + NT * q;
                     *reinterpret_cast<float4*>(&Bs[b][(i / (BN / 4)) * T::LDB + 4 * (i % (BN / 4))]) =
                         make_float4(rb[4 * q], rb[4 * q + 1], rb[4 * q + 2], rb[4 * q + 3]);
                 }
             } else {
 #pragma unroll
                 for (int q = 0; q < LB; ++q) {
-                    const int i = t + 256 * q;
+                    const int i = t + NT * q;
                     Bs[b][(i / BN) * T::LDB + i % BN] = rb[q];
                 }
             }
@@ -208,6 +217,126 @@ __global__ void __launch_bounds__(256, TM == 8 ? 2 : 4) gemm_nn_kernel(const flo
             }
         }
     }
+}
+
+// The same product on 16-byte aligned rows: lda, K and N multiples of 4,
+// every pointer 16-byte aligned.  One tile per block: persistent blocks that
+// prefetch across tiles end unevenly (145,000 x 384 x 128: 355 against 303
+// us).  A stays row-major in shared memory (a thread reads 4 k's of a row at
+// once), its rows padded by 4 floats against bank conflicts; thread (ty, tx)
+// holds rows ty + i NTY and columns tx 4 + j.
+template <int MODE, int BM, int BN, int TM, int TN, int KS>
+struct VecTile {
+    static constexpr int NTX = BN / TN, NTY = BM / TM, NT = NTX * NTY, LDA = KS + 4;
+    static constexpr int SA = BM * LDA, SB = KS * BN, STAGES = 3;
+    static constexpr int SMEM = STAGES * (SA + SB) * 4;
+    static_assert(SMEM <= 48 * 1024, "shared memory without opt-in");
+    static_assert((BM * KS / 4) % NT == 0 && (BN * KS / 4) % NT == 0 && TN % 4 == 0, "16-byte loads");
+};
+
+template <int MODE, int BM, int BN, int TM, int TN, int KS, int PER_SM>
+__global__ void __launch_bounds__(VecTile<MODE, BM, BN, TM, TN, KS>::NT, PER_SM)
+    gemm_nn_vec_kernel(const float* __restrict__ A, const float* __restrict__ B, const float* __restrict__ bias,
+                       float* __restrict__ C, float* __restrict__ C2, const float* __restrict__ Z, int64_t M_static,
+                       const int32_t* __restrict__ m_dev, int N, int K, int lda, const Status* st) {
+    using T = VecTile<MODE, BM, BN, TM, TN, KS>;
+    constexpr int NT = T::NT, STAGES = T::STAGES;
+    extern __shared__ __align__(16) float ring[];
+    if (st->code != 0) return;
+    const int64_t M = m_dev ? (int64_t)(*m_dev) : M_static;
+    const int t = threadIdx.x, tx = t % T::NTX, ty = t / T::NTX;
+    const int n_tiles = (N + BN - 1) / BN, steps = (K + KS - 1) / KS;
+    const int64_t m0 = (blockIdx.x / n_tiles) * (int64_t)BM;
+    const int n0 = (int)(blockIdx.x % n_tiles) * BN;
+    if (m0 >= M) return;
+    auto load = [&](int s) {   // K-step s into its slot of the ring
+        if (s < steps) {
+            float* as = ring + s % STAGES * (T::SA + T::SB);
+            float* bs = as + T::SA;
+            const int k0 = s * KS;
+#pragma unroll
+            for (int q = 0; q < BM * KS / 4 / NT; ++q) {
+                const int i = t + NT * q, r = i / (KS / 4), k = 4 * (i % (KS / 4));
+                const bool ok = m0 + r < M && k0 + k < K;
+                tc::cp_async16_or_zero(as + r * T::LDA + k, ok ? A + (m0 + r) * lda + k0 + k : A, ok);
+            }
+#pragma unroll
+            for (int q = 0; q < BN * KS / 4 / NT; ++q) {
+                const int i = t + NT * q, k = i / (BN / 4), n = 4 * (i % (BN / 4));
+                const bool ok = k0 + k < K && n0 + n < N;
+                tc::cp_async16_or_zero(bs + k * BN + n, ok ? B + (int64_t)(k0 + k) * N + n0 + n : B, ok);
+            }
+        }
+        tc::cp_async_commit();
+    };
+#pragma unroll
+    for (int s = 0; s < STAGES - 1; ++s) load(s);
+    f32x2 acc[TM][TN / 2];
+#pragma unroll
+    for (int i = 0; i < TM; ++i)
+#pragma unroll
+        for (int j = 0; j < TN / 2; ++j) acc[i][j] = pack2(0.f, 0.f);
+    for (int s = 0; s < steps; ++s) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 2) : "memory");
+        __syncthreads();   // the step has landed, and its slot before last is read
+        load(s + STAGES - 1);
+        const float* as = ring + s % STAGES * (T::SA + T::SB);
+        const float* bs = as + T::SA;
+#pragma unroll
+        for (int k4 = 0; k4 < KS; k4 += 4) {
+            float4 a[TM];
+#pragma unroll
+            for (int i = 0; i < TM; ++i)
+                a[i] = *reinterpret_cast<const float4*>(as + (i * T::NTY + ty) * T::LDA + k4);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                float4 b[TN / 4];
+#pragma unroll
+                for (int j = 0; j < TN / 4; ++j)
+                    b[j] = *reinterpret_cast<const float4*>(bs + (k4 + k) * BN + j * (BN / (TN / 4)) + tx * 4);
+#pragma unroll
+                for (int i = 0; i < TM; ++i) {
+                    const float x = k == 0 ? a[i].x : k == 1 ? a[i].y : k == 2 ? a[i].z : a[i].w;
+                    const f32x2 xx = pack2(x, x);
+#pragma unroll
+                    for (int j = 0; j < TN / 4; ++j) {
+                        acc[i][2 * j] = fma2(xx, pack2(b[j].x, b[j].y), acc[i][2 * j]);
+                        acc[i][2 * j + 1] = fma2(xx, pack2(b[j].z, b[j].w), acc[i][2 * j + 1]);
+                    }
+                }
+            }
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < TN / 4; ++j) {
+        const int gn = n0 + j * (BN / (TN / 4)) + tx * 4;
+        if (gn >= N) continue;
+        float bj[4] = {0.f, 0.f, 0.f, 0.f};
+        if (MODE != 2 && bias) {
+#pragma unroll
+            for (int q = 0; q < 4; ++q) bj[q] = __ldg(bias + gn + q);
+        }
+#pragma unroll
+        for (int i = 0; i < TM; ++i) {
+            const int64_t gm = m0 + i * T::NTY + ty;
+            if (gm >= M) break;
+            const int64_t idx = gm * N + gn;
+            float v[4] = {lo2(acc[i][2 * j]), hi2(acc[i][2 * j]), lo2(acc[i][2 * j + 1]), hi2(acc[i][2 * j + 1])};
+            if (MODE != 2 && bias) {
+#pragma unroll
+                for (int q = 0; q < 4; ++q) v[q] += bj[q];
+            }
+            if (MODE == 2) {
+                const float4 z = __ldg(reinterpret_cast<const float4*>(Z + idx));
+                v[0] *= dsilu_f(z.x); v[1] *= dsilu_f(z.y); v[2] *= dsilu_f(z.z); v[3] *= dsilu_f(z.w);
+            }
+            *reinterpret_cast<float4*>(C + idx) = make_float4(v[0], v[1], v[2], v[3]);
+            if (MODE == 1)
+                *reinterpret_cast<float4*>(C2 + idx) =
+                    make_float4(silu_f(v[0]), silu_f(v[1]), silu_f(v[2]), silu_f(v[3]));
+        }
+    }
+    tc::cp_async_wait_all();
 }
 
 // partial[split][m][n] over the split's rows, partial column sums behind the
@@ -308,8 +437,90 @@ __global__ void __launch_bounds__(256, 4) gemm_tn_kernel(GemmRows x, int lda, in
     }
 }
 
+// The same sums on 16-byte aligned rows (lda, ldb, M and N multiples of 4):
+// rows through the cp.async ring, 8 x 4 outputs per thread in packed pairs of
+// m.  The same rows per split in the same order, so the same bits.
+// 145,000 rows, 128 x 384: 298 -> 241 us.
+constexpr int TV_NT = 128, TV_STAGES = 3;
+__global__ void __launch_bounds__(TV_NT, 4) gemm_tn_vec_kernel(GemmRows x, int lda, int ldb, int M, int N,
+                                                               int64_t rows, int nsplit, int want_sum,
+                                                               float* __restrict__ part, const Status* st) {
+    __shared__ __align__(16) float ring[TV_STAGES][2][BK * TNB];
+    if (st->code != 0) return;
+    const int tiles_n = max(1, (N + TNB - 1) / TNB);
+    const int m0 = (blockIdx.x / tiles_n) * TNB, n0 = (blockIdx.x % tiles_n) * TNB;
+    const int seg_splits = x.A1 ? nsplit / 2 : nsplit, seg = blockIdx.y / seg_splits;
+    const float* A = seg ? x.A1 : x.A;
+    const float* B = seg ? x.B1 : x.B;
+    int64_t per = (rows + seg_splits - 1) / seg_splits;
+    if (per < TN_MIN_ROWS) per = TN_MIN_ROWS;
+    const int64_t r0 = (int64_t)(blockIdx.y - seg * seg_splits) * per, r1 = min(rows, r0 + per);
+    const int steps = r0 < r1 ? (int)((r1 - r0 + BK - 1) / BK) : 0;
+    const int t = threadIdx.x, tx = t % 16, ty = t / 16;   // outputs m0 + 4 ty + {0..3, 32..35}, n0 + 4 tx + {0..3}
+    const bool sums = want_sum && n0 == 0 && seg == 0;
+    auto load = [&](int s) {
+        if (s < steps) {
+#pragma unroll
+            for (int q = 0; q < BK * TNB / 4 / TV_NT; ++q) {
+                const int i = t + TV_NT * q, r = i / (TNB / 4), c = 4 * (i % (TNB / 4));
+                const int64_t row = r0 + (int64_t)s * BK + r;
+                const bool oa = row < r1 && m0 + c < M, ob = row < r1 && n0 + c < N;
+                tc::cp_async16_or_zero(&ring[s % TV_STAGES][0][r * TNB + c], oa ? A + row * lda + m0 + c : A, oa);
+                tc::cp_async16_or_zero(&ring[s % TV_STAGES][1][r * TNB + c], ob ? B + row * ldb + n0 + c : B, ob);
+            }
+        }
+        tc::cp_async_commit();
+    };
+    f32x2 acc[4][4], asum[4];   // [pair of m][n]
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        asum[i] = pack2(0.f, 0.f);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[i][j] = pack2(0.f, 0.f);
+    }
+    const f32x2 one = pack2(1.f, 1.f);
+#pragma unroll
+    for (int s = 0; s < TV_STAGES - 1; ++s) load(s);
+    for (int s = 0; s < steps; ++s) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(TV_STAGES - 2) : "memory");
+        __syncthreads();
+        load(s + TV_STAGES - 1);
+        const float* as = ring[s % TV_STAGES][0] + 4 * ty;
+        const float* bs = ring[s % TV_STAGES][1] + 4 * tx;
+#pragma unroll
+        for (int k = 0; k < BK; ++k) {
+            const float4 a0 = *reinterpret_cast<const float4*>(as + k * TNB);
+            const float4 a1 = *reinterpret_cast<const float4*>(as + k * TNB + 32);
+            const float4 b4 = *reinterpret_cast<const float4*>(bs + k * TNB);
+            const f32x2 a[4] = {pack2(a0.x, a0.y), pack2(a0.z, a0.w), pack2(a1.x, a1.y), pack2(a1.z, a1.w)};
+            const f32x2 b[4] = {pack2(b4.x, b4.x), pack2(b4.y, b4.y), pack2(b4.z, b4.z), pack2(b4.w, b4.w)};
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) acc[i][j] = fma2(a[i], b[j], acc[i][j]);
+            if (sums) {
+#pragma unroll
+                for (int i = 0; i < 4; ++i) asum[i] = fma2(a[i], one, asum[i]);
+            }
+        }
+    }
+    tc::cp_async_wait_all();
+    float* out = part + (int64_t)blockIdx.y * M * N;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const int m = m0 + 4 * ty + (i / 4) * 32 + i % 4, n = n0 + 4 * tx;
+        if (m >= M) continue;
+        auto half = [&](f32x2 v) { return i % 2 ? hi2(v) : lo2(v); };
+        if (n < N)
+            *reinterpret_cast<float4*>(out + (int64_t)m * N + n) =
+                make_float4(half(acc[i / 2][0]), half(acc[i / 2][1]), half(acc[i / 2][2]), half(acc[i / 2][3]));
+        if (want_sum && n0 == 0 && tx == 0)
+            part[(int64_t)nsplit * M * N + (int64_t)blockIdx.y * M + m] = half(asum[i / 2]);
+    }
+}
+
 // sums over the splits, in split order: four interleaved chains per output
-__global__ void __launch_bounds__(256) gemm_tn_sum_kernel(const float* __restrict__ part, int64_t MN, int M,
+__global__ void __launch_bounds__(128) gemm_tn_sum_kernel(const float* __restrict__ part, int64_t MN, int M,
                                                           int nsplit, int acc, float* __restrict__ C,
                                                           float* __restrict__ colsum, const Status* st) {
     if (st->code != 0) return;
@@ -321,6 +532,13 @@ __global__ void __launch_bounds__(256) gemm_tn_sum_kernel(const float* __restric
         const int64_t stride = col ? M : MN;
         float s[4] = {0.f, 0.f, 0.f, 0.f};
         int sp = 0;
+        for (; sp + 16 <= nsplit; sp += 16) {   // 16 loads in flight
+            float x[16];
+#pragma unroll
+            for (int q = 0; q < 16; ++q) x[q] = p[(int64_t)(sp + q) * stride];
+#pragma unroll
+            for (int q = 0; q < 16; ++q) s[q & 3] += x[q];
+        }
         for (; sp + 4 <= nsplit; sp += 4)
 #pragma unroll
             for (int q = 0; q < 4; ++q) s[q] += p[(int64_t)(sp + q) * stride];
@@ -331,16 +549,50 @@ __global__ void __launch_bounds__(256) gemm_tn_sum_kernel(const float* __restric
     }
 }
 
-template <int BM, int BN, int TM, int TN>
-int launch_nn(int mode, const float* A, const float* B, const float* bias, float* C, float* C2, const float* Z,
-              int64_t M, const int32_t* m_dev, int N, int K, int lda, const Status* st, cudaStream_t s, int per_sm) {
-    const int64_t tiles = ((M + BM - 1) / BM) * ((N + BN - 1) / BN);
+struct NnArgs {
+    const float *A, *B, *bias;
+    float *C, *C2;
+    const float* Z;
+    int64_t M;
+    const int32_t* m_dev;
+    int N, K, lda;
+    const Status* st;
+};
+
+template <int MODE, int BM, int BN, int TM, int TN>
+int launch_nn(const NnArgs& a, cudaStream_t s, int per_sm) {
+    const int64_t tiles = ((a.M + BM - 1) / BM) * ((a.N + BN - 1) / BN);
     const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>(tiles, (int64_t)num_sms() * per_sm));
-    if (mode == 0) gemm_nn_kernel<0, BM, BN, TM, TN><<<blocks, 256, 0, s>>>(A, B, bias, C, C2, Z, M, m_dev, N, K, lda, st);
-    else if (mode == 1) gemm_nn_kernel<1, BM, BN, TM, TN><<<blocks, 256, 0, s>>>(A, B, bias, C, C2, Z, M, m_dev, N, K, lda, st);
-    else gemm_nn_kernel<2, BM, BN, TM, TN><<<blocks, 256, 0, s>>>(A, B, bias, C, C2, Z, M, m_dev, N, K, lda, st);
+    gemm_nn_kernel<MODE, BM, BN, TM, TN><<<blocks, Tile<BM, BN, TM, TN>::NT, 0, s>>>(
+        a.A, a.B, a.bias, a.C, a.C2, a.Z, a.M, a.m_dev, a.N, a.K, a.lda, a.st);
     MLFF_LAUNCH_CHECK("gemm_nn");
     return MLFF_OK;
+}
+template <int MODE, int BM, int BN, int TM, int TN, int KS, int PER_SM>
+int launch_nn_vec(const NnArgs& a, cudaStream_t s) {
+    using T = VecTile<MODE, BM, BN, TM, TN, KS>;
+    const int64_t tiles = ((a.M + BM - 1) / BM) * ((a.N + BN - 1) / BN);
+    if (tiles == 0) return MLFF_OK;
+    gemm_nn_vec_kernel<MODE, BM, BN, TM, TN, KS, PER_SM><<<(unsigned)tiles, T::NT, T::SMEM, s>>>(
+        a.A, a.B, a.bias, a.C, a.C2, a.Z, a.M, a.m_dev, a.N, a.K, a.lda, a.st);
+    MLFF_LAUNCH_CHECK("gemm_nn_vec");
+    return MLFF_OK;
+}
+
+template <int MODE>
+int nn_mode(const NnArgs& a, cudaStream_t s) {
+    auto tiles = [&](int bm, int bn) { return ((a.M + bm - 1) / bm) * ((a.N + bn - 1) / bn); };
+    const int64_t want = 2LL * num_sms();
+    const bool vec = (a.K & 3) == 0 && (a.lda & 3) == 0 && (a.N & 3) == 0 && aligned16(a.A) && aligned16(a.B) &&
+                     aligned16(a.C) && (MODE != 1 || aligned16(a.C2)) && (MODE != 2 || aligned16(a.Z));
+    if (vec) {
+        // 64 x 128 tiles keep the FP32 pipes busiest once every SM has two (16,000 x 128 x 384: 43
+        // against 49 us); below, 32 x 32 ones fill the SMs (2,400 x 384 x 128: 12 against 29 us)
+        if (a.N > 64 && tiles(64, 128) >= want) return launch_nn_vec<MODE, 64, 128, 8, 8, 16, 4>(a, s);
+        return launch_nn_vec<MODE, 32, 32, 4, 4, 32, 8>(a, s);
+    }
+    if (2 * tiles(64, 64) >= want) return launch_nn<MODE, 64, 64, 4, 4>(a, s, 6);
+    return launch_nn<MODE, 32, 32, 2, 2>(a, s, 8);
 }
 
 }  // namespace
@@ -348,16 +600,8 @@ int launch_nn(int mode, const float* A, const float* B, const float* bias, float
 int gemm_nn(int mode, const float* A, const float* B, const float* bias, float* C, float* C2, const float* Z,
             int64_t M, const int32_t* m_dev, int N, int K, const Status* st, cudaStream_t s, int lda) {
     ProfScope prof(PK_PLAIN_GEMM, s);
-    if (lda == 0) lda = K;
-    // The largest tile that still gives every SM two of them (64 x 64: one):
-    // 128 x 128 keeps the FP32 pipes busiest, small row counts need the tiles
-    // more.
-    auto tiles = [&](int bm, int bn) { return ((M + bm - 1) / bm) * ((N + bn - 1) / bn); };
-    const int64_t want = 2LL * num_sms();
-    if (N > 64 && tiles(128, 128) >= want)
-        return launch_nn<128, 128, 8, 8>(mode, A, B, bias, C, C2, Z, M, m_dev, N, K, lda, st, s, 2);
-    if (2 * tiles(64, 64) >= want) return launch_nn<64, 64, 4, 4>(mode, A, B, bias, C, C2, Z, M, m_dev, N, K, lda, st, s, 6);
-    return launch_nn<32, 32, 2, 2>(mode, A, B, bias, C, C2, Z, M, m_dev, N, K, lda, st, s, 8);
+    const NnArgs a{A, B, bias, C, C2, Z, M, m_dev, N, K, lda ? lda : K, st};
+    return mode == 0 ? nn_mode<0>(a, s) : mode == 1 ? nn_mode<1>(a, s) : nn_mode<2>(a, s);
 }
 
 size_t gemm_tn_floats(int64_t M, int64_t N) { return (size_t)tn_splits(M, N) * (size_t)(M * N + M); }
@@ -369,10 +613,13 @@ int gemm_tn(const GemmRows& x, int lda, int ldb, int M, int N, int64_t rows, flo
     int ns = (int)std::max<int64_t>(1, std::min<int64_t>(tn_splits(M, N), (rows + TN_MIN_ROWS - 1) / TN_MIN_ROWS));
     if (x.A1) ns = 2 * std::max(1, ns / 2);
     dim3 grid(tn_tiles(M) * tn_tiles(N), ns);
-    gemm_tn_kernel<<<grid, 256, 0, s>>>(x, lda, ldb, M, N, rows, ns, colsum != nullptr, part, st);
+    const bool vec = ((lda | ldb | M | N) & 3) == 0 && aligned16(x.A) && aligned16(x.B) && aligned16(x.A1) &&
+                     aligned16(x.B1) && aligned16(part);
+    if (vec) gemm_tn_vec_kernel<<<grid, TV_NT, 0, s>>>(x, lda, ldb, M, N, rows, ns, colsum != nullptr, part, st);
+    else gemm_tn_kernel<<<grid, 256, 0, s>>>(x, lda, ldb, M, N, rows, ns, colsum != nullptr, part, st);
     MLFF_LAUNCH_CHECK("gemm_tn");
     const int64_t out = (int64_t)M * N + M;
-    gemm_tn_sum_kernel<<<(int)std::min<int64_t>((out + 255) / 256, 152 * 8), 256, 0, s>>>(
+    gemm_tn_sum_kernel<<<(int)std::min<int64_t>((out + 127) / 128, 152 * 16), 128, 0, s>>>(
         part, (int64_t)M * N, M, ns, accumulate ? 1 : 0, C, colsum, st);
     MLFF_LAUNCH_CHECK("gemm_tn_sum");
     return MLFF_OK;

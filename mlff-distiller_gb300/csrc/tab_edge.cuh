@@ -2,6 +2,7 @@
 #pragma once
 #include <algorithm>
 #include <type_traits>
+#include "f32x2.cuh"
 #include "tab.cuh"
 #include "tc_layout.cuh"
 #include "tc_ptx.cuh"
@@ -11,30 +12,6 @@ namespace mlff {
 // dt/dd of the table's local coordinate, as the kernels use it in FP32; the
 // build places its nodes with the same rounded value.
 __host__ __device__ inline float tab_scale(float cutoff) { return (float)(2.0 * TAB_NI / (double)cutoff); }
-
-// Two FP32 values in a register pair and their two-wide fused multiply-add:
-// one instruction slot for two roundings-to-nearest fused multiply-adds.
-using f32x2 = unsigned long long;
-__device__ __forceinline__ f32x2 pack2(float lo, float hi) {
-    f32x2 r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-    return r;
-}
-__device__ __forceinline__ float lo2(f32x2 v) {
-    float lo, hi;
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
-    return lo;
-}
-__device__ __forceinline__ float hi2(f32x2 v) {
-    float lo, hi;
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
-    return hi;
-}
-__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
-    f32x2 d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-    return d;
-}
 
 // A condition that is the same in every lane, as a vote: the branch on it
 // needs no divergence bookkeeping and is not turned into predicated code.

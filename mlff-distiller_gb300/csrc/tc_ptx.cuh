@@ -63,7 +63,12 @@ __device__ __forceinline__ void bulk_g2s(void* dst, const void* src, uint32_t by
 }
 
 // Asynchronous global -> shared copies of 16 or 4 bytes (no register
-// staging), completed by cp_async_wait_all.
+// staging), completed by cp_async_wait_all.  _or_zero: zeros when !ok (src is
+// then not read, but stays a valid address).
+__device__ __forceinline__ void cp_async16_or_zero(void* dst, const void* src, bool ok) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(ok ? 16 : 0)
+                 : "memory");
+}
 __device__ __forceinline__ void cp_async16(void* dst, const void* src) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
 }

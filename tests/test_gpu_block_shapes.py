@@ -75,3 +75,9 @@ def test_update_block(H, N):
     block = PaiNNUpdate(H).to(DEV)
     ins = [torch.randn(*s, device=DEV, generator=g).requires_grad_(True) for s in ((N, H), (N, 3, H))]
     compare(block, ins, [], lambda x, p: ref_update(x[0], x[1], *p))
+
+
+@pytest.mark.parametrize("H,R,N,E", [(128, 20, 300, 9999), (132, 24, 200, 7041), (68, 36, 100, 19457)])
+def test_message_block_wide_tiles(H, R, N, E):
+    """Enough rows for the 64 x 128 tiles, with remainders in every direction."""
+    test_message_block(H, R, N, E, 0)
