@@ -73,22 +73,25 @@ PackedOffsets packed_offsets(const mlff_dims& d) {
     return o;
 }
 
-// dst[r][c] = src[c][r] (src rows x cols, zero-padded to dst_rows x dst_cols)
-__global__ void transpose_pad_kernel(const float* __restrict__ src, int rows, int cols,
-                                     float* __restrict__ dst, int dst_rows, int dst_cols) {
-    // dst is [cols_pad][rows_pad]: dst[c * dst_cols + r] = src[r * cols + c]
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < dst_rows * dst_cols; i += gridDim.x * blockDim.x) {
-        int c = i / dst_cols, r = i % dst_cols;
-        dst[i] = (c < cols && r < rows) ? src[(int64_t)r * cols + c] : 0.0f;
-    }
-}
-
-// dst [rows][dst_cols] = src [rows][cols] zero-padded columns
-__global__ void copy_pad_kernel(const float* __restrict__ src, int rows, int cols,
-                                float* __restrict__ dst, int dst_cols) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < rows * dst_cols; i += gridDim.x * blockDim.x) {
-        int r = i / dst_cols, c = i % dst_cols;
-        dst[i] = c < cols ? src[(int64_t)r * cols + c] : 0.0f;
+// One copied or transposed matrix of the packed blob: dst [drows][dcols] =
+// src [rows][cols] or its transpose, zero-padded.
+struct PackJob {
+    const float* src;
+    float* dst;
+    int rows, cols, drows, dcols, transpose;
+};
+// All matrices of a model in one launch (grid y: the matrix).  A training
+// step packs its weights each time; 48 separate copies and transposes cost
+// 0.2 ms of launches.
+constexpr int PACK_JOBS = 64;
+struct PackJobs {
+    PackJob job[PACK_JOBS];
+};
+__global__ void __launch_bounds__(256) pack_fp32_kernel(const __grid_constant__ PackJobs jobs) {
+    const PackJob& j = jobs.job[blockIdx.y];
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < j.drows * j.dcols; i += gridDim.x * blockDim.x) {
+        const int a = i / j.dcols, b = i % j.dcols, r = j.transpose ? b : a, c = j.transpose ? a : b;
+        j.dst[i] = (r < j.rows && c < j.cols) ? j.src[(int64_t)r * j.cols + c] : 0.0f;
     }
 }
 
@@ -104,46 +107,56 @@ __global__ void rbf_pack_kernel(const float* __restrict__ centers, const float* 
 
 int pack_fp32(const mlff_dims& d, const mlff_params& p, float* out, const PackedOffsets& o, cudaStream_t st) {
     const int R = d.n_rbf;
-    auto cp = [&](float* dst, const float* src, int64_t n) -> int {
-        MLFF_CUDA(cudaMemcpyAsync(dst, src, sizeof(float) * n, cudaMemcpyDeviceToDevice, st));
+    PackJobs jobs;   // [0, n_jobs) are set
+    int n_jobs = 0, r = MLFF_OK;
+    auto flush = [&]() -> int {
+        if (r) return r;
+        pack_fp32_kernel<<<dim3(32, n_jobs), 256, 0, st>>>(jobs);
+        n_jobs = 0;
+        MLFF_LAUNCH_CHECK("pack_fp32");
         return MLFF_OK;
     };
-    auto tr = [&](const float* src, int rows, int cols, float* dst, int dst_rows, int dst_cols) -> int {
-        // dst holds src^T padded: dst_rows >= cols, dst_cols >= rows
-        transpose_pad_kernel<<<128, 256, 0, st>>>(src, rows, cols, dst, dst_rows, dst_cols);
-        MLFF_LAUNCH_CHECK("transpose_pad");
-        return MLFF_OK;
+    auto job = [&](const float* src, float* dst, int rows, int cols, int drows, int dcols, int transpose) {
+        if (!src) {
+            set_error("a weight pointer is NULL");
+            r = MLFF_ERR_INVALID;
+        }
+        if (n_jobs == PACK_JOBS) r = flush();
+        if (r) return;
+        jobs.job[n_jobs++] = {src, dst, rows, cols, drows, dcols, transpose};
     };
-    int r;
-    if ((r = cp(out + o.emb, p.embedding, (int64_t)d.n_species * H))) return r;
+    auto cp = [&](float* dst, const float* src, int64_t n) { job(src, dst, 1, (int)n, 1, (int)n, 0); };
+    auto tr = [&](const float* src, int rows, int cols, float* dst, int dst_rows, int dst_cols) {
+        job(src, dst, rows, cols, dst_rows, dst_cols, 1);
+    };
+    cp(out + o.emb, p.embedding, (int64_t)d.n_species * H);
     rbf_pack_kernel<<<1, RMAX, 0, st>>>(p.rbf_centers, p.rbf_widths, R, out + o.centers, out + o.gamma);
     MLFF_LAUNCH_CHECK("rbf_pack");
-    if ((r = tr(p.head_w1, 64, H, out + o.head_w1t, H, 64))) return r;
-    if ((r = cp(out + o.head_w1, p.head_w1, 64 * H))) return r;
-    if ((r = cp(out + o.head_b1, p.head_b1, 64))) return r;
-    if ((r = tr(p.head_w2, 32, 64, out + o.head_w2t, 64, 32))) return r;
-    if ((r = cp(out + o.head_w2, p.head_w2, 32 * 64))) return r;
-    if ((r = cp(out + o.head_b2, p.head_b2, 32))) return r;
-    if ((r = cp(out + o.head_w3, p.head_w3, 32))) return r;
-    if ((r = cp(out + o.head_b3, p.head_b3, 1))) return r;
+    tr(p.head_w1, 64, H, out + o.head_w1t, H, 64);
+    cp(out + o.head_w1, p.head_w1, 64 * H);
+    cp(out + o.head_b1, p.head_b1, 64);
+    tr(p.head_w2, 32, 64, out + o.head_w2t, 64, 32);
+    cp(out + o.head_w2, p.head_w2, 32 * 64);
+    cp(out + o.head_b2, p.head_b2, 32);
+    cp(out + o.head_w3, p.head_w3, 32);
+    cp(out + o.head_b3, p.head_b3, 1);
     for (int l = 0; l < d.n_layers; ++l) {
         const LayerOffsets& L = o.layer[l];
-        if ((r = tr(p.filter_w1[l], H, R, out + L.w1t, RMAX, H))) return r;
-        copy_pad_kernel<<<64, 256, 0, st>>>(p.filter_w1[l], H, R, out + L.w1, RMAX);
-        MLFF_LAUNCH_CHECK("copy_pad");
-        if ((r = cp(out + L.b1, p.filter_b1[l], H))) return r;
-        if ((r = tr(p.filter_w2[l], H3, H, out + L.w2t, H, H3))) return r;
-        if ((r = cp(out + L.w2, p.filter_w2[l], (int64_t)H3 * H))) return r;
-        if ((r = cp(out + L.b2, p.filter_b2[l], H3))) return r;
-        if ((r = cp(out + L.mix, p.mixing[l], 9))) return r;
-        if ((r = tr(p.update_w1[l], H, 2 * H, out + L.u1t, 2 * H, H))) return r;
-        if ((r = cp(out + L.u1, p.update_w1[l], (int64_t)H * 2 * H))) return r;
-        if ((r = cp(out + L.c1, p.update_b1[l], H))) return r;
-        if ((r = tr(p.update_w2[l], H3, H, out + L.u2t, H, H3))) return r;
-        if ((r = cp(out + L.u2, p.update_w2[l], (int64_t)H3 * H))) return r;
-        if ((r = cp(out + L.c2, p.update_b2[l], H3))) return r;
+        tr(p.filter_w1[l], H, R, out + L.w1t, RMAX, H);
+        job(p.filter_w1[l], out + L.w1, H, R, H, RMAX, 0);
+        cp(out + L.b1, p.filter_b1[l], H);
+        tr(p.filter_w2[l], H3, H, out + L.w2t, H, H3);
+        cp(out + L.w2, p.filter_w2[l], (int64_t)H3 * H);
+        cp(out + L.b2, p.filter_b2[l], H3);
+        cp(out + L.mix, p.mixing[l], 9);
+        tr(p.update_w1[l], H, 2 * H, out + L.u1t, 2 * H, H);
+        cp(out + L.u1, p.update_w1[l], (int64_t)H * 2 * H);
+        cp(out + L.c1, p.update_b1[l], H);
+        tr(p.update_w2[l], H3, H, out + L.u2t, H, H3);
+        cp(out + L.u2, p.update_w2[l], (int64_t)H3 * H);
+        cp(out + L.c2, p.update_b2[l], H3);
     }
-    return MLFF_OK;
+    return flush();
 }
 
 // ------------------------------------------------------------- embedding

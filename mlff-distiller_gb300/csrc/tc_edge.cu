@@ -64,9 +64,13 @@ constexpr uint32_t TM_W2LO = 0;
 // followed by the 24 matching lo tiles; W2's third chunk transposed
 // (rows = hidden units, K = channels) -> 8 K-step pairs (hi tile, lo tile)
 // for the per-atom Q rows of the reverse pass.
-__global__ void pack_tc_kernel(const float* __restrict__ w1, const float* __restrict__ w2,
-                               unsigned char* __restrict__ w1_out, unsigned char* __restrict__ w2_out,
-                               uint32_t* __restrict__ w2_tm, unsigned char* __restrict__ w2q_out) {
+__global__ void pack_tc_kernel(float* __restrict__ out, PackedOffsets o) {   // grid y: the layer
+    const LayerOffsets& L = o.layer[blockIdx.y];
+    const float *w1 = out + L.w1, *w2 = out + L.w2;
+    unsigned char* w1_out = reinterpret_cast<unsigned char*>(out + L.w1_bf);
+    unsigned char* w2_out = reinterpret_cast<unsigned char*>(out + L.w2_bf);
+    uint32_t* w2_tm = reinterpret_cast<uint32_t*>(out + L.w2_tm);
+    unsigned char* w2q_out = reinterpret_cast<unsigned char*>(out + L.w2q_tc);
     const int stride = gridDim.x * blockDim.x;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < 8 * 128 * 16; i += stride) {
         const int s = i / 2048, m = (i / 16) % 128, kk = i % 16;
@@ -108,14 +112,8 @@ __global__ void pack_tc_kernel(const float* __restrict__ w1, const float* __rest
 int pack_update_tc(const mlff_dims& d, float* out, const PackedOffsets& o, cudaStream_t st);
 
 int pack_bf16(const mlff_dims& d, float* out, const PackedOffsets& o, cudaStream_t st) {
-    for (int l = 0; l < d.n_layers; ++l) {
-        const LayerOffsets& L = o.layer[l];
-        pack_tc_kernel<<<64, 256, 0, st>>>(out + L.w1, out + L.w2, reinterpret_cast<unsigned char*>(out + L.w1_bf),
-                                           reinterpret_cast<unsigned char*>(out + L.w2_bf),
-                                           reinterpret_cast<uint32_t*>(out + L.w2_tm),
-                                           reinterpret_cast<unsigned char*>(out + L.w2q_tc));
-        MLFF_LAUNCH_CHECK("pack_tc");
-    }
+    pack_tc_kernel<<<dim3(64, d.n_layers), 256, 0, st>>>(out, o);
+    MLFF_LAUNCH_CHECK("pack_tc");
     return pack_update_tc(d, out, o, st);
 }
 

@@ -34,9 +34,11 @@ using namespace tc;
 // ------------------------------------------------------------- packing
 // pair p of a matrix: hi tile at p * A_PAIR, lo tile at p * A_PAIR + A_TILE;
 // element (m, k) of the pair's 128 x 16 block at a_off(m, k).
-__global__ void pack_update_tc_kernel(const float* __restrict__ u1, const float* __restrict__ u2,
-                                      unsigned char* __restrict__ u1p, unsigned char* __restrict__ u2p,
-                                      unsigned char* __restrict__ u2tp, unsigned char* __restrict__ u1tp) {
+__global__ void pack_update_tc_kernel(float* __restrict__ out, PackedOffsets o) {   // grid y: the layer
+    const LayerOffsets& L = o.layer[blockIdx.y];
+    const float *u1 = out + L.u1, *u2 = out + L.u2;
+    auto bytes = [&](int64_t off) { return reinterpret_cast<unsigned char*>(out + off); };
+    unsigned char *u1p = bytes(L.u1_tc), *u2p = bytes(L.u2_tc), *u2tp = bytes(L.u2t_tc), *u1tp = bytes(L.u1t_tc);
     const int stride = gridDim.x * blockDim.x;
     auto put = [](unsigned char* dst, int pair, int m, int kk, float v) {
         __half hi, lo;
@@ -59,13 +61,8 @@ __global__ void pack_update_tc_kernel(const float* __restrict__ u1, const float*
 }
 
 int pack_update_tc(const mlff_dims& d, float* out, const PackedOffsets& o, cudaStream_t st) {
-    for (int l = 0; l < d.n_layers; ++l) {
-        const LayerOffsets& L = o.layer[l];
-        auto b = [&](int64_t off) { return reinterpret_cast<unsigned char*>(out + off); };
-        pack_update_tc_kernel<<<64, 256, 0, st>>>(out + L.u1, out + L.u2, b(L.u1_tc), b(L.u2_tc), b(L.u2t_tc),
-                                                  b(L.u1t_tc));
-        MLFF_LAUNCH_CHECK("pack_update_tc");
-    }
+    pack_update_tc_kernel<<<dim3(64, d.n_layers), 256, 0, st>>>(out, o);
+    MLFF_LAUNCH_CHECK("pack_update_tc");
     return MLFF_OK;
 }
 

@@ -259,8 +259,15 @@ class _EnergyForces(torch.autograd.Function):
         return (-F * g).to(grad_E.dtype), None, None, None
 
 
-def _trainable(model):
-    return [(n, p) for n, p in model.named_parameters() if p.requires_grad]
+def _trainable(model, check: bool = False):
+    """named_parameters() with requires_grad, from the model's slots."""
+    seen, out = set(), []
+    for d, n, full in model._slots(check)[0]:
+        p = d[n]
+        if p is not None and p.requires_grad and id(p) not in seen:
+            seen.add(id(p))
+            out.append((full, p))
+    return out
 
 
 class _EnergyTrain(torch.autograd.Function):
@@ -372,7 +379,7 @@ class StudentForceField(nn.Module):
         self._cell_cache = None                            # last host cell -> checked device box / pbc
         self._batch_cache = None                           # last host structure index -> device offsets
         self._packed_version = None
-        self._weight_slots = None                          # (tensor dict, name) of every parameter and buffer
+        self._weight_slots = None                          # see _slots
 
     def _initialize_parameters(self):
         """Same initialisation as the reference (student_model.py:618-628)."""
@@ -469,17 +476,32 @@ class StudentForceField(nn.Module):
             raise ValueError(f"unknown precision {self.precision!r}; use one of {sorted(_lib.PATHS)}")
         return base if self._engine is None else self._engine.route(base)
 
+    def _slots(self, check: bool = False):
+        """(parameters, all, buffers, modules): (tensor dict, name, full name)
+        of every parameter, (tensor dict, name) of every parameter and
+        buffer, the first form of every buffer, and the modules' state: the
+        modules' own dicts, looked up once (walking the module tree by name
+        costs 0.1 ms, several times a training step) and, with ``check``,
+        again when a module, parameter or buffer was added or replaced by
+        another object."""
+        if check and self._weight_slots is not None and any(
+                len(m._parameters) != np_ or len(m._buffers) != nb or tuple(m._modules.values()) != kids
+                for m, np_, nb, kids in self._weight_slots[3]):
+            self._weight_slots = None
+        if self._weight_slots is None:
+            mods = list(self.named_modules())
+            named = [[(d(m), n, f"{prefix}.{n}" if prefix else n) for prefix, m in mods for n in d(m)]
+                     for d in (lambda m: m._parameters, lambda m: m._buffers)]
+            self._weight_slots = (named[0], [(d, n) for d, n, _ in named[0] + named[1]], named[1],
+                                  [(m, len(m._parameters), len(m._buffers), tuple(m._modules.values()))
+                                   for _, m in mods])
+        return self._weight_slots
+
     def _weights_version(self):
         """(address, in-place version) of every parameter and buffer: changes
-        when a weight is updated in place, reassigned or moved.  The slots
-        are the modules' own parameter / buffer dicts, looked up once."""
-        slots = self._weight_slots
-        if slots is None:
-            slots = [(m._parameters, n) for m in self.modules() for n in m._parameters] + \
-                    [(m._buffers, n) for m in self.modules() for n in m._buffers]
-            self._weight_slots = slots
+        when a weight is updated in place, reassigned or moved."""
         return tuple((t.data_ptr(), t._version) if t is not None else None
-                     for t in (d[n] for d, n in slots))
+                     for t in (d[n] for d, n in self._slots()[1]))
 
     def engine(self) -> Engine:
         dev = self.embedding.weight.device
@@ -491,7 +513,8 @@ class StudentForceField(nn.Module):
             self._packed_version = None
         v = self._weights_version()
         if v != self._packed_version:
-            self._engine.pack(self.state_dict())
+            params, _, buffers, _ = self._slots()
+            self._engine.pack({full: d[n] for d, n, full in params + buffers if d[n] is not None})
             self._packed_version = v
         return self._engine
 
@@ -589,7 +612,7 @@ class StudentForceField(nn.Module):
             E = self._module_energy(positions, bt, mol_index).to(positions.dtype)
             return E.sum() if n_mol <= 1 else E
         bt, mol_index, n_mol = self._make_batch(atomic_numbers, positions, cell, pbc, batch)
-        train = _trainable(self) if self.training and torch.is_grad_enabled() else []
+        train = _trainable(self, True) if self.training and torch.is_grad_enabled() else []
         if train:
             # parameter gradients (to second order, for force losses) from the CUDA passes
             E = _EnergyTrain.apply(positions, self, bt, mol_index, *[p for _, p in train])
@@ -607,11 +630,11 @@ class StudentForceField(nn.Module):
         the reference does, so a loss on them back-propagates into the
         parameters."""
         if not self.fused:
-            train = self.training and torch.is_grad_enabled() and bool(_trainable(self))
+            train = self.training and torch.is_grad_enabled() and bool(_trainable(self, True))
             E, F, _, _ = self._module_call(atomic_numbers, positions, cell, pbc, None, create_graph=train)
             E = E.to(positions.dtype).sum()
             return (E, F.to(positions.dtype)) if train else (E.detach(), F.detach().to(positions.dtype))
-        if self.training and torch.is_grad_enabled() and _trainable(self):
+        if self.training and torch.is_grad_enabled() and _trainable(self, True):
             x = positions if positions.requires_grad else positions.detach().requires_grad_(True)
             E = self.forward(atomic_numbers, x, cell=cell, pbc=pbc)
             F = -torch.autograd.grad(E, x, grad_outputs=torch.ones_like(E), create_graph=True)[0]
