@@ -75,16 +75,18 @@ struct UStream {
     uint64_t* full;
     uint64_t* empty;
     const unsigned char* src[2];   // pair sources of the two GEMMs of a tile
-    int npairs[2];
+    int npairs[2];                 // (the second: chunks of 8 pairs)
     uint32_t issued;               // producer: pairs copied so far (global count)
-    uint32_t consumed;             // consumer: pairs whose copy was seen complete
 };
 
 template <int URING>
 __device__ __forceinline__ const unsigned char* ustream_src(const UStream<URING>& s, uint32_t P) {
     const uint32_t per = s.npairs[0] + s.npairs[1];
     const uint32_t q = P % per;
-    return q < (uint32_t)s.npairs[0] ? s.src[0] + (size_t)q * A_PAIR : s.src[1] + (size_t)(q - s.npairs[0]) * A_PAIR;
+    if (q < (uint32_t)s.npairs[0]) return s.src[0] + (size_t)q * A_PAIR;
+    // K-step by K-step: the chunks of the second GEMM run in parallel
+    const uint32_t chunks = s.npairs[1] / 8, r = q - s.npairs[0];
+    return s.src[1] + (size_t)(r % chunks * 8 + r / chunks) * A_PAIR;
 }
 
 // producer: copy pairs until `target` (exclusive) are issued; a slot is
@@ -103,30 +105,39 @@ __device__ __forceinline__ bool ustream_fill(UStream<URING>& s, uint32_t target)
     return true;
 }
 
-// consumer: one GEMM of a tile.  Pair i of n (global pair P0 + i): D[d_of(i)]
-// += A_hi B_hi(i) + A_hi B_lo(i) + A_lo B_hi(i); the first MMA of pair i
-// overwrites D instead when fresh(i).
-template <int UN, int URING, typename DOf, typename BOf, typename Fresh>
-__device__ __forceinline__ bool ustream_gemm(UStream<URING>& s, uint32_t P0, int n, DOf d_of, BOf b_of, uint64_t bhalf,
-                                             Fresh fresh) {
+// consumer: one accumulator tile of a GEMM.  Pair i of n (global pair
+// P0 + STRIDE i): D += A_hi B_hi(i) + A_hi B_lo(i) + A_lo B_hi(i); with fresh
+// the first MMA overwrites D.  The thread spends about 470 cycles on a pair
+// (three dependent MMAs of 72, the two barriers), so a GEMM of several chunks
+// has one issuing thread per chunk (STRIDE = their number).  A wait names its
+// pair by the parity of the slot's use, so the slot's previous pair must be
+// known to have landed: it is the thread's own (the ring's length is a
+// multiple of STRIDE) or of a GEMM the whole CTA has waited for.  Copies
+// land in any order.
+template <int UN, int STRIDE, int URING, typename BOf>
+__device__ __forceinline__ bool ustream_gemm(UStream<URING>& s, uint32_t P0, int n, uint32_t d, BOf b_of,
+                                             uint64_t bhalf, bool fresh) {
+    static_assert(URING % STRIDE == 0, "a slot is always waited for by the same thread within a GEMM");
     constexpr uint32_t idesc = idesc_f16(UN);
     const uint64_t a0 = sdesc(smem_u32(s.ring), A_LBO, A_SBO);
 #pragma unroll 1
     for (int i = 0; i < n; ++i) {
-        const uint32_t P = P0 + i;
+        const uint32_t P = P0 + STRIDE * i;
         const uint32_t slot = P % URING;
         if (!mbar_wait(&s.full[slot], (P / URING) & 1, WAIT_BUDGET)) return false;
-        s.consumed = P + 1;
         const uint64_t ahi = a0 + (uint64_t)(slot * A_PAIR >> 4), alo = ahi + (A_TILE >> 4);
         const uint64_t bhi = b_of(i);
-        const uint32_t d = d_of(i);
-        mma_f16(d, ahi, bhi, idesc, fresh(i) ? 0u : 1u);
+        mma_f16(d, ahi, bhi, idesc, fresh && i == 0 ? 0u : 1u);
         mma_f16(d, ahi, bhi + bhalf, idesc, 1);
         mma_f16(d, alo, bhi, idesc, 1);
         mma_commit(&s.empty[slot]);
     }
     return true;
 }
+
+// Issuing thread of chunk g (lane 0 of warps 0, 2 and 3; the producer is in
+// warp 1), -1 for the others.
+__device__ __forceinline__ int uissuer(int w, int lane) { return lane != 0 || w == 1 || w > 3 ? -1 : w == 0 ? 0 : w - 1; }
 
 __device__ __forceinline__ void ufill_tmem(uint32_t taddr, float v, int n16) {
     float bv[16];
@@ -201,7 +212,7 @@ __device__ __forceinline__ void uwait_mma(UCtl& c, int w, int where) {
 
 // ------------------------------------------------------- forward kernel
 // smem: B tile [s, |v|] (K = 256: 4 K-blocks; hi half then lo half, 64 KB),
-// the H tile (K = 128, 32 KB) aliased into it after GEMM1, the ring (40 KB).
+// the H tile (K = 128, 32 KB) aliased into it after GEMM1, the ring (48 KB).
 // TMEM: D1 = z (cols 0..UN-1), D2 chunk g = (ds, g1, g2)[g] (UN + UN g).
 // UN-atom tiles, UN = 64 or 32 (the autotuner's update tile: small systems
 // spread over more SMs with 32); the ring takes what two CTAs per SM leave.
@@ -212,12 +223,12 @@ struct UFwd {
     // epilogue 2 stages (ds, g1, g2) of 32 atoms, [3][32][H] floats, in the B region
     static constexpr uint32_t T_BYTES = 3 * 32 * H * 4;
     static constexpr uint32_t B_REGION = 2 * BH > T_BYTES ? 2 * BH : T_BYTES;
-    static constexpr int RING = UN == 64 ? 5 : 7;
+    static constexpr int RING = 6;
     static constexpr uint32_t OFF_B = 0;
     static constexpr uint32_t OFF_RING = OFF_B + B_REGION;
-    static constexpr uint32_t OFF_C = OFF_RING + RING * A_PAIR;      // c1 [H], c2 [3H], mix [9]
-    static constexpr uint32_t OFF_BAR = OFF_C + 4 * (H + H3 + 16);
-    static constexpr uint32_t OFF_MISC = OFF_BAR + 8 * (1 + 2 * RING);
+    static constexpr uint32_t OFF_MIX = OFF_RING + RING * A_PAIR;
+    static constexpr uint32_t OFF_BAR = OFF_MIX + 64;
+    static constexpr uint32_t OFF_MISC = OFF_BAR + 8 * (2 + 2 * RING);
     static constexpr uint32_t SMEM = align1k(OFF_MISC + 16);
     static constexpr uint32_t TMEM_COLS = 4 * UN;
     static_assert(2 * (SMEM + 1024) <= 228 * 1024, "two update CTAs per SM");
@@ -232,11 +243,10 @@ __global__ void __launch_bounds__(UNT, 2) update_fwd_tc_kernel(const float* __re
     using LF = UFwd<UN>;
     extern __shared__ __align__(1024) unsigned char smem[];
     unsigned char* Bs = smem + LF::OFF_B;
-    float* c1s = reinterpret_cast<float*>(smem + LF::OFF_C);
-    float* c2s = c1s + H;
-    float* mix = c2s + H3;
+    float* mix = reinterpret_cast<float*>(smem + LF::OFF_MIX);
     uint64_t* mma_bar = reinterpret_cast<uint64_t*>(smem + LF::OFF_BAR);
-    uint64_t* full = mma_bar + 1;
+    uint64_t* chunk_bar = mma_bar + 1;   // the second GEMM: one commit per chunk
+    uint64_t* full = mma_bar + 2;
     uint64_t* empty = full + LF::RING;
     uint32_t* tslot = reinterpret_cast<uint32_t*>(smem + LF::OFF_MISC);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + LF::OFF_MISC + 4);
@@ -248,6 +258,7 @@ __global__ void __launch_bounds__(UNT, 2) update_fwd_tc_kernel(const float* __re
     }
     if (t == 0) {
         mbar_init(mma_bar, 1);
+        mbar_init(chunk_bar, 3);
         for (int i = 0; i < LF::RING; ++i) {
             mbar_init(&full[i], 1);
             mbar_init(&empty[i], 1);
@@ -255,8 +266,6 @@ __global__ void __launch_bounds__(UNT, 2) update_fwd_tc_kernel(const float* __re
         fence_mbar_init();
         *abort_flag = 0;
     }
-    for (int i = t; i < H; i += UNT) c1s[i] = P[lo.c1 + i];
-    for (int i = t; i < H3; i += UNT) c2s[i] = P[lo.c2 + i];
     if (t < 9) mix[t] = P[lo.mix + t];
     fence_before_sync();
     __syncthreads();
@@ -264,8 +273,8 @@ __global__ void __launch_bounds__(UNT, 2) update_fwd_tc_kernel(const float* __re
     const uint32_t tmem = *tslot;
     UStream<LF::RING> ws{smem + LF::OFF_RING, full, empty,
                {reinterpret_cast<const unsigned char*>(P + lo.u1_tc), reinterpret_cast<const unsigned char*>(P + lo.u2_tc)},
-               {16, 24}, 0, 0};
-    UCtl ctl{mma_bar, abort_flag, st, 0};
+               {16, 24}, 0};
+    UCtl ctl{mma_bar, abort_flag, st, 0}, ctl2{chunk_bar, abort_flag, st, 0};
     const int my_tiles = blockIdx.x < ntiles ? (ntiles - 1 - blockIdx.x) / gridDim.x + 1 : 0;
     const uint32_t P_end = (uint32_t)my_tiles * 40;
     const bool producer = t == 32;
@@ -277,14 +286,15 @@ __global__ void __launch_bounds__(UNT, 2) update_fwd_tc_kernel(const float* __re
     pdl_trigger();
     const int q = w & 3, hh = w >> 2, c = 32 * q + lane;
     const uint32_t lane_base = tmem + ((uint32_t)(32 * q) << 16);
+    const float c1c = P[lo.c1 + c], c2c[3] = {P[lo.c2 + c], P[lo.c2 + H + c], P[lo.c2 + 2 * H + c]};
     uint32_t P0 = 0;
 
     for (int tile = blockIdx.x; tile < ntiles && !*abort_flag; tile += gridDim.x, P0 += 40) {
         const int a0 = tile * UN;
         // accumulators <- bias: D1 c1, D2 chunk g c2[g]
-        ufill_tmem(lane_base + (UN / 2) * hh, c1s[c], UN / 32);
-#pragma unroll 1
-        for (int g = 0; g < 3; ++g) ufill_tmem(lane_base + UN + UN * g + (UN / 2) * hh, c2s[g * H + c], UN / 32);
+        ufill_tmem(lane_base + (UN / 2) * hh, c1c, UN / 32);
+#pragma unroll
+        for (int g = 0; g < 3; ++g) ufill_tmem(lane_base + UN + UN * g + (UN / 2) * hh, c2c[g], UN / 32);
         // B tile: row = atom, K = [s (128), |v| (128)]; warp w builds rows w, w + 8, ...,
         // two rows per step so that their loads overlap
 #pragma unroll 1
@@ -313,9 +323,8 @@ __global__ void __launch_bounds__(UNT, 2) update_fwd_tc_kernel(const float* __re
         if (t == 0) {   // GEMM1: z^T = U1 [s, |v|]^T, K = 256
             fence_after_sync();
             const uint64_t b0 = sdesc_b(smem_u32(Bs));
-            if (!ustream_gemm<UN>(ws, P0, 16, [&](int) { return tmem; },
-                              [&](int i) { return b0 + (uint64_t)(b_kstep_off(UN, i) >> 4); }, (uint64_t)(LF::BH >> 4),
-                              [](int) { return false; }))
+            if (!ustream_gemm<UN, 1>(ws, P0, 16, tmem, [&](int i) { return b0 + (uint64_t)(b_kstep_off(UN, i) >> 4); },
+                                  (uint64_t)(LF::BH >> 4), false))
                 ufail(ctl, 21);
             mma_commit(mma_bar);
         }
@@ -344,17 +353,18 @@ __global__ void __launch_bounds__(UNT, 2) update_fwd_tc_kernel(const float* __re
         fence_async_smem();
         fence_before_sync();
         __syncthreads();
-        if (t == 0) {   // GEMM2: a^T = U2 h^T, 3 chunks x 8 K-steps
+        if (const int g = uissuer(w, lane); g >= 0) {   // GEMM2: a^T = U2 h^T, 3 chunks x 8 K-steps
             fence_after_sync();
             const uint64_t b0 = sdesc_b(smem_u32(Bs));
-            if (!ustream_gemm<UN>(ws, P0 + 16, 24, [&](int i) { return tmem + UN + UN * (i >> 3); },
-                              [&](int i) { return b0 + (uint64_t)(b_kstep_off(UN, i & 7) >> 4); },
-                              (uint64_t)(LF::HH >> 4), [](int) { return false; }))
-                ufail(ctl, 23);
-            mma_commit(mma_bar);
+            if (!ustream_gemm<UN, 3>(ws, P0 + 16 + g, 8, tmem + UN + UN * g,
+                                  [&](int i) { return b0 + (uint64_t)(b_kstep_off(UN, i) >> 4); },
+                                  (uint64_t)(LF::HH >> 4), false))
+                ufail(ctl2, 23);
+            mma_commit(chunk_bar);
         }
+        __syncwarp();
         if (producer && !ustream_fill(ws, min(P0 + 40, P_end))) ufail(ctl, 28);
-        uwait_mma(ctl, w, 24);
+        uwait_mma(ctl2, w, 24);
         // the next tile's GEMM1 pairs arrive while this epilogue and the next build run
         if (producer && !ustream_fill(ws, min(P0 + 40 + LF::RING, P_end))) ufail(ctl, 29);
         {   // epilogue 2: (ds, g1, g2) -> ua; s' = s + ds, v' = v g1 + (M v) g2 (:452-468).
@@ -486,12 +496,12 @@ template <int UN>
 struct UBwd {
     static constexpr uint32_t AH = 6 * b_block(UN);
     static constexpr uint32_t ZH = 2 * b_block(UN);
-    static constexpr int RING = UN == 64 ? 2 : 7;
+    static constexpr int RING = UN == 64 ? 2 : 8;
     static constexpr uint32_t OFF_B = 0;
     static constexpr uint32_t OFF_RING = OFF_B + 2 * AH;
     static constexpr uint32_t OFF_MIX = OFF_RING + RING * A_PAIR;
     static constexpr uint32_t OFF_BAR = OFF_MIX + 64;
-    static constexpr uint32_t OFF_MISC = OFF_BAR + 8 * (1 + 2 * RING);
+    static constexpr uint32_t OFF_MISC = OFF_BAR + 8 * (2 + 2 * RING);
     static constexpr uint32_t SMEM = align1k(OFF_MISC + 16);
     static constexpr uint32_t TMEM_COLS = UN == 64 ? 256 : 128;   // 3 UN columns, a power of two
     static_assert(2 * (SMEM + 1024) <= 228 * 1024, "two update reverse CTAs per SM");
@@ -509,7 +519,8 @@ __global__ void __launch_bounds__(UNT, 2) update_bwd_tc_kernel(const float* __re
     unsigned char* Bs = smem + LB::OFF_B;
     float* mix = reinterpret_cast<float*>(smem + LB::OFF_MIX);
     uint64_t* mma_bar = reinterpret_cast<uint64_t*>(smem + LB::OFF_BAR);
-    uint64_t* full = mma_bar + 1;
+    uint64_t* chunk_bar = mma_bar + 1;   // the second GEMM: one commit per chunk
+    uint64_t* full = mma_bar + 2;
     uint64_t* empty = full + LB::RING;
     uint32_t* tslot = reinterpret_cast<uint32_t*>(smem + LB::OFF_MISC);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + LB::OFF_MISC + 4);
@@ -521,6 +532,7 @@ __global__ void __launch_bounds__(UNT, 2) update_bwd_tc_kernel(const float* __re
     }
     if (t == 0) {
         mbar_init(mma_bar, 1);
+        mbar_init(chunk_bar, 2);
         for (int i = 0; i < LB::RING; ++i) {
             mbar_init(&full[i], 1);
             mbar_init(&empty[i], 1);
@@ -535,8 +547,8 @@ __global__ void __launch_bounds__(UNT, 2) update_bwd_tc_kernel(const float* __re
     const uint32_t tmem = *tslot;
     UStream<LB::RING> ws{smem + LB::OFF_RING, full, empty,
                {reinterpret_cast<const unsigned char*>(P + lo.u2t_tc), reinterpret_cast<const unsigned char*>(P + lo.u1t_tc)},
-               {24, 16}, 0, 0};
-    UCtl ctl{mma_bar, abort_flag, st, 0};
+               {24, 16}, 0};
+    UCtl ctl{mma_bar, abort_flag, st, 0}, ctl2{chunk_bar, abort_flag, st, 0};
     const int my_tiles = blockIdx.x < ntiles ? (ntiles - 1 - blockIdx.x) / gridDim.x + 1 : 0;
     const uint32_t P_end = (uint32_t)my_tiles * 40;
     const bool producer = t == 32;
@@ -593,9 +605,8 @@ __global__ void __launch_bounds__(UNT, 2) update_bwd_tc_kernel(const float* __re
         if (t == 0) {   // GEMM3: zbar_pre^T = U2^T abar^T, K = 384
             fence_after_sync();
             const uint64_t b0 = sdesc_b(smem_u32(Bs));
-            if (!ustream_gemm<UN>(ws, P0, 24, [&](int) { return tmem; },
-                              [&](int i) { return b0 + (uint64_t)(b_kstep_off(UN, i) >> 4); }, (uint64_t)(LB::AH >> 4),
-                              [](int i) { return i == 0; }))
+            if (!ustream_gemm<UN, 1>(ws, P0, 24, tmem, [&](int i) { return b0 + (uint64_t)(b_kstep_off(UN, i) >> 4); },
+                                  (uint64_t)(LB::AH >> 4), true))
                 ufail(ctl, 31);
             mma_commit(mma_bar);
         }
@@ -622,17 +633,18 @@ __global__ void __launch_bounds__(UNT, 2) update_bwd_tc_kernel(const float* __re
         fence_async_smem();
         fence_before_sync();
         __syncthreads();
-        if (t == 0) {   // GEMM4: cb^T = U1^T zbar^T, 2 chunks x 8 K-steps
+        if (const int g = uissuer(w, lane); g >= 0 && g < 2) {   // GEMM4: cb^T = U1^T zbar^T, 2 chunks x 8 K-steps
             fence_after_sync();
             const uint64_t b0 = sdesc_b(smem_u32(Bs));
-            if (!ustream_gemm<UN>(ws, P0 + 24, 16, [&](int i) { return tmem + UN + UN * (i >> 3); },
-                              [&](int i) { return b0 + (uint64_t)(b_kstep_off(UN, i & 7) >> 4); },
-                              (uint64_t)(LB::ZH >> 4), [](int i) { return (i & 7) == 0; }))
-                ufail(ctl, 33);
-            mma_commit(mma_bar);
+            if (!ustream_gemm<UN, 2>(ws, P0 + 24 + g, 8, tmem + UN + UN * g,
+                                  [&](int i) { return b0 + (uint64_t)(b_kstep_off(UN, i) >> 4); },
+                                  (uint64_t)(LB::ZH >> 4), true))
+                ufail(ctl2, 33);
+            mma_commit(chunk_bar);
         }
+        __syncwarp();
         if (producer && !ustream_fill(ws, min(P0 + 40, P_end))) ufail(ctl, 38);
-        uwait_mma(ctl, w, 34);
+        uwait_mma(ctl2, w, 34);
         if (producer && !ustream_fill(ws, min(P0 + 40 + LB::RING, P_end))) ufail(ctl, 39);
         {   // epilogue 4: xtbar = (sb + cs, xb g1 + M^T xb g2 + cn v / |v|).  The
             // TMEM owner of channel c writes (cs, cn) of its 32 atoms to shared
