@@ -431,6 +431,22 @@ __device__ __forceinline__ void cols_free_sync(int pp, int n) {
     asm volatile("bar.sync %0, %1;" ::"r"(5 + pp), "r"(n) : "memory");
 }
 
+// One pipeline's GEMM2 at a time: sharing the tensor core evenly, the two
+// pipelines stay in step and then both wait for MMAs and both run epilogues;
+// taking turns, one's GEMM2 runs during the other's epilogues.  Lane 0 of the
+// pipeline's warp 0 takes the lock; true when it has it.
+__device__ __forceinline__ bool g2_acquire(const EdgeArgs& a, int* lock, volatile int* abort_flag) {
+    const long long t0 = clock64();
+    while (atomicCAS(lock, 0, 1) != 0) {
+        if (clock64() - t0 > WAIT_BUDGET) {
+            signal_timeout(a, abort_flag, 10);
+            return false;
+        }
+        __nanosleep(32);
+    }
+    return true;
+}
+
 // ------------------------------------------------------- forward kernel
 // 64-edge tiles per pipeline: GEMM1 (z = W1 e, two N = 32 halves, one per
 // [E; E'] tile) into the columns of the pipeline's chunk 0, epilogue 1
@@ -442,6 +458,16 @@ __device__ __forceinline__ void cols_free_sync(int pp, int n) {
 // receiver.  Padding edges of a partition's last tile get h = 0 and a zero
 // bias fill (a fix-up after epilogue 1): their filter is exactly zero and
 // every gather runs unpredicated.
+//
+// L0, the first layer: v = 0, so chunk 1 (phi_v1) is left out, and the next
+// tile's z goes to its columns: GEMM1 runs during epilogue 2 instead of after
+// it (16,900 atoms, 860,000 edges: 418 -> 372 us).
+//
+// Another layer's 64-edge tile takes 16,200 cycles: GEMM1 1300, epilogue 1
+// 2400, GEMM2 6300 (72 MMAs of 48-50, the commit's latency, the first
+// gathers), epilogue 2 5000, barriers the rest.  425 -> 410 us by taking turns
+// in GEMM2 (g2_acquire), issuing a tile's MMAs before its gathers and GEMM1's
+// halves from two threads.
 constexpr int QN = 64;                               // edges per forward tile
 constexpr uint32_t Q_HH = 2 * b_block(QN);           // one half (hi or lo) of the H tile: 16 KB
 constexpr uint32_t Q_SB_US = 0;
@@ -465,6 +491,7 @@ static_assert(4 * ET_E <= 2 * Q_HH, "the E rows of two [E; E'] tiles fit in the 
 static_assert(Q_SB_BYTES % 16 == 0, "edge array alignment");
 static_assert(Q_SMEM <= 232448, "forward kernel shared memory");
 
+template <bool L0>
 __global__ void __launch_bounds__(NT, 1) edge_fwd_tc_kernel(EdgeArgs a, const unsigned char* __restrict__ w1g,
                                                             const unsigned char* __restrict__ w2g) {
     extern __shared__ __align__(1024) unsigned char smem[];
@@ -478,6 +505,7 @@ __global__ void __launch_bounds__(NT, 1) edge_fwd_tc_kernel(EdgeArgs a, const un
     uint64_t* never_bar = bars + 1;                 // test hook: nothing arrives here
     uint32_t* tslot = reinterpret_cast<uint32_t*>(smem + Q_OFF_MISC);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + Q_OFF_MISC + 4);
+    int* g2_lock = reinterpret_cast<int*>(smem + Q_OFF_MISC + 8);
 
     // waits for the previous kernel at entry: reading the status word first
     // and returning early keeps the main loop's register allocation lean
@@ -492,12 +520,13 @@ __global__ void __launch_bounds__(NT, 1) edge_fwd_tc_kernel(EdgeArgs a, const un
         mbar_init(w2h_bar, 1);
         mbar_init(never_bar, 1);
         for (int p = 0; p < 2; ++p) {
-            mbar_init(bars + 2 + 3 * p, 1);   // GEMM1
-            mbar_init(bars + 3 + 3 * p, 1);   // E tile
-            mbar_init(bars + 4 + 3 * p, 3);   // GEMM2: one commit per chunk issuer
+            mbar_init(bars + 2 + 3 * p, 2);            // GEMM1: one commit per half
+            mbar_init(bars + 3 + 3 * p, 1);            // E tile
+            mbar_init(bars + 4 + 3 * p, L0 ? 2 : 3);   // GEMM2: one commit per chunk issuer
         }
         fence_mbar_init();
         *abort_flag = 0;
+        *g2_lock = 0;
     }
     for (int i = t; i < (int)(W1_BYTES / 16); i += NT)
         reinterpret_cast<uint4*>(w1s)[i] = reinterpret_cast<const uint4*>(w1g)[i];
@@ -522,6 +551,7 @@ __global__ void __launch_bounds__(NT, 1) edge_fwd_tc_kernel(EdgeArgs a, const un
     // ---- this thread's pipeline
     const int pp = w >> 3, wl = w & 7, tp = t & (PT - 1), hh = wl >> 2;
     const uint32_t TB = 128 + 192 * pp;             // the pipeline's TMEM columns: chunk g at TB + 64 g
+    const uint32_t TZ = TB + (L0 ? 64 : 0);         // z: in chunk 0's columns, L0 chunk 1's
     unsigned char* Hs = smem + Q_OFF_H + pp * 2 * Q_HH;   // H hi, then lo
     unsigned char* Es = Hs;                         // [E; E'] tiles (bulk-copied) before H is written
     uint64_t* mma_bar = bars + 2 + 3 * pp;
@@ -546,15 +576,16 @@ __global__ void __launch_bounds__(NT, 1) edge_fwd_tc_kernel(EdgeArgs a, const un
         fetch_tile_edges(a, tp, QN, t0, nn, reinterpret_cast<float4*>(sbx + Q_SB_US),
                          reinterpret_cast<int*>(sbx + Q_SB_SRC), reinterpret_cast<int*>(sbx + Q_SB_RCV));
     };
-    // z^T = W1 e^T into chunk 0's columns, once the copies have landed
-    // (thread tp 0): the tile's 64 edges are the E rows (0-31) of nt
-    // consecutive [E; E'] tiles, copied to Es (edges 32 j .. 32 j + 31 from
-    // tile j: its hi E rows at 4 KB j, its lo E rows 2 KB further)
-    auto issue_gemm1 = [&](int nt) {
+    // half j of z^T = W1 e^T into its columns, once the copies have landed
+    // (lane 0 of warp j < 2: a thread spends 72 cycles on each of the 6 MMAs):
+    // the tile's 64 edges are the E rows (0-31) of nt consecutive [E; E']
+    // tiles, copied to Es (edges 32 j .. 32 j + 31 from tile j: its hi E rows
+    // at 4 KB j, its lo E rows 2 KB further)
+    auto issue_gemm1 = [&](int j, int nt) {
         if (!mbar_wait(e_bar, e_phase, WAIT_BUDGET)) signal_timeout(a, abort_flag, 8);
         fence_after_sync();
         constexpr uint32_t idesc = idesc_f16(32);
-        for (int j = 0; j < nt; ++j)
+        if (j < nt)
 #pragma unroll
             for (int s = 0; s < 2; ++s)
 #pragma unroll
@@ -563,7 +594,7 @@ __global__ void __launch_bounds__(NT, 1) edge_fwd_tc_kernel(EdgeArgs a, const un
                     const uint64_t ad = sdesc(smem_u32(w1s + s * SLAB + ahl * A_TILE), A_LBO, A_SBO);
                     const uint64_t bd =
                         sdesc(smem_u32(Es + j * 2 * ET_E + bhl * ET_E + s * 2 * ET_LBO), ET_LBO, ET_SBO);
-                    mma_f16(tmem + TB + 32 * j, ad, bd, idesc, (s | pr) != 0);
+                    mma_f16(tmem + TZ + 32 * j, ad, bd, idesc, (s | pr) != 0);
                 }
         mma_commit(mma_bar);
     };
@@ -597,6 +628,10 @@ __global__ void __launch_bounds__(NT, 1) edge_fwd_tc_kernel(EdgeArgs a, const un
             pipe_sync(pp);
             if (tp < QN) prep(sbase, min(QN, e1 - e0), j0);
             pipe_sync(pp);
+            if (L0) {
+                if (wl < 2 && lane == 0) issue_gemm1(wl, (min(QN, e1 - e0) + 31) / 32);
+                e_phase ^= 1;
+            }
         }
         for (int k = 0; k < ntl; ++k) {
             const int t0 = e0 + k * QN, n = min(QN, e1 - t0), buf = k & 1;
@@ -608,10 +643,12 @@ __global__ void __launch_bounds__(NT, 1) edge_fwd_tc_kernel(EdgeArgs a, const un
             const uint32_t* chg = reinterpret_cast<const uint32_t*>(sb + Q_SB_CHG);
             // z^T = W1 e^T on the bulk-copied tile, into chunk 0's columns (read
             // by the scalar warps until the end of the previous tile's epilogue 2)
-            if (tp == 0) issue_gemm1((n + 31) / 32);
-            e_phase ^= 1;
+            if (!L0) {
+                if (wl < 2 && lane == 0) issue_gemm1(wl, (n + 31) / 32);
+                e_phase ^= 1;
+            }
+            if (wl < 2) __syncwarp();
             if (wl == 0) {
-                __syncwarp();
                 // one warp polls the MMA barrier; the others wait at the pipeline barrier
                 if ((a.stall_test & 1) && k == 0 && !mbar_wait(never_bar, 0, STALL_BUDGET))
                     signal_timeout(a, abort_flag, WHERE_STALL_TEST);
@@ -628,12 +665,14 @@ __global__ void __launch_bounds__(NT, 1) edge_fwd_tc_kernel(EdgeArgs a, const un
                 const BColumn hc(Hs, Q_HH, QN, col, c);
                 // GEMM2 accumulates onto b2 (0 for padding edges): this warp refills the
                 // chunk-0 cells it has just read and all 64 columns of chunk 1 + hh
+                // (L0: its edges' columns of chunks 0 and 2)
                 float bv[16];
-                const float b0c = b2s[c], bch = b2s[(1 + hh) * H + c];
+                const int ch = L0 ? 2 : 1 + hh;
+                const float b0c = b2s[c], bch = b2s[ch * H + c];
 #pragma unroll
                 for (int i0 = 0; i0 < 32; i0 += 16) {   // 16 edges per TMEM load
                     float z[16];
-                    tmem_ld16(lane_base + TB + col + i0, z);
+                    tmem_ld16(lane_base + TZ + col + i0, z);
                     tmem_ld_wait();
 #pragma unroll
                     for (int i = 0; i < 16; i += 2) {
@@ -647,8 +686,13 @@ __global__ void __launch_bounds__(NT, 1) edge_fwd_tc_kernel(EdgeArgs a, const un
                 tmem_st16(lane_base + TB + col + 16, bv);
 #pragma unroll
                 for (int i = 0; i < 16; ++i) bv[i] = bch;
+                if (L0) {
+                    tmem_st16(lane_base + TB + 128 + col, bv);
+                    tmem_st16(lane_base + TB + 128 + col + 16, bv);
+                } else {
 #pragma unroll
-                for (int kk = 0; kk < 4; ++kk) tmem_st16(lane_base + TB + 64 * (1 + hh) + 16 * kk, bv);
+                    for (int kk = 0; kk < 4; ++kk) tmem_st16(lane_base + TB + 64 * ch + 16 * kk, bv);
+                }
                 if (n < QN) {   // the last tile of a partition: its padding edges get h = 0 and no bias
                     tmem_st_wait();   // the fills above land before the zeros below
 #pragma unroll 1
@@ -656,32 +700,41 @@ __global__ void __launch_bounds__(NT, 1) edge_fwd_tc_kernel(EdgeArgs a, const un
 #pragma unroll 1
                     for (int i = max(nv, 0); i < 32; ++i) tmem_st1(lane_base + TB + col + i, 0.f);
 #pragma unroll 1
-                    for (int i = n; i < QN; ++i) tmem_st1(lane_base + TB + 64 * (1 + hh) + i, 0.f);
+                    for (int i = L0 ? col + max(nv, 0) : n; i < (L0 ? col + 32 : QN); ++i)
+                        tmem_st1(lane_base + TB + 64 * ch + i, 0.f);
                 }
                 tmem_st_wait();
             }
             fence_async_smem();
             fence_before_sync();
+            bool locked = false;
+            if (wl == 0) {
+                if (lane == 0) locked = g2_acquire(a, g2_lock, abort_flag);
+                __syncwarp();
+            }
             pipe_sync(pp);
             // epilogue 2's first two 8-edge blocks of sender features are
             // gathered while GEMM2 runs (padding edges read row 0)
             float xa0[8], xa1[8], xb0[8], xb1[8];
             auto gather8 = [&](float (&x0)[8], float (&x1)[8], int col) {
+                if (L0 && hh != 0) return;
 #pragma unroll
                 for (int i = 0; i < 8; i += 4) {
                     const int4 so = *reinterpret_cast<const int4*>(soff + col + i);
                     const int sv[4] = {so.x, so.y, so.z, so.w};
 #pragma unroll
                     for (int j = 0; j < 4; ++j) {
-                        const float2 v = __ldg(xx + sv[j]);
-                        x0[i + j] = v.x;
-                        x1[i + j] = v.y;
+                        if (L0) {
+                            x0[i + j] = __ldg(reinterpret_cast<const float*>(xx + sv[j]));
+                        } else {
+                            const float2 v = __ldg(xx + sv[j]);
+                            x0[i + j] = v.x;
+                            x1[i + j] = v.y;
+                        }
                     }
                 }
             };
-            gather8(xa0, xa1, 0);
-            if (8 < n) gather8(xb0, xb1, 8);
-            if (wl < 3 && lane == 0) {   // f^T = W2 h^T, chunk wl issued by warp wl
+            if (wl < 3 && lane == 0 && !(L0 && wl == 1)) {   // f^T = W2 h^T, chunk wl issued by warp wl
                 fence_after_sync();
                 if (!w2h_ready) {
                     if (!mbar_wait(w2h_bar, 0, WAIT_BUDGET)) signal_timeout(a, abort_flag, 6);
@@ -691,7 +744,10 @@ __global__ void __launch_bounds__(NT, 1) edge_fwd_tc_kernel(EdgeArgs a, const un
                 mma_commit(g2_bar);
             }
             if (wl < 3) __syncwarp();   // lanes 1-31 of the issuing warps wait here, not in a spin loop
+            gather8(xa0, xa1, 0);
+            if (8 < n) gather8(xb0, xb1, 8);
             if (wl == 0 && !mbar_wait(g2_bar, g2_phase, WAIT_BUDGET)) signal_timeout(a, abort_flag, 4);
+            if (locked) atomicExch(g2_lock, 0);
             g2_phase ^= 1;
             fence_before_sync();
             // the abort decision is the same for every thread of the pipeline
@@ -714,7 +770,7 @@ __global__ void __launch_bounds__(NT, 1) edge_fwd_tc_kernel(EdgeArgs a, const un
                     constexpr int HH = decltype(hc)::value;
                     float fa[8], f1[8], f2[8];
                     if (HH == 0) tmem_ld8(lane_base + TB + col, fa);   // phi_s
-                    tmem_ld8(lane_base + TB + 64 + col, f1);            // phi_v1
+                    if (!L0) tmem_ld8(lane_base + TB + 64 + col, f1);   // phi_v1
                     tmem_ld8(lane_base + TB + 128 + col, f2);           // phi_v2
                     const uint32_t m = (chg[col >> 5] >> (col & 31)) & 0xFFu;
                     // the block's u components, two 16-byte shared loads per array
@@ -731,8 +787,10 @@ __global__ void __launch_bounds__(NT, 1) edge_fwd_tc_kernel(EdgeArgs a, const un
                     // both branches (a block's branch depends on where the tile starts)
                     auto add_m = [&](int i) {
                         if (HH == 0) acc0 = fmaf(x0[i], fa[i], acc0);
+                        else if (L0) acc0 = fmaf(ua[i], f2[i], acc0);
                         else acc0 = fmaf(x0[i], f1[i], fmaf(ua[i], f2[i], acc0));
-                        acc1 = fmaf(x1[i], f1[i], fmaf(ub[i], f2[i], acc1));
+                        if (L0) acc1 = fmaf(ub[i], f2[i], acc1);
+                        else acc1 = fmaf(x1[i], f1[i], fmaf(ub[i], f2[i], acc1));
                     };
                     if (m == 0) {
 #pragma unroll
@@ -754,6 +812,11 @@ __global__ void __launch_bounds__(NT, 1) edge_fwd_tc_kernel(EdgeArgs a, const un
                 };
                 auto blocks = [&](auto hc) {
                     for (int col = 0; col < n; col += 16) {   // blocks col and col + 8 are in flight
+                        if (L0 && col == QN / 2 && more) {   // the next tile's E rows have arrived by now
+                            if (wl < 2 && lane == 0)
+                                issue_gemm1(wl, (min(QN, e1 - t0 - QN) + 31) / 32);
+                            __syncwarp();
+                        }
                         process8(hc, xa0, xa1, col);
                         if (col + 8 >= n) break;
                         if (col + 16 < n) gather8(xa0, xa1, col + 16);
@@ -764,6 +827,7 @@ __global__ void __launch_bounds__(NT, 1) edge_fwd_tc_kernel(EdgeArgs a, const un
                 if (hh == 0) blocks(std::integral_constant<int, 0>{});
                 else blocks(std::integral_constant<int, 1>{});
             }
+            if (L0 && more) e_phase ^= 1;
             if (more && tp < QN) {   // the next tile's prep, by the two warps that fetched it
                 cp_async_wait_all();
                 pipe_sync_first(pp, QN);
@@ -1590,19 +1654,23 @@ static int tc_grid(int nparts) {
     return std::max(1, std::min(sms, nparts));
 }
 
-int launch_edge_fwd_tc(const EdgeArgs& a, int layer, cudaStream_t st) {
-    (void)layer;
+template <bool L0>
+static int launch_edge_fwd_tc_t(const EdgeArgs& a, cudaStream_t st) {
     static std::once_flag once;
     static cudaError_t attr_err = cudaSuccess;
     std::call_once(once, [] {
-        attr_err = cudaFuncSetAttribute(edge_fwd_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Q_SMEM);
+        attr_err = cudaFuncSetAttribute(edge_fwd_tc_kernel<L0>, cudaFuncAttributeMaxDynamicSharedMemorySize, Q_SMEM);
     });
     if (attr_err != cudaSuccess) return cuda_status(attr_err, "edge_fwd_tc smem attribute");
     const unsigned char* w1 = reinterpret_cast<const unsigned char*>(a.P + a.lo.w1_bf);
     const unsigned char* w2 = reinterpret_cast<const unsigned char*>(a.P + a.lo.w2_bf);
     // two pipelines (partitions) per CTA
-    MLFF_LAUNCH_PDL("edge_fwd_tc", edge_fwd_tc_kernel, tc_grid((a.nparts + 1) / 2), NT, Q_SMEM, st, a, w1, w2);
+    MLFF_LAUNCH_PDL("edge_fwd_tc", edge_fwd_tc_kernel<L0>, tc_grid((a.nparts + 1) / 2), NT, Q_SMEM, st, a, w1, w2);
     return MLFF_OK;
+}
+
+int launch_edge_fwd_tc(const EdgeArgs& a, int layer, cudaStream_t st) {
+    return layer == 0 ? launch_edge_fwd_tc_t<true>(a, st) : launch_edge_fwd_tc_t<false>(a, st);
 }
 
 int launch_edge_bwd_tc(const EdgeArgs& a, int layer, cudaStream_t st) {
