@@ -67,7 +67,20 @@ int pack_update_tc(const mlff_dims& d, float* out, const PackedOffsets& o, cudaS
 }
 
 // ------------------------------------------------------- weight stream
-constexpr int UNT = 256;
+// Threads per CTA: 256, two CTAs per SM; or 512 when one tile per SM is all
+// there is (UThreads).  A CTA's warps are GRP groups of four TMEM lane
+// quarters, a group holding UN / GRP of the tile's atoms.
+template <int UN, int NT>
+struct UThreads {
+    static constexpr int WARPS = NT / 32, GRP = NT / 128, NC = UN / GRP;
+    static_assert(NC == 8 || NC == 16 || NC == 32, "atoms per group");
+};
+template <int NC>
+__device__ __forceinline__ void uload(uint32_t taddr, float (&v)[NC]) {
+    if constexpr (NC == 32) tmem_ld32(taddr, v);
+    else if constexpr (NC == 16) tmem_ld16(taddr, v);
+    else tmem_ld8(taddr, v);
+}
 
 template <int URING>
 struct UStream {
@@ -139,11 +152,18 @@ __device__ __forceinline__ bool ustream_gemm(UStream<URING>& s, uint32_t P0, int
 // warp 1), -1 for the others.
 __device__ __forceinline__ int uissuer(int w, int lane) { return lane != 0 || w == 1 || w > 3 ? -1 : w == 0 ? 0 : w - 1; }
 
-__device__ __forceinline__ void ufill_tmem(uint32_t taddr, float v, int n16) {
-    float bv[16];
+template <int NC>
+__device__ __forceinline__ void ufill_tmem(uint32_t taddr, float v) {
+    if constexpr (NC == 8) {
+        const float bv[8] = {v, v, v, v, v, v, v, v};
+        tmem_st8(taddr, bv);
+    } else {
+        float bv[16];
 #pragma unroll
-    for (int i = 0; i < 16; ++i) bv[i] = v;
-    for (int k = 0; k < n16; ++k) tmem_st16(taddr + 16 * k, bv);
+        for (int i = 0; i < 16; ++i) bv[i] = v;
+#pragma unroll
+        for (int k = 0; k < NC / 16; ++k) tmem_st16(taddr + 16 * k, bv);
+    }
 }
 
 // four consecutive K values (k % 4 == 0) of one row as split fp16
@@ -234,13 +254,15 @@ struct UFwd {
     static_assert(2 * (SMEM + 1024) <= 228 * 1024, "two update CTAs per SM");
 };
 
-template <int UN>
-__global__ void __launch_bounds__(UNT, 2) update_fwd_tc_kernel(const float* __restrict__ P, LayerOffsets lo,
+template <int UN, int NT>
+__global__ void __launch_bounds__(NT, NT == 512 ? 1 : 2) update_fwd_tc_kernel(const float* __restrict__ P, LayerOffsets lo,
                                                                const float* __restrict__ Xt, int32_t n_atoms,
                                                                float* __restrict__ Xout, int out_layout,
                                                                float* __restrict__ uz, float* __restrict__ ua,
                                                                Status* st) {
     using LF = UFwd<UN>;
+    using UT = UThreads<UN, NT>;
+    constexpr int NC = UT::NC, WARPS = UT::WARPS;
     extern __shared__ __align__(1024) unsigned char smem[];
     unsigned char* Bs = smem + LF::OFF_B;
     float* mix = reinterpret_cast<float*>(smem + LF::OFF_MIX);
@@ -292,17 +314,17 @@ __global__ void __launch_bounds__(UNT, 2) update_fwd_tc_kernel(const float* __re
     for (int tile = blockIdx.x; tile < ntiles && !*abort_flag; tile += gridDim.x, P0 += 40) {
         const int a0 = tile * UN;
         // accumulators <- bias: D1 c1, D2 chunk g c2[g]
-        ufill_tmem(lane_base + (UN / 2) * hh, c1c, UN / 32);
+        ufill_tmem<NC>(lane_base + NC * hh, c1c);
 #pragma unroll
-        for (int g = 0; g < 3; ++g) ufill_tmem(lane_base + UN + UN * g + (UN / 2) * hh, c2c[g], UN / 32);
-        // B tile: row = atom, K = [s (128), |v| (128)]; warp w builds rows w, w + 8, ...,
-        // two rows per step so that their loads overlap
+        for (int g = 0; g < 3; ++g) ufill_tmem<NC>(lane_base + UN + UN * g + NC * hh, c2c[g]);
+        // B tile: row = atom, K = [s (128), |v| (128)]; warp w builds rows w, w + WARPS,
+        // ..., two rows per step so that their loads overlap
 #pragma unroll 1
-        for (int i0 = w; i0 < UN; i0 += 16) {
+        for (int i0 = w; i0 < UN; i0 += 2 * WARPS) {
             float4 r[2][4];
 #pragma unroll
             for (int k = 0; k < 2; ++k) {
-                const int a = a0 + i0 + 8 * k;
+                const int a = a0 + i0 + WARPS * k;
                 const float4* x = reinterpret_cast<const float4*>(Xt + (int64_t)(a < n_atoms ? a : 0) * 4 * H);
 #pragma unroll
                 for (int j = 0; j < 4; ++j) r[k][j] = a < n_atoms ? x[32 * j + lane] : make_float4(0.f, 0.f, 0.f, 0.f);
@@ -312,8 +334,8 @@ __global__ void __launch_bounds__(UNT, 2) update_fwd_tc_kernel(const float* __re
                 const float4 vx = r[k][1], vy = r[k][2], vz = r[k][3];
                 const float4 nv = make_float4(pair_distance(vx.x, vy.x, vz.x), pair_distance(vx.y, vy.y, vz.y),
                                               pair_distance(vx.z, vy.z, vz.z), pair_distance(vx.w, vy.w, vz.w));  // |v| (:437)
-                store_row4(Bs, LF::BH, UN, i0 + 8 * k, 4 * lane, r[k][0]);
-                store_row4(Bs, LF::BH, UN, i0 + 8 * k, H + 4 * lane, nv);
+                store_row4(Bs, LF::BH, UN, i0 + WARPS * k, 4 * lane, r[k][0]);
+                store_row4(Bs, LF::BH, UN, i0 + WARPS * k, H + 4 * lane, nv);
             }
         }
         tmem_st_wait();
@@ -333,11 +355,9 @@ __global__ void __launch_bounds__(UNT, 2) update_fwd_tc_kernel(const float* __re
         // GEMM1 is done, so every slot is free: fetch GEMM2's pairs during epilogue 1
         if (producer && !ustream_fill(ws, min(P0 + 16 + LF::RING, P_end))) ufail(ctl, 27);
         {   // epilogue 1: z -> uz, h = silu(z) -> H tile (aliases the B tile)
-            constexpr int NC = UN / 2;   // this warp half's atoms
-            const int col = NC * hh;
+            const int col = NC * hh;   // this group's atoms
             float z[NC];
-            if constexpr (NC == 32) tmem_ld32(lane_base + col, z);
-            else tmem_ld16(lane_base + col, z);
+            uload(lane_base + col, z);
             tmem_ld_wait();
             const BColumn hcol(Bs, LF::HH, UN, col, c);
 #pragma unroll
@@ -374,30 +394,30 @@ __global__ void __launch_bounds__(UNT, 2) update_fwd_tc_kernel(const float* __re
             float* T = reinterpret_cast<float*>(Bs);      // [3][32 atoms][H]
 #pragma unroll 1
             for (int pass = 0; pass < UN / 32; ++pass) {
-                if (hh == pass) {
+                if (NC * hh / 32 == pass) {
 #pragma unroll 1
                     for (int g = 0; g < 3; ++g) {
-                        float v[32];
-                        tmem_ld32(lane_base + UN + UN * g + 32 * pass, v);
+                        float v[NC];
+                        uload(lane_base + UN + UN * g + NC * hh, v);
                         tmem_ld_wait();
 #pragma unroll
-                        for (int i = 0; i < 32; ++i) T[(g * 32 + i) * H + c] = v[i];
+                        for (int i = 0; i < NC; ++i) T[(g * 32 + NC * hh % 32 + i) * H + c] = v[i];
                     }
                 }
                 __syncthreads();
 #pragma unroll 1
-                for (int i0 = w; i0 < 32; i0 += 16) {
+                for (int i0 = w; i0 < 32; i0 += 2 * WARPS) {
                     float4 x[2][4];
 #pragma unroll
                     for (int k = 0; k < 2; ++k) {
-                        const int a = a0 + 32 * pass + i0 + 8 * k;
+                        const int a = a0 + 32 * pass + i0 + WARPS * k;
                         const float4* xr = reinterpret_cast<const float4*>(Xt + (int64_t)(a < n_atoms ? a : 0) * 4 * H);
 #pragma unroll
                         for (int j = 0; j < 4; ++j) x[k][j] = a < n_atoms ? xr[32 * j + lane] : make_float4(0.f, 0.f, 0.f, 0.f);
                     }
 #pragma unroll
                     for (int k = 0; k < 2; ++k) {
-                        const int i = i0 + 8 * k, a = a0 + 32 * pass + i;
+                        const int i = i0 + WARPS * k, a = a0 + 32 * pass + i;
                         if (a >= n_atoms) continue;
                         const float4 ds = reinterpret_cast<const float4*>(T + (0 * 32 + i) * H)[lane];
                         const float4 g1 = reinterpret_cast<const float4*>(T + (1 * 32 + i) * H)[lane];
@@ -453,14 +473,17 @@ __global__ void __launch_bounds__(UNT, 2) update_fwd_tc_kernel(const float* __re
 }
 
 // UN-atom tiles, two CTAs per SM: one CTA's epilogues overlap the other's
-// weight stream and MMAs
-template <int UN>
+// weight stream and MMAs.  Up to one tile per SM there is no other CTA, and
+// 512 threads halve the build and the epilogues, 19,000 of a 32-atom tile's
+// 31,000 cycles with 256 (a water box of 3000 atoms 928 -> 887 us a call).
+static bool one_tile_per_sm(const WsLayout& L) { return (L.N + L.UT - 1) / L.UT <= num_sms(); }
+template <int UN, int NT>
 static int launch_update_fwd_tc_t(const float* packed, const LayerOffsets& lo, const WsLayout& L, void* ws, int layer,
                                   cudaStream_t st) {
     static std::once_flag once;
     static cudaError_t attr_err = cudaSuccess;
     std::call_once(once, [] {
-        attr_err = cudaFuncSetAttribute(update_fwd_tc_kernel<UN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        attr_err = cudaFuncSetAttribute(update_fwd_tc_kernel<UN, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                         UFwd<UN>::SMEM);
     });
     if (attr_err != cudaSuccess) return cuda_status(attr_err, "update_fwd_tc smem attribute");
@@ -475,15 +498,16 @@ static int launch_update_fwd_tc_t(const float* packed, const LayerOffsets& lo, c
     // the next layer's input in the layout of the edge kernels' gathers; the
     // last layer's output (read by the readout) component-major
     const int out_layout = layer + 1 < L.L ? L.gather : GATHER_ROWS;
-    MLFF_LAUNCH_PDL("update_fwd_tc", update_fwd_tc_kernel<UN>, grid, UNT, UFwd<UN>::SMEM, st, packed, lo, Xt, L.N,
+    MLFF_LAUNCH_PDL("update_fwd_tc", (update_fwd_tc_kernel<UN, NT>), grid, NT, UFwd<UN>::SMEM, st, packed, lo, Xt, L.N,
                     Xout, out_layout, uz, ua, ws_ptr<Status>(ws, L.status));
     return MLFF_OK;
 }
 
 int launch_update_fwd_tc(const float* packed, const LayerOffsets& lo, const WsLayout& L, void* ws, int layer,
                          cudaStream_t st) {
-    return L.UT == 32 ? launch_update_fwd_tc_t<32>(packed, lo, L, ws, layer, st)
-                      : launch_update_fwd_tc_t<64>(packed, lo, L, ws, layer, st);
+    if (L.UT != 32) return launch_update_fwd_tc_t<64, 256>(packed, lo, L, ws, layer, st);
+    return one_tile_per_sm(L) ? launch_update_fwd_tc_t<32, 512>(packed, lo, L, ws, layer, st)
+                              : launch_update_fwd_tc_t<32, 256>(packed, lo, L, ws, layer, st);
 }
 
 // ------------------------------------------------------- reverse kernel
@@ -508,13 +532,15 @@ struct UBwd {
     static_assert(2 * UN * H * 4 <= 2 * AH, "epilogue 4 stages (cs, cn) of the tile in the abar region");
 };
 
-template <int UN>
-__global__ void __launch_bounds__(UNT, 2) update_bwd_tc_kernel(const float* __restrict__ P, LayerOffsets lo,
+template <int UN, int NT>
+__global__ void __launch_bounds__(NT, NT == 512 ? 1 : 2) update_bwd_tc_kernel(const float* __restrict__ P, LayerOffsets lo,
                                                                const float* __restrict__ Xt, const float* __restrict__ uz,
                                                                const float* __restrict__ ua,
                                                                const float* __restrict__ xbo, int32_t n_atoms,
                                                                float* __restrict__ xtbar, int out_layout, Status* st) {
     using LB = UBwd<UN>;
+    using UT = UThreads<UN, NT>;
+    constexpr int NC = UT::NC, WARPS = UT::WARPS;
     extern __shared__ __align__(1024) unsigned char smem[];
     unsigned char* Bs = smem + LB::OFF_B;
     float* mix = reinterpret_cast<float*>(smem + LB::OFF_MIX);
@@ -572,11 +598,11 @@ __global__ void __launch_bounds__(UNT, 2) update_bwd_tc_kernel(const float* __re
                  b_z * (mix[6] * v_x + mix[7] * v_y + mix[8] * v_z);
         };
 #pragma unroll 1
-        for (int i0 = w; i0 < UN; i0 += 16) {
+        for (int i0 = w; i0 < UN; i0 += 2 * WARPS) {
             float4 r[2][7];
 #pragma unroll
             for (int k = 0; k < 2; ++k) {
-                const int a = a0 + i0 + 8 * k;
+                const int a = a0 + i0 + WARPS * k;
                 const int64_t aa = a < n_atoms ? a : 0;
                 const float4* xo = reinterpret_cast<const float4*>(xbo + aa * 4 * H);
                 const float4* x = reinterpret_cast<const float4*>(Xt + aa * 4 * H);
@@ -593,7 +619,7 @@ __global__ void __launch_bounds__(UNT, 2) update_bwd_tc_kernel(const float* __re
                 gpart(bx.y, by.y, bz.y, vx.y, vy.y, vz.y, g1.y, g2.y);
                 gpart(bx.z, by.z, bz.z, vx.z, vy.z, vz.z, g1.z, g2.z);
                 gpart(bx.w, by.w, bz.w, vx.w, vy.w, vz.w, g1.w, g2.w);
-                const int i = i0 + 8 * k;
+                const int i = i0 + WARPS * k;
                 store_row4(Bs, LB::AH, UN, i, 4 * lane, r[k][0]);
                 store_row4(Bs, LB::AH, UN, i, H + 4 * lane, g1);
                 store_row4(Bs, LB::AH, UN, i, 2 * H + 4 * lane, g2);
@@ -614,11 +640,9 @@ __global__ void __launch_bounds__(UNT, 2) update_bwd_tc_kernel(const float* __re
         uwait_mma(ctl, w, 32);
         if (producer && !ustream_fill(ws, min(P0 + 24 + LB::RING, P_end))) ufail(ctl, 37);
         {   // epilogue 3: zbar = D3 silu'(uz) -> zbar tile (aliases the abar tile)
-            constexpr int NC = UN / 2;   // this warp half's atoms
-            const int col = NC * hh;
+            const int col = NC * hh;   // this group's atoms
             float zb[NC];
-            if constexpr (NC == 32) tmem_ld32(lane_base + col, zb);
-            else tmem_ld16(lane_base + col, zb);
+            uload(lane_base + col, zb);
             float zz[NC];
 #pragma unroll
             for (int i = 0; i < NC; ++i) {
@@ -653,21 +677,19 @@ __global__ void __launch_bounds__(UNT, 2) update_bwd_tc_kernel(const float* __re
             float* T = reinterpret_cast<float*>(Bs);      // [2][UN atoms][H]
 #pragma unroll 1
             for (int g = 0; g < 2; ++g) {
-                constexpr int NC = UN / 2;
                 float v[NC];
-                if constexpr (NC == 32) tmem_ld32(lane_base + UN + UN * g + NC * hh, v);
-                else tmem_ld16(lane_base + UN + UN * g + NC * hh, v);
+                uload(lane_base + UN + UN * g + NC * hh, v);
                 tmem_ld_wait();
 #pragma unroll
                 for (int i = 0; i < NC; ++i) T[(g * UN + NC * hh + i) * H + c] = v[i];
             }
             __syncthreads();
 #pragma unroll 1
-            for (int i0 = w; i0 < UN; i0 += 16) {
+            for (int i0 = w; i0 < UN; i0 += 2 * WARPS) {
                 float4 r[2][9];
 #pragma unroll
                 for (int k = 0; k < 2; ++k) {
-                    const int a = a0 + i0 + 8 * k;
+                    const int a = a0 + i0 + WARPS * k;
                     const int64_t aa = a < n_atoms ? a : 0;
                     const float4* xo = reinterpret_cast<const float4*>(xbo + aa * 4 * H);
                     const float4* x = reinterpret_cast<const float4*>(Xt + aa * 4 * H);
@@ -681,7 +703,7 @@ __global__ void __launch_bounds__(UNT, 2) update_bwd_tc_kernel(const float* __re
                 }
 #pragma unroll
                 for (int k = 0; k < 2; ++k) {
-                    const int i = i0 + 8 * k, a = a0 + i;
+                    const int i = i0 + WARPS * k, a = a0 + i;
                     if (a >= n_atoms) continue;
                     const float4 cs = reinterpret_cast<const float4*>(T + i * H)[lane];
                     const float4 cn = reinterpret_cast<const float4*>(T + (UN + i) * H)[lane];
@@ -726,13 +748,13 @@ __global__ void __launch_bounds__(UNT, 2) update_bwd_tc_kernel(const float* __re
     if (w == 0) tmem_dealloc(tmem, LB::TMEM_COLS);
 }
 
-template <int UN>
+template <int UN, int NT>
 static int launch_update_bwd_tc_t(const float* packed, const LayerOffsets& lo, const WsLayout& L, void* ws, int layer,
                                   const float* xbar_out, float* xtbar, cudaStream_t st) {
     static std::once_flag once;
     static cudaError_t attr_err = cudaSuccess;
     std::call_once(once, [] {
-        attr_err = cudaFuncSetAttribute(update_bwd_tc_kernel<UN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        attr_err = cudaFuncSetAttribute(update_bwd_tc_kernel<UN, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                         UBwd<UN>::SMEM);
     });
     if (attr_err != cudaSuccess) return cuda_status(attr_err, "update_bwd_tc smem attribute");
@@ -743,15 +765,16 @@ static int launch_update_bwd_tc_t(const float* packed, const LayerOffsets& lo, c
     const float* ua = ws_ptr<float>(ws, L.ua) + (int64_t)layer * L.N * H3;
     const int ntiles = (L.N + UN - 1) / UN;
     const int grid = std::max(1, std::min(ntiles, 2 * num_sms()));
-    MLFF_LAUNCH_PDL("update_bwd_tc", update_bwd_tc_kernel<UN>, grid, UNT, UBwd<UN>::SMEM, st, packed, lo, Xt, uz, ua,
+    MLFF_LAUNCH_PDL("update_bwd_tc", (update_bwd_tc_kernel<UN, NT>), grid, NT, UBwd<UN>::SMEM, st, packed, lo, Xt, uz, ua,
                     xbar_out, L.N, xtbar, L.gather_bar, ws_ptr<Status>(ws, L.status));
     return MLFF_OK;
 }
 
 int launch_update_bwd_tc(const float* packed, const LayerOffsets& lo, const WsLayout& L, void* ws, int layer,
                          const float* xbar_out, float* xtbar, cudaStream_t st) {
-    return L.UT == 32 ? launch_update_bwd_tc_t<32>(packed, lo, L, ws, layer, xbar_out, xtbar, st)
-                      : launch_update_bwd_tc_t<64>(packed, lo, L, ws, layer, xbar_out, xtbar, st);
+    if (L.UT != 32) return launch_update_bwd_tc_t<64, 256>(packed, lo, L, ws, layer, xbar_out, xtbar, st);
+    return one_tile_per_sm(L) ? launch_update_bwd_tc_t<32, 512>(packed, lo, L, ws, layer, xbar_out, xtbar, st)
+                              : launch_update_bwd_tc_t<32, 256>(packed, lo, L, ws, layer, xbar_out, xtbar, st);
 }
 
 }  // namespace mlff
