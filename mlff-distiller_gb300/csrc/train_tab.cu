@@ -319,12 +319,26 @@ __global__ void __launch_bounds__(H) node_adjoint_kernel(const float* __restrict
     if (st->code != 0) return;
     const int i = blockIdx.x, row = blockIdx.y, c = threadIdx.x;
     const int plane = row / (3 * TAB_NC), g = row / TAB_NC % 3, j = row % TAB_NC;
-    double s[4] = {0.0, 0.0, 0.0, 0.0};
+    // two chains of compensated sums (Knuth's two-sum): the FP64 units are too
+    // few for a sum per chunk
+    float s[2] = {0.f, 0.f}, lo[2] = {0.f, 0.f};
     const float* p = part + (int64_t)row * H + c;
-    const int q0 = cst[i], q1 = cst[i + 1];
-#pragma unroll 4
-    for (int q = q0; q < q1; ++q) s[(q - q0) & 3] += (double)p[(int64_t)q * rows * H];
-    out[(int64_t)plane * NODES * H3 + (int64_t)(i * TAB_NC + j) * H3 + g * H + c] = (float)((s[0] + s[1]) + (s[2] + s[3]));
+    const int64_t stride = (int64_t)rows * H;
+    const int q1 = cst[i + 1];
+    for (int q = cst[i]; q < q1; q += 8) {   // 8 loads in flight
+        float x[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) x[u] = q + u < q1 ? p[(q + u) * stride] : 0.f;
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+            const float t = __fadd_rn(s[u & 1], x[u]), z = __fsub_rn(t, s[u & 1]);
+            lo[u & 1] = __fadd_rn(lo[u & 1],
+                                  __fadd_rn(__fsub_rn(s[u & 1], __fsub_rn(t, z)), __fsub_rn(x[u], z)));
+            s[u & 1] = t;
+        }
+    }
+    out[(int64_t)plane * NODES * H3 + (int64_t)(i * TAB_NC + j) * H3 + g * H + c] =
+        (float)(((double)s[0] + (double)s[1]) + ((double)lo[0] + (double)lo[1]));
 }
 
 // Adjoints of the network's hidden layer at the nodes, in place: of z =
