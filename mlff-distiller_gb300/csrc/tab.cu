@@ -742,13 +742,16 @@ template <bool L0>
 int launch_fwd(const TabShape& s, const TabArgs& a, cudaStream_t st) {
     if (s.G == 4) return launch_fwd_t<4, true, L0>(a, st);
     if (s.G == 2) return launch_fwd_t<2, true, L0>(a, st);
+    if (s.smem) return launch_fwd_t<1, true, L0>(a, st);
     return launch_fwd_t<1, false, L0>(a, st);
 }
 template <bool L0, bool PAIRS>
 int launch_bwd(const TabShape& s, const TabArgs& a, float scale, cudaStream_t st) {
     if (s.G == 4) return launch_bwd_t<4, true, L0, PAIRS>(a, scale, st);
     if (s.G == 2) return launch_bwd_t<2, true, L0, PAIRS>(a, scale, st);
-    return launch_bwd_t<1, false, L0, PAIRS>(a, scale, st);
+    if (s.smem) return launch_bwd_t<1, true, L0, PAIRS>(a, scale, st);
+    if constexpr (!PAIRS) return launch_bwd_t<1, false, L0, PAIRS>(a, scale, st);
+    else return launch_bwd_t<1, true, L0, PAIRS>(a, scale, st);   // (always staged)
 }
 
 }  // namespace
@@ -771,7 +774,7 @@ TabArgs tab_args(const WsLayout& L, void* ws) {
 int launch_records(const mlff_dims& d, const float* P, const PackedOffsets& po, const mlff_system& sys,
                    const WsLayout& L, void* ws, int path, cudaStream_t st) {
     ProfScope prof(PK_NEIGHBORS, st);
-    const TabShape shape = tab_shape(L.N);
+    const TabShape shape = tab_shape(L.N, path);
     const int ngroups = (L.N + shape.G - 1) / shape.G;
     const int grid = std::max(1, std::min((ngroups + REC_WARPS - 1) / REC_WARPS, num_sms() * 16));
     const RecArgs ra{ws_ptr<float4>(ws, L.pos4), ws_ptr<int32_t>(ws, L.atom_mol), sys.box, sys.pbc,
@@ -786,7 +789,7 @@ int launch_records(const mlff_dims& d, const float* P, const PackedOffsets& po, 
 int table_forward(const mlff_dims& d, const float* P, const PackedOffsets& po, const mlff_system& sys,
                   const WsLayout& L, void* ws, int path, cudaStream_t st) {
     const int64_t NX = (int64_t)L.N * 4 * H;
-    const TabShape shape = tab_shape(L.N);
+    const TabShape shape = tab_shape(L.N, path);
     int r;
     if ((r = launch_embed(d, P, po, sys, L, ws, st))) return r;
     if ((r = launch_records(d, P, po, sys, L, ws, path, st))) return r;
@@ -824,7 +827,7 @@ int run_table_reverse(const mlff_dims& d, const float* P, const PackedOffsets& p
                       const WsLayout& L, void* ws, const mlff_outputs& out, int path, cudaStream_t st,
                       const VerletFuse* vf) {
     const int64_t NX = (int64_t)L.N * 4 * H;
-    const TabShape shape = tab_shape(L.N);
+    const TabShape shape = tab_shape(L.N, path);
     const bool tc = path == MLFF_PATH_TABLE;
     const float scale = tab_scale(d.cutoff);
     int r;

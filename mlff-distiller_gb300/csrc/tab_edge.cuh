@@ -239,15 +239,21 @@ struct TabLaunch {
     }
 };
 
-// Receivers per group and where the table is read from.
+// Receivers per group, and whether a CTA stages its table slice in shared
+// memory (221 KB, one bulk copy that overlaps the kernel before when that
+// leaves SMs idle).  After the tensor-core path's update kernels, which take
+// one SM per 32 atoms, it always pays (60 atoms: 390 against 405 us a call,
+// 1400: 661 against 688); the FP32 update kernels take more SMs (path 6: 60
+// atoms 466 against 423, 500: 556 against 543, 1000: 631 against 662; a
+// training step, 550 atoms, 2.96 against 3.17 ms of kernels).
 struct TabShape {
     int G;
     bool smem;
 };
-inline TabShape tab_shape(int n_atoms) {
+inline TabShape tab_shape(int n_atoms, int path) {
     if (n_atoms >= 4096) return {4, true};
     if (n_atoms >= 1500) return {2, true};
-    return {1, false};
+    return {1, path == MLFF_PATH_TABLE || n_atoms >= (path == MLFF_PATH_TRAIN_TABLE ? 400 : 750)};
 }
 
 }  // namespace mlff

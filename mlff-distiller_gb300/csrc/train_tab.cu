@@ -514,7 +514,7 @@ int launch_pass_t(const PassArgs& a, cudaStream_t st) {
 template <int MODE, bool L0>
 int launch_pass(const PassArgs& a, cudaStream_t st) {
     ProfScope prof(PK_PLAIN_EDGE, st);
-    const TabShape s = tab_shape(a.n_atoms);
+    const TabShape s = tab_shape(a.n_atoms, MLFF_PATH_TRAIN_TABLE);
     if (s.G == 4) return launch_pass_t<MODE, 4, true, L0>(a, st);
     if (s.G == 2) return launch_pass_t<MODE, 2, true, L0>(a, st);
     return launch_pass_t<MODE, 1, false, L0>(a, st);
