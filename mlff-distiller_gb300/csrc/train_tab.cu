@@ -18,9 +18,12 @@
 // by interval once per call (a stable counting sort) and summed in chunks of
 // 64 in a fixed order, so repeated calls give the same bits.
 //
-// The force term's value forward pass is the plain path's own (plain_forward):
-// its gradients pass through the second derivative of |v|, ~1/|v|, which turns
-// a last-bit change of v into 1e-5 of a gradient.
+// The value forward pass is the plain path's own (plain_forward).  Gradients
+// of the force term pass through the second derivative of |v|, ~1/|v|, which
+// turns a last-bit change of v into 1e-5 of a gradient; those of the mixing
+// matrices cancel to 1e-6.  Errors against float64 are then the plain path's
+// own instead of others as large (of 40 random steps of 8 molecules, 10 had a
+// tensor 1.5 times further off with a table forward pass, 3 with this one).
 //
 // Measured (64 molecules of 10..60 atoms, 64k edges, energy + force terms):
 // 48.3 -> 12.9 ms a step against the plain Dual path, whose weight gradients
@@ -517,6 +520,7 @@ int launch_pass(const PassArgs& a, cudaStream_t st) {
     const TabShape s = tab_shape(a.n_atoms, MLFF_PATH_TRAIN_TABLE);
     if (s.G == 4) return launch_pass_t<MODE, 4, true, L0>(a, st);
     if (s.G == 2) return launch_pass_t<MODE, 2, true, L0>(a, st);
+    if (s.smem) return launch_pass_t<MODE, 1, true, L0>(a, st);
     return launch_pass_t<MODE, 1, false, L0>(a, st);
 }
 
@@ -896,19 +900,14 @@ int run_train(const mlff_dims& d, const float* P, const PackedOffsets& po, const
     const bool acc = DUAL;
     int r;
 
-    // Value forward pass (records, X, Xt, uz, ua of every layer).  The force
-    // term's second derivative of |v| grows as 1 / |v|, so its gradients carry
-    // the rounding of the smallest |v| (1e-5 to 1e-4, in any FP32 evaluation);
-    // it starts from the plain path's forward pass, bit for bit, and so gives
-    // that path's gradients rather than others as far off.
-    if constexpr (DUAL) {
-        if ((r = launch_records(d, P, po, sys, L, ws, MLFF_PATH_TABLE_FP32, st))) return r;
+    // Value forward pass (records, X, Xt, uz, ua of every layer): the plain
+    // path's, bit for bit (see the head of the file).
+    if ((r = launch_records(d, P, po, sys, L, ws, MLFF_PATH_TABLE_FP32, st))) return r;
+    {
         float* rowsX = ws_ptr<float>(ws, L.prows);   // [L + 1][N][4][H]
         if ((r = plain_forward(d, P, po, sys, L, ws, rowsX, st))) return r;
         TT_LAUNCH(rows_to_gather_kernel, (int64_t)L.L * NH, rowsX, N, L.L, X, status);
         MLFF_CUDA(cudaMemcpyAsync(X + L.L * NX, rowsX + L.L * NX, sizeof(float) * NX, cudaMemcpyDeviceToDevice, st));
-    } else {
-        if ((r = table_forward(d, P, po, sys, L, ws, MLFF_PATH_TABLE_FP32, st))) return r;
     }
     {
         ProfScope prof(PK_OTHER, st);
