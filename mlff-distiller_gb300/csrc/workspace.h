@@ -32,6 +32,7 @@ struct WsLayout {
     size_t rev;                // int32 [cap]  index of the reversed edge
     size_t edge_acc;           // float4 [cap] (dE/dd, dE/du) summed over layers
     size_t scan_tmp;           // int32 [scan_blocks + 1]
+    size_t pbase, pidx, pedge; // int32 [N + 1], [cap], [cap / 2 + 1]  plain path: pairs of atoms
     size_t mol_grid;           // int4 [B + 1]  (ncx, ncy, ncz, first cell code); [B].x = codes in use
     size_t mol_box;            // float4 [2 B]  open structures with a cell grid: origin, 1 / cell width
     size_t cell_count;         // int32 [ncell_cap + 1]
