@@ -56,8 +56,10 @@ typedef struct CUstream_st *mlff_stream_t; /* same type as cudaStream_t */
  * word; mlff_filter_table_class tells beforehand. */
 #define MLFF_PATH_TABLE 5         /* path 1's forward pass, reverse pass from the tables (class 1 or 2) */
 #define MLFF_PATH_TABLE_FP32 6    /* path 2 from the tables, both passes (class 2) */
-
-#define MLFF_PATH_TRAIN_TABLE 7   /* mlff_param_grads_table and its force term (workspace sizing) */
+/* a training step: path 2's forward pass bit for bit, reverse pass from the
+ * tables (class 2); the workspace also serves mlff_param_grads_table and its
+ * force term */
+#define MLFF_PATH_TRAIN_TABLE 7
 
 #define MLFF_MAX_LAYERS 8
 

@@ -104,7 +104,10 @@ __global__ void __launch_bounds__(Tile<BM, BN, TM, TN>::NT, 4)
 #pragma unroll
         for (int i = 0; i < TM; ++i)
 #pragma unroll
-            for (int j = 0; j < TN; ++j) acc[i][j] = 0.f;
+            for (int j = 0; j < TN; ++j) {
+                const int gn = n0 + T::col(tx, j);
+                acc[i][j] = MODE >= 3 && gn < N ? bias[gn] : 0.f;
+            }
         float ra[LA], rb[LB];
         auto fetch = [&](int k0) {
             if (va && LA >= 4) {
@@ -191,13 +194,17 @@ __global__ void __launch_bounds__(Tile<BM, BN, TM, TN>::NT, 4)
                     float v[4];
 #pragma unroll
                     for (int j = 0; j < T::CN; ++j) v[j] = acc[i][j0 + j];
-                    if (MODE != 2 && bias) {
+                    if (MODE < 2 && bias) {
 #pragma unroll
                         for (int j = 0; j < T::CN; ++j) v[j] += bias[gn + j];
                     }
                     if (MODE == 2) {
                         const float4 z = *reinterpret_cast<const float4*>(Z + idx);
                         v[0] *= dsilu_f(z.x); v[1] *= dsilu_f(z.y); v[2] *= dsilu_f(z.z); v[3] *= dsilu_f(z.w);
+                    }
+                    if (MODE == 4) {
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) v[j] = silu_f(v[j]);
                     }
                     *reinterpret_cast<float4*>(C + idx) = make_float4(v[0], v[1], v[2], v[3]);
                     if (MODE == 1)
@@ -208,9 +215,9 @@ __global__ void __launch_bounds__(Tile<BM, BN, TM, TN>::NT, 4)
                     for (int j = 0; j < T::CN; ++j) {
                         if (gn + j >= N) continue;
                         float v = acc[i][j0 + j];
-                        if (MODE != 2 && bias) v += bias[gn + j];
+                        if (MODE < 2 && bias) v += bias[gn + j];
                         if (MODE == 2) v *= dsilu_f(Z[idx + j]);
-                        C[idx + j] = v;
+                        C[idx + j] = MODE == 4 ? silu_f(v) : v;
                         if (MODE == 1) C2[idx + j] = silu_f(v);
                     }
                 }
@@ -273,9 +280,12 @@ __global__ void __launch_bounds__(VecTile<MODE, BM, BN, TM, TN, KS>::NT, PER_SM)
     for (int s = 0; s < STAGES - 1; ++s) load(s);
     f32x2 acc[TM][TN / 2];
 #pragma unroll
-    for (int i = 0; i < TM; ++i)
+    for (int j = 0; j < TN / 2; ++j) {
+        const int gn = n0 + (j / 2) * (BN / (TN / 4)) + tx * 4 + 2 * (j % 2);
+        const f32x2 a0 = MODE >= 3 && gn < N ? pack2(bias[gn], bias[gn + 1]) : pack2(0.f, 0.f);
 #pragma unroll
-        for (int j = 0; j < TN / 2; ++j) acc[i][j] = pack2(0.f, 0.f);
+        for (int i = 0; i < TM; ++i) acc[i][j] = a0;
+    }
     for (int s = 0; s < steps; ++s) {
         asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 2) : "memory");
         __syncthreads();   // the step has landed, and its slot before last is read
@@ -312,7 +322,7 @@ __global__ void __launch_bounds__(VecTile<MODE, BM, BN, TM, TN, KS>::NT, PER_SM)
         const int gn = n0 + j * (BN / (TN / 4)) + tx * 4;
         if (gn >= N) continue;
         float bj[4] = {0.f, 0.f, 0.f, 0.f};
-        if (MODE != 2 && bias) {
+        if (MODE < 2 && bias) {
 #pragma unroll
             for (int q = 0; q < 4; ++q) bj[q] = __ldg(bias + gn + q);
         }
@@ -322,13 +332,17 @@ __global__ void __launch_bounds__(VecTile<MODE, BM, BN, TM, TN, KS>::NT, PER_SM)
             if (gm >= M) break;
             const int64_t idx = gm * N + gn;
             float v[4] = {lo2(acc[i][2 * j]), hi2(acc[i][2 * j]), lo2(acc[i][2 * j + 1]), hi2(acc[i][2 * j + 1])};
-            if (MODE != 2 && bias) {
+            if (MODE < 2 && bias) {
 #pragma unroll
                 for (int q = 0; q < 4; ++q) v[q] += bj[q];
             }
             if (MODE == 2) {
                 const float4 z = __ldg(reinterpret_cast<const float4*>(Z + idx));
                 v[0] *= dsilu_f(z.x); v[1] *= dsilu_f(z.y); v[2] *= dsilu_f(z.z); v[3] *= dsilu_f(z.w);
+            }
+            if (MODE == 4) {
+#pragma unroll
+                for (int q = 0; q < 4; ++q) v[q] = silu_f(v[q]);
             }
             *reinterpret_cast<float4*>(C + idx) = make_float4(v[0], v[1], v[2], v[3]);
             if (MODE == 1)
@@ -601,7 +615,11 @@ int gemm_nn(int mode, const float* A, const float* B, const float* bias, float* 
             int64_t M, const int32_t* m_dev, int N, int K, const Status* st, cudaStream_t s, int lda) {
     ProfScope prof(PK_PLAIN_GEMM, s);
     const NnArgs a{A, B, bias, C, C2, Z, M, m_dev, N, K, lda ? lda : K, st};
-    return mode == 0 ? nn_mode<0>(a, s) : mode == 1 ? nn_mode<1>(a, s) : nn_mode<2>(a, s);
+    return mode == 0   ? nn_mode<0>(a, s)
+           : mode == 1 ? nn_mode<1>(a, s)
+           : mode == 2 ? nn_mode<2>(a, s)
+           : mode == 3 ? nn_mode<3>(a, s)
+                       : nn_mode<4>(a, s);
 }
 
 size_t gemm_tn_floats(int64_t M, int64_t N) { return (size_t)tn_splits(M, N) * (size_t)(M * N + M); }

@@ -11,6 +11,8 @@ namespace mlff {
 //   mode 0: C = acc + bias (bias may be NULL)
 //   mode 1: the same, and C2 = silu(C)
 //   mode 2: C = acc * silu'(Z), Z shaped like C
+//   mode 3: C = acc, the sums starting from the bias
+//   mode 4: C = silu of that
 // M sizes the grid; with m_dev the kernel reads the row count there (M is
 // then an upper bound).
 int gemm_nn(int mode, const float* A, const float* B, const float* bias, float* C, float* C2, const float* Z,

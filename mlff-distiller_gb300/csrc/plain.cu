@@ -801,6 +801,93 @@ int plain_forward(const mlff_dims& d, const float* P, const PackedOffsets& po, c
     return MLFF_OK;
 }
 
+// The fused FP32 path's message step (edge_fwd_simt_kernel) on filters by
+// pair: the same sums in the same order.  Block per receiver, thread =
+// channel; X of layer 0 its s rows, later quads.
+template <bool L0>
+__global__ void __launch_bounds__(128) pair_message_kernel(const float* __restrict__ X, const float* __restrict__ F,
+                                                           const float4* __restrict__ geo,
+                                                           const int32_t* __restrict__ col,
+                                                           const int32_t* __restrict__ row_ptr,
+                                                           const int32_t* __restrict__ pair, int32_t n_atoms,
+                                                           float* __restrict__ Xt, const Status* st) {
+    if (st->code != 0) return;
+    const int c = threadIdx.x;
+    auto row = [&](int a) {
+        return L0 ? make_float4(X[(int64_t)a * H + c], 0.f, 0.f, 0.f)
+                  : reinterpret_cast<const float4*>(X)[(int64_t)a * H + c];
+    };
+    for (int a = blockIdx.x; a < n_atoms; a += gridDim.x) {
+        float s = 0.f, v0 = 0.f, v1 = 0.f, v2 = 0.f;
+        const int k1 = row_ptr[a + 1];
+#pragma unroll 4
+        for (int k = row_ptr[a]; k < k1; ++k) {
+            const float4 x = row(col[k]), g = geo[k];
+            const float* f = F + (int64_t)pair[k] * H3 + c;
+            const float f2 = f[2 * H];
+            s = fmaf(x.x, f[0], s);
+            if (L0) {
+                v0 = fmaf(g.x, f2, v0);
+                v1 = fmaf(g.y, f2, v1);
+                v2 = fmaf(g.z, f2, v2);
+            } else {
+                const float f1 = f[H];
+                v0 = fmaf(x.y, f1, fmaf(g.x, f2, v0));
+                v1 = fmaf(x.z, f1, fmaf(g.y, f2, v1));
+                v2 = fmaf(x.w, f1, fmaf(g.z, f2, v2));
+            }
+        }
+        const float4 x = row(a);
+        float* xt = Xt + (int64_t)a * 4 * H + c;
+        xt[0] = x.x + s;
+        xt[H] = x.y + v0;
+        xt[2 * H] = x.z + v1;
+        xt[3 * H] = x.w + v2;
+    }
+}
+
+// Forward pass with the arithmetic of the fused FP32 path (path 2), bit for
+// bit: filters by pair of atoms as GEMMs whose sums start from the bias.  X in
+// the table path's layout.
+int fused_fp32_forward(const mlff_dims& d, const float* P, const PackedOffsets& po, const mlff_system& sys,
+                       const WsLayout& L, void* ws, cudaStream_t st) {
+    const int N = sys.n_atoms;
+    const int64_t NX = (int64_t)N * 4 * H, pairs = L.cap / 2 + 1;
+    const Status* status = ws_ptr<Status>(ws, L.status);
+    const int32_t *row_ptr = ws_ptr<int32_t>(ws, L.row_ptr), *col = ws_ptr<int32_t>(ws, L.col);
+    float4* geo = ws_ptr<float4>(ws, L.pgeo);
+    float *erbf = ws_ptr<float>(ws, L.erbf), *fh = ws_ptr<float>(ws, L.fh), *ff = ws_ptr<float>(ws, L.ff);
+    const int rblocks = std::max(1, std::min(N, 152 * 16));
+    int r;
+    Pairs pr{};
+    if ((r = make_pairs(L, ws, N, pr, st))) return r;
+    {
+        ProfScope prof(PK_PLAIN_EDGE, st);
+        pl_geom_kernel<float><<<152 * 8, 256, 0, st>>>(ws_ptr<float4>(ws, L.pos4), nullptr, nullptr,
+                                                       ws_ptr<int32_t>(ws, L.atom_mol), sys.box, sys.pbc, row_ptr, col,
+                                                       ws_ptr<int32_t>(ws, L.erecv), N, P + po.centers, P + po.gamma,
+                                                       d.n_rbf, d.cutoff, geo, erbf, nullptr, pr, status);
+        MLFF_LAUNCH_CHECK("pl_geom");
+    }
+    for (int l = 0; l < d.n_layers; ++l) {
+        const LayerOffsets& lo = po.layer[l];
+        const float* X = ws_ptr<float>(ws, L.X) + l * NX;
+        float* Xt = ws_ptr<float>(ws, L.Xt) + l * NX;
+        if ((r = gemm_nn(4, erbf, P + lo.w1t, P + lo.b1, fh, nullptr, nullptr, pairs, pr.base + N, H, RMAX, status,
+                         st))) return r;
+        if ((r = gemm_nn(3, fh, P + lo.w2t, P + lo.b2, ff, nullptr, nullptr, pairs, pr.base + N, H3, H, status, st)))
+            return r;
+        {
+            ProfScope prof(PK_PLAIN_EDGE, st);
+            if (l == 0) pair_message_kernel<true><<<rblocks, 128, 0, st>>>(X, ff, geo, col, row_ptr, pr.idx, N, Xt, status);
+            else pair_message_kernel<false><<<rblocks, 128, 0, st>>>(X, ff, geo, col, row_ptr, pr.idx, N, Xt, status);
+            MLFF_LAUNCH_CHECK("pair_message");
+        }
+        if ((r = launch_update_fwd(d, P, lo, L, ws, l, st))) return r;
+    }
+    return MLFF_OK;
+}
+
 int run_plain(const mlff_dims& d, const float* P, const PackedOffsets& po, const mlff_system& sys,
               const WsLayout& L, void* ws, const mlff_outputs& out, cudaStream_t st, const GradCtx* grad,
               const VerletFuse* vf) {

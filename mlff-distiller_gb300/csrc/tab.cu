@@ -807,10 +807,21 @@ int table_forward(const mlff_dims& d, const float* P, const PackedOffsets& po, c
     return MLFF_OK;
 }
 
-// The FP32 path with tabulated filters (MLFF_PATH_TABLE_FP32).
+// The FP32 path with tabulated filters (MLFF_PATH_TABLE_FP32; MLFF_PATH_TRAIN_TABLE:
+// its reverse pass).
 int run_table(const mlff_dims& d, const float* P, const PackedOffsets& po, const mlff_system& sys, const WsLayout& L,
               void* ws, const mlff_outputs& out, int path, cudaStream_t st, const VerletFuse* vf) {
-    int r = table_forward(d, P, po, sys, L, ws, path, st);
+    int r;
+    if (path == MLFF_PATH_TRAIN_TABLE) {
+        // A training step's energies and forces: the fused FP32 path's forward
+        // pass, bit for bit.  The loss divides by |F| and the gradients by |v|,
+        // so another forward pass, as exact, moves them by up to 5e-5.
+        if ((r = launch_embed(d, P, po, sys, L, ws, st))) return r;
+        if ((r = launch_records(d, P, po, sys, L, ws, path, st))) return r;
+        r = fused_fp32_forward(d, P, po, sys, L, ws, st);
+    } else {
+        r = table_forward(d, P, po, sys, L, ws, path, st);
+    }
     if (r) return r;
     const bool want_grad = out.forces != nullptr || out.virial != nullptr;
     if ((r = launch_readout(d, P, po, sys, L, ws, out, want_grad ? 1 : 0, st))) return r;

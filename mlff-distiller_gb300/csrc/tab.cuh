@@ -61,6 +61,9 @@ int launch_records(const mlff_dims& d, const float* P, const PackedOffsets& po, 
 // forward pass of the plain FP32 path; X [L + 1][N][4][H] component-major
 int plain_forward(const mlff_dims& d, const float* P, const PackedOffsets& po, const mlff_system& sys,
                   const WsLayout& L, void* ws, float* X, cudaStream_t st);
+// the same of the fused FP32 path, X in the tables' layout
+int fused_fp32_forward(const mlff_dims& d, const float* P, const PackedOffsets& po, const mlff_system& sys,
+                       const WsLayout& L, void* ws, cudaStream_t st);
 // forward pass with the tables: records, X, Xt, uz, ua of every layer
 int table_forward(const mlff_dims& d, const float* P, const PackedOffsets& po, const mlff_system& sys,
                   const WsLayout& L, void* ws, int path, cudaStream_t st);

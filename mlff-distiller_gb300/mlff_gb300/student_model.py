@@ -289,7 +289,10 @@ class _EnergyTrain(torch.autograd.Function):
     def forward(ctx, positions, model, batch, mol_index, *params):
         from . import _lib
         eng = model.engine()
-        E, F, _ = eng.energy_forces(batch, eng.route(_lib.PATH_TUNED_FP32), forces=True)
+        path = eng.route(_lib.PATH_TUNED_FP32)
+        if path == _lib.PATH_TABLE_FP32:
+            path = _lib.PATH_TRAIN_TABLE   # path 2's forward pass, reverse pass through the tables
+        E, F, _ = eng.energy_forces(batch, path, forces=True)
         ctx.model, ctx.batch = model, batch
         ctx.save_for_backward(F, mol_index, *params)
         return E.to(positions.dtype)

@@ -34,3 +34,17 @@ def test_pairs_match_directed_edges(weights_bias, name):
     assert torch.equal(E, E0)
     assert float(F0.norm()) == 0.0 or rel(F, F0) < 1e-5
     assert (float(F.norm()) == 0.0) == (float(F0.norm()) == 0.0)
+
+
+@pytest.mark.parametrize("name", ["one", "apart", "pair", "isolated", "molecules1", "molecules7", "water64", "box1503"])
+def test_training_forward_keeps_the_fused_fp32_bits(weights_bias, name):
+    """The forward pass of a training step on pairs against the fused FP32
+    kernels' (equal energies); forces with the tables' 2e-5."""
+    from mlff_gb300 import _lib
+    s = {"one": lambda: cluster(1, 1.0), "apart": lambda: cluster(2, 20.0), "pair": lambda: cluster(2, 1.1)}.get(
+        name, lambda: system(name))()
+    b, eng = batch_of(s), model(weights_bias, "tuned_fp32").engine()
+    E, F, _ = eng.energy_forces(b, _lib.PATH_TRAIN_TABLE, graph=False)
+    E0, F0, _ = eng.energy_forces(b, _lib.PATH_TUNED_FP32, graph=False)
+    assert torch.equal(E, E0)
+    assert float((F - F0).norm()) <= 2e-5 * float(F0.norm())
