@@ -1104,12 +1104,13 @@ size_t train_table_workspace(WsLayout& L, const mlff_dims& d, size_t p) {
     L.tcst = take(4 * (TAB_NI + 1));
     L.thead = take(sizeof(float) * N * (2 * 64 * 3 + 2 * 32 * 2 + 32 + 1));
     L.tadj = take(sizeof(float) * (L.cap / CHUNK + TAB_NI + 1) * 6 * TAB_NC * H);
-    // the plain forward pass of the force term
+    // the forward passes, filters by pair of atoms
+    const int64_t pairs = L.cap / 2 + 1;
     L.prows = take(sizeof(float) * (L.L + 1) * N * 4 * H);
-    L.erbf = take(sizeof(float) * L.cap * RMAX);
-    L.fz = take(sizeof(float) * L.cap * H);
-    L.fh = take(sizeof(float) * L.cap * H);
-    L.ff = take(sizeof(float) * L.cap * H3);
+    L.erbf = take(sizeof(float) * pairs * RMAX);
+    L.fz = take(sizeof(float) * pairs * H);
+    L.fh = take(sizeof(float) * pairs * H);
+    L.ff = take(sizeof(float) * pairs * H3);
     L.pgeo = take(sizeof(float4) * L.cap);
     L.tnode = take(sizeof(float) * 2 * NODES * (H3 + H));
     L.temb = take(sizeof(float) * EMB_SPLIT * (size_t)d.n_species * H);
