@@ -488,16 +488,17 @@ class StudentForceField(nn.Module):
         again when a module, parameter or buffer was added or replaced by
         another object."""
         if check and self._weight_slots is not None and any(
-                len(m._parameters) != np_ or len(m._buffers) != nb or tuple(m._modules.values()) != kids
-                for m, np_, nb, kids in self._weight_slots[3]):
+                len(par) != n_par or len(buf) != n_buf or tuple(sub.values()) != kids
+                for par, n_par, buf, n_buf, sub, kids in self._weight_slots[3]):
             self._weight_slots = None
         if self._weight_slots is None:
             mods = list(self.named_modules())
             named = [[(d(m), n, f"{prefix}.{n}" if prefix else n) for prefix, m in mods for n in d(m)]
                      for d in (lambda m: m._parameters, lambda m: m._buffers)]
             self._weight_slots = (named[0], [(d, n) for d, n, _ in named[0] + named[1]], named[1],
-                                  [(m, len(m._parameters), len(m._buffers), tuple(m._modules.values()))
-                                   for _, m in mods])
+                                  # (the dicts, not the modules: this one would keep itself alive)
+                                  [(m._parameters, len(m._parameters), m._buffers, len(m._buffers), m._modules,
+                                    tuple(m._modules.values())) for _, m in mods])
         return self._weight_slots
 
     def _weights_version(self):
