@@ -25,11 +25,11 @@
 // own instead of others as large (of 40 random steps of 8 molecules, 10 had a
 // tensor 1.5 times further off with a table forward pass, 3 with this one).
 //
-// Measured (64 molecules of 10..60 atoms, 64k edges, energy + force terms):
-// 48.3 -> 12.9 ms a step against the plain Dual path, whose weight gradients
-// (20 ms) and GEMMs (19 ms) run over every edge; 8 molecules 15.2 -> 8.6 ms
-// (launches and host), energy term of 100 molecules 14.0 -> 5.4 ms.  Against
-// float64 the errors are those of the plain path (2e-7 .. 2e-6 per tensor).
+// Measured (64 molecules of 10..120 atoms, 184,000 edges, energy + force
+// terms): 48.3 -> 11.9 ms a step against the plain and Dual passes, whose
+// weight gradients (20 ms) and GEMMs (19 ms) run over every edge; 8 molecules
+// 15.2 -> 7.7 ms (launches and host), energy term of 100 molecules 14.0 -> 5.7
+// ms.
 #include <algorithm>
 #include <mutex>
 #include "common.cuh"
