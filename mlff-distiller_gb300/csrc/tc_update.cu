@@ -82,53 +82,54 @@ __device__ __forceinline__ void uload(uint32_t taddr, float (&v)[NC]) {
     else tmem_ld8(taddr, v);
 }
 
-template <int URING>
+// The ring's slots hold U consecutive K-steps' pairs each (a unit).
+template <int URING, int U>
 struct UStream {
     unsigned char* ring;
     uint64_t* full;
     uint64_t* empty;
     const unsigned char* src[2];   // pair sources of the two GEMMs of a tile
-    int npairs[2];                 // (the second: chunks of 8 pairs)
-    uint32_t issued;               // producer: pairs copied so far (global count)
+    int nunits[2];                 // (the second: chunks of 8 pairs)
+    uint32_t issued;               // producer: units copied so far (global count)
 };
 
-template <int URING>
-__device__ __forceinline__ const unsigned char* ustream_src(const UStream<URING>& s, uint32_t P) {
-    const uint32_t per = s.npairs[0] + s.npairs[1];
+template <int URING, int U>
+__device__ __forceinline__ const unsigned char* ustream_src(const UStream<URING, U>& s, uint32_t P) {
+    const uint32_t per = s.nunits[0] + s.nunits[1];
     const uint32_t q = P % per;
-    if (q < (uint32_t)s.npairs[0]) return s.src[0] + (size_t)q * A_PAIR;
-    // K-step by K-step: the chunks of the second GEMM run in parallel
-    const uint32_t chunks = s.npairs[1] / 8, r = q - s.npairs[0];
-    return s.src[1] + (size_t)(r % chunks * 8 + r / chunks) * A_PAIR;
+    if (q < (uint32_t)s.nunits[0]) return s.src[0] + (size_t)q * U * A_PAIR;
+    // unit by unit across the chunks: the chunks of the second GEMM run in parallel
+    const uint32_t chunks = s.nunits[1] * U / 8, r = q - s.nunits[0];
+    return s.src[1] + (size_t)(r % chunks * 8 + r / chunks * U) * A_PAIR;
 }
 
-// producer: copy pairs until `target` (exclusive) are issued; a slot is
-// reused once the commit of the pair that used it URING pairs earlier has
+// producer: copy units until `target` (exclusive) are issued; a slot is
+// reused once the commit of the unit that used it URING units earlier has
 // arrived
-template <int URING>
-__device__ __forceinline__ bool ustream_fill(UStream<URING>& s, uint32_t target) {
+template <int URING, int U>
+__device__ __forceinline__ bool ustream_fill(UStream<URING, U>& s, uint32_t target) {
     while (s.issued < target) {
         const uint32_t slot = s.issued % URING;
         if (s.issued >= (uint32_t)URING && !mbar_wait(&s.empty[slot], ((s.issued / URING) - 1) & 1, WAIT_BUDGET))
             return false;
-        mbar_expect_tx(&s.full[slot], A_PAIR);
-        bulk_g2s(s.ring + slot * A_PAIR, ustream_src(s, s.issued), A_PAIR, &s.full[slot]);
+        mbar_expect_tx(&s.full[slot], U * A_PAIR);
+        bulk_g2s(s.ring + slot * U * A_PAIR, ustream_src(s, s.issued), U * A_PAIR, &s.full[slot]);
         ++s.issued;
     }
     return true;
 }
 
-// consumer: one accumulator tile of a GEMM.  Pair i of n (global pair
-// P0 + STRIDE i): D += A_hi B_hi(i) + A_hi B_lo(i) + A_lo B_hi(i); with fresh
-// the first MMA overwrites D.  The thread spends about 470 cycles on a pair
-// (three dependent MMAs of 72, the two barriers), so a GEMM of several chunks
-// has one issuing thread per chunk (STRIDE = their number).  A wait names its
-// pair by the parity of the slot's use, so the slot's previous pair must be
-// known to have landed: it is the thread's own (the ring's length is a
-// multiple of STRIDE) or of a GEMM the whole CTA has waited for.  Copies
-// land in any order.
-template <int UN, int STRIDE, int URING, typename BOf>
-__device__ __forceinline__ bool ustream_gemm(UStream<URING>& s, uint32_t P0, int n, uint32_t d, BOf b_of,
+// consumer: one accumulator tile of a GEMM.  Unit i of n (global unit
+// P0 + STRIDE i), each of its pairs k: D += A_hi B_hi(k) + A_hi B_lo(k) + A_lo
+// B_hi(k); with fresh the first MMA overwrites D.  The thread spends 216
+// cycles on a pair (three dependent MMAs of 72) and 140 on a unit's two
+// barriers, so a GEMM of several chunks has one issuing thread per chunk
+// (STRIDE = their number).  A wait names its unit by the parity of the slot's
+// use, so the slot's previous unit must be known to have landed: it is the
+// thread's own (the ring's length is a multiple of STRIDE) or of a GEMM the
+// whole CTA has waited for.  Copies land in any order.
+template <int UN, int STRIDE, int URING, int U, typename BOf>
+__device__ __forceinline__ bool ustream_gemm(UStream<URING, U>& s, uint32_t P0, int n, uint32_t d, BOf b_of,
                                              uint64_t bhalf, bool fresh) {
     static_assert(URING % STRIDE == 0, "a slot is always waited for by the same thread within a GEMM");
     constexpr uint32_t idesc = idesc_f16(UN);
@@ -138,11 +139,14 @@ __device__ __forceinline__ bool ustream_gemm(UStream<URING>& s, uint32_t P0, int
         const uint32_t P = P0 + STRIDE * i;
         const uint32_t slot = P % URING;
         if (!mbar_wait(&s.full[slot], (P / URING) & 1, WAIT_BUDGET)) return false;
-        const uint64_t ahi = a0 + (uint64_t)(slot * A_PAIR >> 4), alo = ahi + (A_TILE >> 4);
-        const uint64_t bhi = b_of(i);
-        mma_f16(d, ahi, bhi, idesc, fresh && i == 0 ? 0u : 1u);
-        mma_f16(d, ahi, bhi + bhalf, idesc, 1);
-        mma_f16(d, alo, bhi, idesc, 1);
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const uint64_t ahi = a0 + (uint64_t)((slot * U + u) * A_PAIR >> 4), alo = ahi + (A_TILE >> 4);
+            const uint64_t bhi = b_of(i * U + u);
+            mma_f16(d, ahi, bhi, idesc, fresh && i == 0 && u == 0 ? 0u : 1u);
+            mma_f16(d, ahi, bhi + bhalf, idesc, 1);
+            mma_f16(d, alo, bhi, idesc, 1);
+        }
         mma_commit(&s.empty[slot]);
     }
     return true;
@@ -236,22 +240,25 @@ __device__ __forceinline__ void uwait_mma(UCtl& c, int w, int where) {
 // TMEM: D1 = z (cols 0..UN-1), D2 chunk g = (ds, g1, g2)[g] (UN + UN g).
 // UN-atom tiles, UN = 64 or 32 (the autotuner's update tile: small systems
 // spread over more SMs with 32); the ring takes what two CTAs per SM leave.
-template <int UN>
+// 512 threads: one CTA per SM, so the ring holds 12 pairs in units of two
+// (more would take the L1 that the epilogues' row reads hit: 20 pairs cost
+// more than they gave).
+template <int UN, int NT>
 struct UFwd {
     static constexpr uint32_t BH = 4 * b_block(UN);
     static constexpr uint32_t HH = 2 * b_block(UN);
     // epilogue 2 stages (ds, g1, g2) of 32 atoms, [3][32][H] floats, in the B region
     static constexpr uint32_t T_BYTES = 3 * 32 * H * 4;
     static constexpr uint32_t B_REGION = 2 * BH > T_BYTES ? 2 * BH : T_BYTES;
-    static constexpr int RING = 6;
+    static constexpr int U = NT == 512 ? 2 : 1, RING = 6;
     static constexpr uint32_t OFF_B = 0;
     static constexpr uint32_t OFF_RING = OFF_B + B_REGION;
-    static constexpr uint32_t OFF_MIX = OFF_RING + RING * A_PAIR;
+    static constexpr uint32_t OFF_MIX = OFF_RING + RING * U * A_PAIR;
     static constexpr uint32_t OFF_BAR = OFF_MIX + 64;
     static constexpr uint32_t OFF_MISC = OFF_BAR + 8 * (2 + 2 * RING);
     static constexpr uint32_t SMEM = align1k(OFF_MISC + 16);
     static constexpr uint32_t TMEM_COLS = 4 * UN;
-    static_assert(2 * (SMEM + 1024) <= 228 * 1024, "two update CTAs per SM");
+    static_assert((NT == 512 ? 1 : 2) * (SMEM + 1024) <= 228 * 1024, "one or two update CTAs per SM");
 };
 
 template <int UN, int NT>
@@ -260,7 +267,8 @@ __global__ void __launch_bounds__(NT, NT == 512 ? 1 : 2) update_fwd_tc_kernel(co
                                                                float* __restrict__ Xout, int out_layout,
                                                                float* __restrict__ uz, float* __restrict__ ua,
                                                                Status* st) {
-    using LF = UFwd<UN>;
+    using LF = UFwd<UN, NT>;
+    constexpr int U = LF::U;
     using UT = UThreads<UN, NT>;
     constexpr int NC = UT::NC, WARPS = UT::WARPS;
     extern __shared__ __align__(1024) unsigned char smem[];
@@ -293,12 +301,12 @@ __global__ void __launch_bounds__(NT, NT == 512 ? 1 : 2) update_fwd_tc_kernel(co
     __syncthreads();
     fence_after_sync();
     const uint32_t tmem = *tslot;
-    UStream<LF::RING> ws{smem + LF::OFF_RING, full, empty,
+    UStream<LF::RING, U> ws{smem + LF::OFF_RING, full, empty,
                {reinterpret_cast<const unsigned char*>(P + lo.u1_tc), reinterpret_cast<const unsigned char*>(P + lo.u2_tc)},
-               {16, 24}, 0};
+               {16 / U, 24 / U}, 0};
     UCtl ctl{mma_bar, abort_flag, st, 0}, ctl2{chunk_bar, abort_flag, st, 0};
     const int my_tiles = blockIdx.x < ntiles ? (ntiles - 1 - blockIdx.x) / gridDim.x + 1 : 0;
-    const uint32_t P_end = (uint32_t)my_tiles * 40;
+    const uint32_t P_end = (uint32_t)my_tiles * (40 / U);
     const bool producer = t == 32;
     if (producer && !ustream_fill(ws, min((uint32_t)LF::RING, P_end))) ufail(ctl, 20);
     // everything above reads packed weights only and overlaps the previous kernel
@@ -311,7 +319,7 @@ __global__ void __launch_bounds__(NT, NT == 512 ? 1 : 2) update_fwd_tc_kernel(co
     const float c1c = P[lo.c1 + c], c2c[3] = {P[lo.c2 + c], P[lo.c2 + H + c], P[lo.c2 + 2 * H + c]};
     uint32_t P0 = 0;
 
-    for (int tile = blockIdx.x; tile < ntiles && !*abort_flag; tile += gridDim.x, P0 += 40) {
+    for (int tile = blockIdx.x; tile < ntiles && !*abort_flag; tile += gridDim.x, P0 += 40 / U) {
         const int a0 = tile * UN;
         // accumulators <- bias: D1 c1, D2 chunk g c2[g]
         ufill_tmem<NC>(lane_base + NC * hh, c1c);
@@ -345,15 +353,15 @@ __global__ void __launch_bounds__(NT, NT == 512 ? 1 : 2) update_fwd_tc_kernel(co
         if (t == 0) {   // GEMM1: z^T = U1 [s, |v|]^T, K = 256
             fence_after_sync();
             const uint64_t b0 = sdesc_b(smem_u32(Bs));
-            if (!ustream_gemm<UN, 1>(ws, P0, 16, tmem, [&](int i) { return b0 + (uint64_t)(b_kstep_off(UN, i) >> 4); },
+            if (!ustream_gemm<UN, 1>(ws, P0, 16 / U, tmem, [&](int i) { return b0 + (uint64_t)(b_kstep_off(UN, i) >> 4); },
                                   (uint64_t)(LF::BH >> 4), false))
                 ufail(ctl, 21);
             mma_commit(mma_bar);
         }
-        if (producer && !ustream_fill(ws, min(P0 + 16, P_end))) ufail(ctl, 26);
+        if (producer && !ustream_fill(ws, min(P0 + 16 / U, P_end))) ufail(ctl, 26);
         uwait_mma(ctl, w, 22);
         // GEMM1 is done, so every slot is free: fetch GEMM2's pairs during epilogue 1
-        if (producer && !ustream_fill(ws, min(P0 + 16 + LF::RING, P_end))) ufail(ctl, 27);
+        if (producer && !ustream_fill(ws, min(P0 + 16 / U + LF::RING, P_end))) ufail(ctl, 27);
         {   // epilogue 1: z -> uz, h = silu(z) -> H tile (aliases the B tile)
             const int col = NC * hh;   // this group's atoms
             float z[NC];
@@ -376,17 +384,17 @@ __global__ void __launch_bounds__(NT, NT == 512 ? 1 : 2) update_fwd_tc_kernel(co
         if (const int g = uissuer(w, lane); g >= 0) {   // GEMM2: a^T = U2 h^T, 3 chunks x 8 K-steps
             fence_after_sync();
             const uint64_t b0 = sdesc_b(smem_u32(Bs));
-            if (!ustream_gemm<UN, 3>(ws, P0 + 16 + g, 8, tmem + UN + UN * g,
+            if (!ustream_gemm<UN, 3>(ws, P0 + 16 / U + g, 8 / U, tmem + UN + UN * g,
                                   [&](int i) { return b0 + (uint64_t)(b_kstep_off(UN, i) >> 4); },
                                   (uint64_t)(LF::HH >> 4), false))
                 ufail(ctl2, 23);
             mma_commit(chunk_bar);
         }
         __syncwarp();
-        if (producer && !ustream_fill(ws, min(P0 + 40, P_end))) ufail(ctl, 28);
+        if (producer && !ustream_fill(ws, min(P0 + 40 / U, P_end))) ufail(ctl, 28);
         uwait_mma(ctl2, w, 24);
         // the next tile's GEMM1 pairs arrive while this epilogue and the next build run
-        if (producer && !ustream_fill(ws, min(P0 + 40 + LF::RING, P_end))) ufail(ctl, 29);
+        if (producer && !ustream_fill(ws, min(P0 + 40 / U + LF::RING, P_end))) ufail(ctl, 29);
         {   // epilogue 2: (ds, g1, g2) -> ua; s' = s + ds, v' = v g1 + (M v) g2 (:452-468).
             // The TMEM owner of channel c writes (ds, g1, g2) of 32 atoms to
             // shared memory (the B tile is free), then each warp handles
@@ -475,7 +483,7 @@ __global__ void __launch_bounds__(NT, NT == 512 ? 1 : 2) update_fwd_tc_kernel(co
 // UN-atom tiles, two CTAs per SM: one CTA's epilogues overlap the other's
 // weight stream and MMAs.  Up to one tile per SM there is no other CTA, and
 // 512 threads halve the build and the epilogues, 19,000 of a 32-atom tile's
-// 31,000 cycles with 256 (a water box of 3000 atoms 928 -> 887 us a call).
+// 31,000 cycles with 256 (a water box of 3000 atoms 928 -> 887 us a call; 878 with the ring in units of two pairs).
 static bool one_tile_per_sm(const WsLayout& L) { return (L.N + L.UT - 1) / L.UT <= num_sms(); }
 template <int UN, int NT>
 static int launch_update_fwd_tc_t(const float* packed, const LayerOffsets& lo, const WsLayout& L, void* ws, int layer,
@@ -484,7 +492,7 @@ static int launch_update_fwd_tc_t(const float* packed, const LayerOffsets& lo, c
     static cudaError_t attr_err = cudaSuccess;
     std::call_once(once, [] {
         attr_err = cudaFuncSetAttribute(update_fwd_tc_kernel<UN, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        UFwd<UN>::SMEM);
+                                        (UFwd<UN, NT>::SMEM));
     });
     if (attr_err != cudaSuccess) return cuda_status(attr_err, "update_fwd_tc smem attribute");
     ProfScope prof(PK_UPDATE_FWD, st);
@@ -498,7 +506,7 @@ static int launch_update_fwd_tc_t(const float* packed, const LayerOffsets& lo, c
     // the next layer's input in the layout of the edge kernels' gathers; the
     // last layer's output (read by the readout) component-major
     const int out_layout = layer + 1 < L.L ? L.gather : GATHER_ROWS;
-    MLFF_LAUNCH_PDL("update_fwd_tc", (update_fwd_tc_kernel<UN, NT>), grid, NT, UFwd<UN>::SMEM, st, packed, lo, Xt, L.N,
+    MLFF_LAUNCH_PDL("update_fwd_tc", (update_fwd_tc_kernel<UN, NT>), grid, NT, (UFwd<UN, NT>::SMEM), st, packed, lo, Xt, L.N,
                     Xout, out_layout, uz, ua, ws_ptr<Status>(ws, L.status));
     return MLFF_OK;
 }
@@ -516,19 +524,19 @@ int launch_update_fwd_tc(const float* packed, const LayerOffsets& lo, const WsLa
 // smem: abar B tile (K = 384: 6 K-blocks, hi then lo, 96 KB), the zbar tile
 // (K = 128, 32 KB) aliased into it after GEMM3, the ring (16 KB).
 // TMEM: D3 = zbar pre-activation (cols 0..UN-1), D4 = (cs, cn) (UN + UN g).
-template <int UN>
+template <int UN, int NT>
 struct UBwd {
     static constexpr uint32_t AH = 6 * b_block(UN);
     static constexpr uint32_t ZH = 2 * b_block(UN);
-    static constexpr int RING = UN == 64 ? 2 : 8;
+    static constexpr int U = NT == 512 ? 2 : 1, RING = NT == 512 ? 6 : UN == 64 ? 2 : 8;
     static constexpr uint32_t OFF_B = 0;
     static constexpr uint32_t OFF_RING = OFF_B + 2 * AH;
-    static constexpr uint32_t OFF_MIX = OFF_RING + RING * A_PAIR;
+    static constexpr uint32_t OFF_MIX = OFF_RING + RING * U * A_PAIR;
     static constexpr uint32_t OFF_BAR = OFF_MIX + 64;
     static constexpr uint32_t OFF_MISC = OFF_BAR + 8 * (2 + 2 * RING);
     static constexpr uint32_t SMEM = align1k(OFF_MISC + 16);
     static constexpr uint32_t TMEM_COLS = UN == 64 ? 256 : 128;   // 3 UN columns, a power of two
-    static_assert(2 * (SMEM + 1024) <= 228 * 1024, "two update reverse CTAs per SM");
+    static_assert((NT == 512 ? 1 : 2) * (SMEM + 1024) <= 228 * 1024, "one or two update reverse CTAs per SM");
     static_assert(2 * UN * H * 4 <= 2 * AH, "epilogue 4 stages (cs, cn) of the tile in the abar region");
 };
 
@@ -538,7 +546,8 @@ __global__ void __launch_bounds__(NT, NT == 512 ? 1 : 2) update_bwd_tc_kernel(co
                                                                const float* __restrict__ ua,
                                                                const float* __restrict__ xbo, int32_t n_atoms,
                                                                float* __restrict__ xtbar, int out_layout, Status* st) {
-    using LB = UBwd<UN>;
+    using LB = UBwd<UN, NT>;
+    constexpr int U = LB::U;
     using UT = UThreads<UN, NT>;
     constexpr int NC = UT::NC, WARPS = UT::WARPS;
     extern __shared__ __align__(1024) unsigned char smem[];
@@ -571,12 +580,12 @@ __global__ void __launch_bounds__(NT, NT == 512 ? 1 : 2) update_bwd_tc_kernel(co
     __syncthreads();
     fence_after_sync();
     const uint32_t tmem = *tslot;
-    UStream<LB::RING> ws{smem + LB::OFF_RING, full, empty,
+    UStream<LB::RING, U> ws{smem + LB::OFF_RING, full, empty,
                {reinterpret_cast<const unsigned char*>(P + lo.u2t_tc), reinterpret_cast<const unsigned char*>(P + lo.u1t_tc)},
-               {24, 16}, 0};
+               {24 / U, 16 / U}, 0};
     UCtl ctl{mma_bar, abort_flag, st, 0}, ctl2{chunk_bar, abort_flag, st, 0};
     const int my_tiles = blockIdx.x < ntiles ? (ntiles - 1 - blockIdx.x) / gridDim.x + 1 : 0;
-    const uint32_t P_end = (uint32_t)my_tiles * 40;
+    const uint32_t P_end = (uint32_t)my_tiles * (40 / U);
     const bool producer = t == 32;
     if (producer && !ustream_fill(ws, min((uint32_t)LB::RING, P_end))) ufail(ctl, 30);
     // everything above reads packed weights only and overlaps the previous kernel
@@ -588,7 +597,7 @@ __global__ void __launch_bounds__(NT, NT == 512 ? 1 : 2) update_bwd_tc_kernel(co
     const uint32_t lane_base = tmem + ((uint32_t)(32 * q) << 16);
     uint32_t P0 = 0;
 
-    for (int tile = blockIdx.x; tile < ntiles && !*abort_flag; tile += gridDim.x, P0 += 40) {
+    for (int tile = blockIdx.x; tile < ntiles && !*abort_flag; tile += gridDim.x, P0 += 40 / U) {
         const int a0 = tile * UN;
         // abar tile: row = atom; K = [sb, sum_i xb_i v_i, sum_i xb_i (M v)_i]; warp w builds
         // rows w, w + 8, ..., two rows per step so that their loads overlap
@@ -631,14 +640,14 @@ __global__ void __launch_bounds__(NT, NT == 512 ? 1 : 2) update_bwd_tc_kernel(co
         if (t == 0) {   // GEMM3: zbar_pre^T = U2^T abar^T, K = 384
             fence_after_sync();
             const uint64_t b0 = sdesc_b(smem_u32(Bs));
-            if (!ustream_gemm<UN, 1>(ws, P0, 24, tmem, [&](int i) { return b0 + (uint64_t)(b_kstep_off(UN, i) >> 4); },
+            if (!ustream_gemm<UN, 1>(ws, P0, 24 / U, tmem, [&](int i) { return b0 + (uint64_t)(b_kstep_off(UN, i) >> 4); },
                                   (uint64_t)(LB::AH >> 4), true))
                 ufail(ctl, 31);
             mma_commit(mma_bar);
         }
-        if (producer && !ustream_fill(ws, min(P0 + 24, P_end))) ufail(ctl, 36);
+        if (producer && !ustream_fill(ws, min(P0 + 24 / U, P_end))) ufail(ctl, 36);
         uwait_mma(ctl, w, 32);
-        if (producer && !ustream_fill(ws, min(P0 + 24 + LB::RING, P_end))) ufail(ctl, 37);
+        if (producer && !ustream_fill(ws, min(P0 + 24 / U + LB::RING, P_end))) ufail(ctl, 37);
         {   // epilogue 3: zbar = D3 silu'(uz) -> zbar tile (aliases the abar tile)
             const int col = NC * hh;   // this group's atoms
             float zb[NC];
@@ -660,16 +669,16 @@ __global__ void __launch_bounds__(NT, NT == 512 ? 1 : 2) update_bwd_tc_kernel(co
         if (const int g = uissuer(w, lane); g >= 0 && g < 2) {   // GEMM4: cb^T = U1^T zbar^T, 2 chunks x 8 K-steps
             fence_after_sync();
             const uint64_t b0 = sdesc_b(smem_u32(Bs));
-            if (!ustream_gemm<UN, 2>(ws, P0 + 24 + g, 8, tmem + UN + UN * g,
+            if (!ustream_gemm<UN, 2>(ws, P0 + 24 / U + g, 8 / U, tmem + UN + UN * g,
                                   [&](int i) { return b0 + (uint64_t)(b_kstep_off(UN, i) >> 4); },
                                   (uint64_t)(LB::ZH >> 4), true))
                 ufail(ctl2, 33);
             mma_commit(chunk_bar);
         }
         __syncwarp();
-        if (producer && !ustream_fill(ws, min(P0 + 40, P_end))) ufail(ctl, 38);
+        if (producer && !ustream_fill(ws, min(P0 + 40 / U, P_end))) ufail(ctl, 38);
         uwait_mma(ctl2, w, 34);
-        if (producer && !ustream_fill(ws, min(P0 + 40 + LB::RING, P_end))) ufail(ctl, 39);
+        if (producer && !ustream_fill(ws, min(P0 + 40 / U + LB::RING, P_end))) ufail(ctl, 39);
         {   // epilogue 4: xtbar = (sb + cs, xb g1 + M^T xb g2 + cn v / |v|).  The
             // TMEM owner of channel c writes (cs, cn) of its 32 atoms to shared
             // memory (the abar tile is free), then each warp handles whole atom
@@ -755,7 +764,7 @@ static int launch_update_bwd_tc_t(const float* packed, const LayerOffsets& lo, c
     static cudaError_t attr_err = cudaSuccess;
     std::call_once(once, [] {
         attr_err = cudaFuncSetAttribute(update_bwd_tc_kernel<UN, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        UBwd<UN>::SMEM);
+                                        (UBwd<UN, NT>::SMEM));
     });
     if (attr_err != cudaSuccess) return cuda_status(attr_err, "update_bwd_tc smem attribute");
     ProfScope prof(PK_UPDATE_BWD, st);
@@ -765,7 +774,7 @@ static int launch_update_bwd_tc_t(const float* packed, const LayerOffsets& lo, c
     const float* ua = ws_ptr<float>(ws, L.ua) + (int64_t)layer * L.N * H3;
     const int ntiles = (L.N + UN - 1) / UN;
     const int grid = std::max(1, std::min(ntiles, 2 * num_sms()));
-    MLFF_LAUNCH_PDL("update_bwd_tc", (update_bwd_tc_kernel<UN, NT>), grid, NT, UBwd<UN>::SMEM, st, packed, lo, Xt, uz, ua,
+    MLFF_LAUNCH_PDL("update_bwd_tc", (update_bwd_tc_kernel<UN, NT>), grid, NT, (UBwd<UN, NT>::SMEM), st, packed, lo, Xt, uz, ua,
                     xbar_out, L.N, xtbar, L.gather_bar, ws_ptr<Status>(ws, L.status));
     return MLFF_OK;
 }
