@@ -209,10 +209,9 @@ int launch_embed(const mlff_dims& d, const float* packed, const PackedOffsets& p
 // ---------------------------------------------------------------- readout
 // Per atom: E_a = w3 . silu(W2 silu(W1 s + b1) + b2) + b3 and, when
 // requested, dE_a/ds written as the adjoint seed (v adjoint = 0).
-// One CTA of 256 threads per SM walks groups of RO_ATOMS atoms; the head's
+// CTAs of 256 threads walk groups of A atoms; the head's
 // four weight matrices (80 KB) are staged in shared memory once per CTA with
 // independent 128-bit loads, so the dot products read shared memory only.
-constexpr int RO_ATOMS = 32;
 constexpr int RO_NT = 256;
 // the head's weights transposed, rows padded by one float so that both the
 // forward (threads along a row) and the backward products (threads along a
@@ -220,98 +219,109 @@ constexpr int RO_NT = 256;
 constexpr int RO_W1T_LD = 64 + 1, RO_W2T_LD = 32 + 1;
 constexpr int RO_W1T = 0;                       // [H][65]: W1T[i][o] = W1[o][i]
 constexpr int RO_W2T = RO_W1T + H * RO_W1T_LD;  // [64][33]
-constexpr int RO_S = ((RO_W2T + 64 * RO_W2T_LD) + 3) & ~3;   // [RO_ATOMS][H]     s (16-byte aligned)
-constexpr int RO_Z1 = RO_S + RO_ATOMS * H;      // [RO_ATOMS][64]    z1
-constexpr int RO_H1 = RO_Z1 + RO_ATOMS * 64;    // [RO_ATOMS][64]    silu(z1)
-constexpr int RO_G1 = RO_H1 + RO_ATOMS * 64;    // [RO_ATOMS][64]    dE/dz1
-constexpr int RO_Z2 = RO_G1 + RO_ATOMS * 64;    // [RO_ATOMS][32]    z2
-constexpr int RO_G2 = RO_Z2 + RO_ATOMS * 32;    // [RO_ATOMS][32]    dE/dz2
-constexpr int RO_FLOATS = RO_G2 + RO_ATOMS * 32;
-constexpr size_t RO_SMEM = sizeof(float) * RO_FLOATS;
+constexpr int RO_S = ((RO_W2T + 64 * RO_W2T_LD) + 3) & ~3;   // (16-byte aligned)
+// A atoms per block iteration: 32, or 8 where that still fits two rounds of
+// blocks (a group of 32 takes 12 us of shared-memory reads, the same per atom
+// whatever the group: 60 atoms 15 -> 7 us, 3,000 atoms 12 -> 10)
+template <int A>
+struct RoLayout {
+    static constexpr int S = RO_S;                // [A][H]     s
+    static constexpr int Z1 = S + A * H;          // [A][64]    z1
+    static constexpr int H1 = Z1 + A * 64;        // [A][64]    silu(z1)
+    static constexpr int G1 = H1 + A * 64;        // [A][64]    dE/dz1
+    static constexpr int Z2 = G1 + A * 64;        // [A][32]    z2
+    static constexpr int G2 = Z2 + A * 32;        // [A][32]    dE/dz2
+    static constexpr size_t SMEM = sizeof(float) * (G2 + A * 32);
+};
 
 // rows x cols floats into rows of ld floats
 __device__ __forceinline__ void ro_stage(float* dst, const float* __restrict__ src, int rows, int cols, int ld) {
     for (int i = threadIdx.x; i < rows * cols; i += RO_NT) dst[(i / cols) * ld + i % cols] = __ldg(src + i);
 }
 
+template <int A>
 __global__ void __launch_bounds__(RO_NT, 2) readout_kernel(const float* __restrict__ P, PackedOffsets po,
                                                         const float* __restrict__ X, int32_t n_atoms,
                                                         float* __restrict__ e_atom, float* __restrict__ xbar,
                                                         int want_grad, const Status* st) {
     extern __shared__ __align__(16) float ro[];
+    using R = RoLayout<A>;
     const int t = threadIdx.x;
     ro_stage(ro + RO_W1T, P + po.head_w1t, H, 64, RO_W1T_LD);
     ro_stage(ro + RO_W2T, P + po.head_w2t, 64, 32, RO_W2T_LD);
     pdl_wait();   // the weights above overlap the previous kernel
     pdl_trigger();
     if (st->code != 0) return;
-    float* S = ro + RO_S;
-    float* Z1 = ro + RO_Z1;
-    float* H1 = ro + RO_H1;
-    float* G1 = ro + RO_G1;
-    float* Z2 = ro + RO_Z2;
-    float* G2 = ro + RO_G2;
-    for (int a0 = blockIdx.x * RO_ATOMS; a0 < n_atoms; a0 += gridDim.x * RO_ATOMS) {
+    float* S = ro + R::S;
+    float* Z1 = ro + R::Z1;
+    float* H1 = ro + R::H1;
+    float* G1 = ro + R::G1;
+    float* Z2 = ro + R::Z2;
+    float* G2 = ro + R::G2;
+    for (int a0 = blockIdx.x * A; a0 < n_atoms; a0 += gridDim.x * A) {
         // s rows of the group (128-bit, one warp per atom row)
-        for (int i = t; i < RO_ATOMS * (H / 4); i += RO_NT) {
+        for (int i = t; i < A * (H / 4); i += RO_NT) {
             const int q = i / (H / 4), k = i % (H / 4), a = a0 + q;
             reinterpret_cast<float4*>(S + q * H)[k] =
                 a < n_atoms ? __ldg(reinterpret_cast<const float4*>(X + (int64_t)a * 4 * H) + k)
                             : make_float4(0.f, 0.f, 0.f, 0.f);
         }
         __syncthreads();
-        {   // z1 = W1 s + b1: thread -> output o, atoms 8 (t / 64) .. + 8
-            const int o = t & 63, q0 = (t >> 6) * 8;
-            float acc[8];
+        {   // z1 = W1 s + b1: thread -> output o, A / 4 atoms
+            constexpr int Q = A / 4;
+            const int o = t & 63, q0 = (t >> 6) * Q;
+            float acc[Q];
             const float b = P[po.head_b1 + o];
 #pragma unroll
-            for (int q = 0; q < 8; ++q) acc[q] = b;
+            for (int q = 0; q < Q; ++q) acc[q] = b;
 #pragma unroll 4
             for (int i = 0; i < H; i += 4) {
                 const float w0 = ro[RO_W1T + (i + 0) * RO_W1T_LD + o], w1 = ro[RO_W1T + (i + 1) * RO_W1T_LD + o];
                 const float w2 = ro[RO_W1T + (i + 2) * RO_W1T_LD + o], w3 = ro[RO_W1T + (i + 3) * RO_W1T_LD + o];
 #pragma unroll
-                for (int q = 0; q < 8; ++q) {
+                for (int q = 0; q < Q; ++q) {
                     const float4 x = *reinterpret_cast<const float4*>(S + (q0 + q) * H + i);
                     acc[q] = fmaf(w3, x.w, fmaf(w2, x.z, fmaf(w1, x.y, fmaf(w0, x.x, acc[q]))));
                 }
             }
 #pragma unroll
-            for (int q = 0; q < 8; ++q) {
+            for (int q = 0; q < Q; ++q) {
                 Z1[(q0 + q) * 64 + o] = acc[q];
                 H1[(q0 + q) * 64 + o] = silu_f(acc[q]);
             }
         }
         __syncthreads();
-        {   // z2 = W2 h1 + b2: thread -> output o, atoms 4 (t / 32) .. + 4
-            const int o = t & 31, q0 = (t >> 5) * 4;
-            float acc[4];
+        {   // z2 = W2 h1 + b2: thread -> output o, A / 8 atoms
+            constexpr int Q = A / 8;
+            const int o = t & 31, q0 = (t >> 5) * Q;
+            float acc[Q];
             const float b = P[po.head_b2 + o];
 #pragma unroll
-            for (int q = 0; q < 4; ++q) acc[q] = b;
+            for (int q = 0; q < Q; ++q) acc[q] = b;
 #pragma unroll 4
             for (int i = 0; i < 64; i += 4) {
                 const float w0 = ro[RO_W2T + (i + 0) * RO_W2T_LD + o], w1 = ro[RO_W2T + (i + 1) * RO_W2T_LD + o];
                 const float w2 = ro[RO_W2T + (i + 2) * RO_W2T_LD + o], w3 = ro[RO_W2T + (i + 3) * RO_W2T_LD + o];
 #pragma unroll
-                for (int q = 0; q < 4; ++q) {
+                for (int q = 0; q < Q; ++q) {
                     const float4 h = *reinterpret_cast<const float4*>(H1 + (q0 + q) * 64 + i);
                     acc[q] = fmaf(w3, h.w, fmaf(w2, h.z, fmaf(w1, h.y, fmaf(w0, h.x, acc[q]))));
                 }
             }
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
+            for (int q = 0; q < Q; ++q) {
                 Z2[(q0 + q) * 32 + o] = acc[q];
                 // adjoint seed of the last layer: dE/dz2 = w3 * silu'(z2)
                 G2[(q0 + q) * 32 + o] = P[po.head_w3 + o] * dsilu_f(acc[q]);
             }
         }
         __syncthreads();
-        {   // E_a = w3 . silu(z2) + b3: warp w -> atoms 4w .. 4w + 3, lanes over the 32 inputs
+        {   // E_a = w3 . silu(z2) + b3: warp w -> A / 8 atoms, lanes over the 32 inputs
+            constexpr int Q = A / 8;
             const int w = t >> 5, lane = t & 31;
             const float w3 = P[po.head_w3 + lane];
 #pragma unroll
-            for (int q = 4 * w; q < 4 * w + 4; ++q) {
+            for (int q = Q * w; q < Q * w + Q; ++q) {
                 float e = w3 * silu_f(Z2[q * 32 + lane]);
 #pragma unroll
                 for (int off = 16; off > 0; off >>= 1) e += __shfl_xor_sync(0xffffffffu, e, off);
@@ -319,44 +329,46 @@ __global__ void __launch_bounds__(RO_NT, 2) readout_kernel(const float* __restri
             }
         }
         if (want_grad) {
-            {   // dE/dz1 = (W2^T g2) * silu'(z1): thread -> output o, atoms 8 (t / 64) .. + 8
-                const int o = t & 63, q0 = (t >> 6) * 8;
-                float acc[8];
+            {   // dE/dz1 = (W2^T g2) * silu'(z1): thread -> output o, A / 4 atoms
+                constexpr int Q = A / 4;
+                const int o = t & 63, q0 = (t >> 6) * Q;
+                float acc[Q];
 #pragma unroll
-                for (int q = 0; q < 8; ++q) acc[q] = 0.0f;
+                for (int q = 0; q < Q; ++q) acc[q] = 0.0f;
 #pragma unroll 4
                 for (int j = 0; j < 32; ++j) {
                     const float w = ro[RO_W2T + o * RO_W2T_LD + j];   // W2[j][o]
 #pragma unroll
-                    for (int q = 0; q < 8; ++q) acc[q] = fmaf(w, G2[(q0 + q) * 32 + j], acc[q]);
+                    for (int q = 0; q < Q; ++q) acc[q] = fmaf(w, G2[(q0 + q) * 32 + j], acc[q]);
                 }
 #pragma unroll
-                for (int q = 0; q < 8; ++q) G1[(q0 + q) * 64 + o] = acc[q] * dsilu_f(Z1[(q0 + q) * 64 + o]);
+                for (int q = 0; q < Q; ++q) G1[(q0 + q) * 64 + o] = acc[q] * dsilu_f(Z1[(q0 + q) * 64 + o]);
             }
             __syncthreads();
-            {   // dE/ds = W1^T g1: thread -> output o, atoms 16 (t / 128) .. + 16
-                const int o = t & 127, q0 = (t >> 7) * 16;
-                float acc[16];
+            {   // dE/ds = W1^T g1: thread -> output o, A / 2 atoms
+                constexpr int Q = A / 2;
+                const int o = t & 127, q0 = (t >> 7) * Q;
+                float acc[Q];
 #pragma unroll
-                for (int q = 0; q < 16; ++q) acc[q] = 0.0f;
+                for (int q = 0; q < Q; ++q) acc[q] = 0.0f;
 #pragma unroll 2
                 for (int j = 0; j < 64; j += 4) {
                     const float* wr = ro + RO_W1T + o * RO_W1T_LD + j;   // W1[j .. j + 3][o]
                     const float w0 = wr[0], w1 = wr[1], w2 = wr[2], w3 = wr[3];
 #pragma unroll
-                    for (int q = 0; q < 16; ++q) {
+                    for (int q = 0; q < Q; ++q) {
                         const float4 g = *reinterpret_cast<const float4*>(G1 + (q0 + q) * 64 + j);
                         acc[q] = fmaf(w3, g.w, fmaf(w2, g.z, fmaf(w1, g.y, fmaf(w0, g.x, acc[q]))));
                     }
                 }
 #pragma unroll
-                for (int q = 0; q < 16; ++q) {
+                for (int q = 0; q < Q; ++q) {
                     const int a = a0 + q0 + q;
                     if (a < n_atoms) xbar[(int64_t)a * 4 * H + o] = acc[q];
                 }
             }
             // the vector part of the seed is zero
-            for (int i = t; i < RO_ATOMS * (3 * H / 4); i += RO_NT) {
+            for (int i = t; i < A * (3 * H / 4); i += RO_NT) {
                 const int q = i / (3 * H / 4), k = i % (3 * H / 4), a = a0 + q;
                 if (a < n_atoms)
                     reinterpret_cast<float4*>(xbar + (int64_t)a * 4 * H + H)[k] = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -404,15 +416,23 @@ int launch_readout(const mlff_dims& d, const float* packed, const PackedOffsets&
     float* e_atom = ws_ptr<float>(ws, L.e_atom);
     float* xbar = ws_ptr<float>(ws, L.xbar);  // buffer 0
     const Status* status = ws_ptr<Status>(ws, L.status);
-    static std::once_flag once;
-    static cudaError_t attr_err = cudaSuccess;
-    std::call_once(once, [] {
-        attr_err = cudaFuncSetAttribute(readout_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)RO_SMEM);
-    });
-    if (attr_err != cudaSuccess) return cuda_status(attr_err, "readout smem attribute");
-    const int blocks = (int)std::min<int64_t>((sys.n_atoms + RO_ATOMS - 1) / RO_ATOMS, 2 * num_sms());
-    MLFF_LAUNCH_PDL("readout", readout_kernel, std::max(blocks, 1), RO_NT, RO_SMEM, st, packed, po, X, sys.n_atoms,
-                    e_atom, xbar, want_grad, status);
+    auto readout = [&](auto atoms) -> int {
+        constexpr int A = decltype(atoms)::value;
+        static std::once_flag once;
+        static cudaError_t attr_err = cudaSuccess;
+        std::call_once(once, [] {
+            attr_err = cudaFuncSetAttribute(readout_kernel<A>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                            (int)RoLayout<A>::SMEM);
+        });
+        if (attr_err != cudaSuccess) return cuda_status(attr_err, "readout smem attribute");
+        const int blocks = (int)std::min<int64_t>((sys.n_atoms + A - 1) / A, 2 * num_sms());
+        MLFF_LAUNCH_PDL("readout", readout_kernel<A>, std::max(blocks, 1), RO_NT, RoLayout<A>::SMEM, st, packed, po, X,
+                        sys.n_atoms, e_atom, xbar, want_grad, status);
+        return MLFF_OK;
+    };
+    const int r = sys.n_atoms <= 2 * 8 * 2 * num_sms() ? readout(std::integral_constant<int, 8>{})
+                                                       : readout(std::integral_constant<int, 32>{});
+    if (r) return r;
     MLFF_LAUNCH_PDL("energy_sum", energy_sum_kernel, std::min(std::max(sys.n_mol, 1), 152 * 8), 256, 0, st, e_atom, sys.mol_ptr, sys.n_mol,
                                                                                  out.energy, status);
     if (out.atom_energy)
