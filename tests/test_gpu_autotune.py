@@ -64,3 +64,27 @@ def test_autotune_caches_a_candidate(weights_bias):
     np.testing.assert_array_equal(E0.cpu().numpy(), E1.cpu().numpy())
     np.testing.assert_array_equal(F0.cpu().numpy(), F1.cpu().numpy())
     lib.mlff_autotune_set(_lib.PATH_TUNED_TC, b.n_atoms, b.n_mol, 0)
+
+
+@pytest.mark.parametrize("n", [1, 31, 33, 1000, 4863, 4865, 9800])
+def test_update_tiles_on_both_sides_of_one_tile_per_sm(weights_bias, n):
+    """The 32-atom update kernels (512 threads up to one tile per SM, 256 and
+    several tiles per CTA beyond) against the 64-atom ones: the same bits."""
+    from mlff_gb300 import _lib, systems
+    from mlff_gb300.engine import make_batch
+    lib = _lib.load()
+    s = systems.large_box(n, seed=5) if n >= 1000 else systems.lattice_molecule(n, seed=5)
+    per = bool(s.pbc.any())
+    b = make_batch(s.Z, s.pos.astype(np.float32), s.mol_ptr, s.box if per else None, s.pbc if per else None)
+    m = _model(weights_bias)
+    eng = m.engine()
+    eng.auto_tune = False
+    res = []
+    try:
+        for ut in (64, 32):
+            _lib.check(lib.mlff_autotune_set_shape(m.path, b.n_atoms, b.n_mol, 1, ut))
+            E, F, _ = eng.energy_forces(b, m.path, graph=False)
+            res.append((E, F))
+    finally:
+        lib.mlff_autotune_reset()
+    assert torch.equal(res[0][0], res[1][0]) and torch.equal(res[0][1], res[1][1])
