@@ -750,14 +750,12 @@ int launch_bwd_t(const TabArgs& a, float scale, cudaStream_t st) {
 
 template <bool L0>
 int launch_fwd(const TabShape& s, const TabArgs& a, cudaStream_t st) {
-    if (s.G == 4) return launch_fwd_t<4, true, L0>(a, st);
     if (s.G == 2) return launch_fwd_t<2, true, L0>(a, st);
     if (s.smem) return launch_fwd_t<1, true, L0>(a, st);
     return launch_fwd_t<1, false, L0>(a, st);
 }
 template <bool L0, bool PAIRS>
 int launch_bwd(const TabShape& s, const TabArgs& a, float scale, cudaStream_t st) {
-    if (s.G == 4) return launch_bwd_t<4, true, L0, PAIRS>(a, scale, st);
     if (s.G == 2) return launch_bwd_t<2, true, L0, PAIRS>(a, scale, st);
     if (s.smem) return launch_bwd_t<1, true, L0, PAIRS>(a, scale, st);
     if constexpr (!PAIRS) return launch_bwd_t<1, false, L0, PAIRS>(a, scale, st);

@@ -241,19 +241,27 @@ struct TabLaunch {
 
 // Receivers per group, and whether a CTA stages its table slice in shared
 // memory (221 KB, one bulk copy that overlaps the kernel before when that
-// leaves SMs idle).  After the tensor-core path's update kernels, which take
-// one SM per 32 atoms, it always pays (60 atoms: 390 against 405 us a call,
-// 1400: 661 against 688); the FP32 update kernels take more SMs (path 6: 60
-// atoms 466 against 423, 500: 556 against 543, 1000: 631 against 662; a
-// training step, 550 atoms, 2.96 against 3.17 ms of kernels).
+// leaves SMs idle).
+//
+// Groups share coefficient loads between receivers but choose the receiver's
+// sums per edge: 2 receivers are best for inference from 1,500 atoms
+// (16,858 atoms, path 5: 1 receiver 1,513 us of reverse pass, 2: 1,432, 4:
+// 1,505; path 6, both passes: 2,676, 2,473, 2,498), 1 for the passes of
+// training, which read more per edge (3,804 atoms: 1,246 against 1,337).
+//
+// After the tensor-core path's update kernels, which take one SM per 32 atoms,
+// staging always pays (60 atoms: 390 against 405 us a call, 1400: 661 against
+// 688); the FP32 update kernels take more SMs (path 6: 60 atoms 466 against
+// 423, 500: 556 against 543, 1000: 631 against 662; a training step, 550
+// atoms, 2.96 against 3.17 ms of kernels).
 struct TabShape {
     int G;
     bool smem;
 };
 inline TabShape tab_shape(int n_atoms, int path) {
-    if (n_atoms >= 4096) return {4, true};
+    if (path == MLFF_PATH_TRAIN_TABLE) return {1, n_atoms >= 400};
     if (n_atoms >= 1500) return {2, true};
-    return {1, path == MLFF_PATH_TABLE || n_atoms >= (path == MLFF_PATH_TRAIN_TABLE ? 400 : 750)};
+    return {1, path == MLFF_PATH_TABLE || n_atoms >= 750};
 }
 
 }  // namespace mlff

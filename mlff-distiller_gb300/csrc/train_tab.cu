@@ -518,8 +518,6 @@ template <int MODE, bool L0>
 int launch_pass(const PassArgs& a, cudaStream_t st) {
     ProfScope prof(PK_PLAIN_EDGE, st);
     const TabShape s = tab_shape(a.n_atoms, MLFF_PATH_TRAIN_TABLE);
-    if (s.G == 4) return launch_pass_t<MODE, 4, true, L0>(a, st);
-    if (s.G == 2) return launch_pass_t<MODE, 2, true, L0>(a, st);
     if (s.smem) return launch_pass_t<MODE, 1, true, L0>(a, st);
     return launch_pass_t<MODE, 1, false, L0>(a, st);
 }
@@ -902,7 +900,7 @@ int run_train(const mlff_dims& d, const float* P, const PackedOffsets& po, const
 
     // Value forward pass (records, X, Xt, uz, ua of every layer): the plain
     // path's, bit for bit (see the head of the file).
-    if ((r = launch_records(d, P, po, sys, L, ws, MLFF_PATH_TABLE_FP32, st))) return r;
+    if ((r = launch_records(d, P, po, sys, L, ws, MLFF_PATH_TRAIN_TABLE, st))) return r;
     {
         float* rowsX = ws_ptr<float>(ws, L.prows);   // [L + 1][N][4][H]
         if ((r = plain_forward(d, P, po, sys, L, ws, rowsX, st))) return r;
