@@ -382,8 +382,7 @@ __global__ void __launch_bounds__(REC_WARPS * 32) tab_records_kernel(RecArgs a) 
                 const int p = e0 + at + __popc(peers & lt);
                 float4* o = reinterpret_cast<float4*>(a.rec + p);
                 o[0] = make_float4(e.t, e.t, e.uy, e.uz);
-                o[1] = make_float4(e.ux, __int_as_float(e.b), __int_as_float(e.key * TAB_ROW_BYTES),
-                                   __int_as_float(e.r));
+                o[1] = make_float4(e.ux, __int_as_float(e.key * TAB_ROW_BYTES | e.r), __int_as_float(e.b), 0.f);
                 a.perm[p] = k;
             }
             if ((peers & lt) == 0) hw[e.key] = at + __popc(peers);
@@ -424,6 +423,7 @@ __global__ void __launch_bounds__(REC_WARPS * 32) tab_records_kernel(RecArgs a) 
     }
 }
 static_assert(TAB_NI < 127, "slot 127 holds the padding lanes");
+static_assert(TAB_ROW_BYTES % 16 == 0, "the receiver in the low bits of a row's offset");
 
 // ----------------------------------------------------------- edge kernels
 struct TabArgs {
@@ -474,9 +474,10 @@ __global__ void __launch_bounds__(NT, SMEM ? 1 : 4) tab_fwd_kernel(TabArgs a) {
                 }
             };
             auto edge = [&](const TabRec* rp, const float4& x) {
-                const float4 ra = reinterpret_cast<const float4*>(rp)[0], rb = reinterpret_cast<const float4*>(rp)[1];
-                const int off = __float_as_int(rb.z);
-                if (uni(off != cur)) {
+                const float4 ra = reinterpret_cast<const float4*>(rp)[0];
+                const float2 rb = reinterpret_cast<const float2*>(rp)[2];
+                const int off = __float_as_int(rb.y);
+                if (uni(other_row(off, cur))) {
                     c.load<SMEM>(table, off, lane);
                     cur = off;
                 }
@@ -503,7 +504,7 @@ __global__ void __launch_bounds__(NT, SMEM ? 1 : 4) tab_fwd_kernel(TabArgs a) {
                         s3 = fmaf(x.w, f1, fmaf(ra.w, f2, s3));
                     }
                 };
-                tab_switch<G>(__float_as_int(rb.w), [&](auto r) {
+                tab_switch<G>(off, [&](auto r) {
                     constexpr int R = decltype(r)::value;
                     add(acc01[R], acc2[R], acc3[R]);
                 });
@@ -612,9 +613,10 @@ __global__ void __launch_bounds__(NT, SMEM ? 1 : 4) tab_bwd_kernel(TabArgs a, fl
                 }
             };
             auto edge = [&](const TabRec* rp, const float4& x, const float4& y, float* v) {
-                const float4 ra = reinterpret_cast<const float4*>(rp)[0], rb = reinterpret_cast<const float4*>(rp)[1];
-                const int off = __float_as_int(rb.z);
-                if (uni(off != cur)) {
+                const float4 ra = reinterpret_cast<const float4*>(rp)[0];
+                const float2 rb = reinterpret_cast<const float2*>(rp)[2];
+                const int off = __float_as_int(rb.y);
+                if (uni(other_row(off, cur))) {
                     c.load<SMEM>(table, off, lane);
                     cur = off;
                 }
@@ -645,7 +647,7 @@ __global__ void __launch_bounds__(NT, SMEM ? 1 : 4) tab_bwd_kernel(TabArgs a, fl
                     v[2] = ti.z * f2;
                     v[3] = ti.w * f2;
                 };
-                tab_switch<G>(__float_as_int(rb.w), [&](auto r) {
+                tab_switch<G>(off, [&](auto r) {
                     constexpr int R = decltype(r)::value;
                     add(ta[R], acc01[R], acc2[R], acc3[R]);
                 });

@@ -48,15 +48,20 @@ __device__ __forceinline__ float reduce16(const float (&v)[16], int lane) {
 }
 
 // ------------------------------------------------------------ edge records
+// (a load that every lane makes of the same bytes costs the shared-memory
+// pipe a cycle per word, so an edge reads its first six words and a gather
+// the sender alone)
 struct __align__(16) TabRec {
     float t, t2;      // local coordinate, twice (an operand pair)
     float uy, uz;
     float ux;
+    int32_t off;      // byte offset of the interval's row in a table slice | receiver within the group
     int32_t sender;
-    int32_t off;      // byte offset of the interval's row in a table slice
-    int32_t r;        // receiver within the group
+    int32_t pad;
 };
-static_assert(sizeof(TabRec) == 32, "two 16-byte loads");
+static_assert(sizeof(TabRec) == 32, "a 16-byte and an 8-byte load");
+// the intervals of two edges differ (rows are multiples of 16 bytes)
+__device__ __forceinline__ bool other_row(int off, int cur) { return (unsigned)(off ^ cur) >= 4u; }
 
 // The 18 coefficients of one channel: pairs (phi_s, phi_v1) and phi_v2.
 struct Coef {
@@ -64,8 +69,9 @@ struct Coef {
     float b[TAB_NC];
     template <bool SMEM>
     __device__ __forceinline__ void load(const char* table, int off, int lane) {
-        const float4* q = reinterpret_cast<const float4*>(table + off) + lane;
-        const float2* q2 = reinterpret_cast<const float2*>(table + off + 2048) + lane;
+        const char* row = table + (off & ~3);
+        const float4* q = reinterpret_cast<const float4*>(row) + lane;
+        const float2* q2 = reinterpret_cast<const float2*>(row + 2048) + lane;
         float4 v[4];
 #pragma unroll
         for (int j = 0; j < 4; ++j) v[j] = SMEM ? q[32 * j] : __ldg(q + 32 * j);

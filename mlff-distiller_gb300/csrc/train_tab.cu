@@ -84,7 +84,7 @@ __global__ void __launch_bounds__(256) edge_maps_kernel(MapArgs a) {
         const int k = a.perm[p];
         const float4 ra = reinterpret_cast<const float4*>(a.rec + p)[0], rb = reinterpret_cast<const float4*>(a.rec + p)[1];
         a.geo[k] = make_float4(rb.x, ra.z, ra.w, ra.x);
-        a.key[k] = __float_as_int(rb.z) / TAB_ROW_BYTES;
+        a.key[k] = __float_as_int(rb.y) / TAB_ROW_BYTES;
         if (!a.dual) continue;
         const int i = a.erecv[k], j = a.col[k], m = a.atom_mol[i];
         Box bx;
@@ -424,9 +424,10 @@ __global__ void __launch_bounds__(NT, SMEM ? 1 : 4) tab_pass_kernel(PassArgs a) 
                 }
             };
             auto edge = [&](const TabRec* rp, const In& in) {
-                const float4 ra = reinterpret_cast<const float4*>(rp)[0], rb = reinterpret_cast<const float4*>(rp)[1];
-                const int off = __float_as_int(rb.z);
-                if (uni(off != cur)) {
+                const float4 ra = reinterpret_cast<const float4*>(rp)[0];
+                const float2 rb = reinterpret_cast<const float2*>(rp)[2];
+                const int off = __float_as_int(rb.y);
+                if (uni(other_row(off, cur))) {
                     c.load<SMEM>(table, off, lane);
                     cur = off;
                 }
@@ -454,7 +455,7 @@ __global__ void __launch_bounds__(NT, SMEM ? 1 : 4) tab_pass_kernel(PassArgs a) 
                         m[3] = fmaf(in.gt.z, f2, fmaf(ra.w, d2, m[3]));
                     }
                 }
-                tab_switch<G>(__float_as_int(rb.w), [&](auto r) {
+                tab_switch<G>(off, [&](auto r) {
                     constexpr int R = decltype(r)::value;
 #pragma unroll
                     for (int k = 0; k < 4; ++k) acc[R][k] += m[k];
