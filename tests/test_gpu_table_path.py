@@ -1,6 +1,6 @@
 """Tabulated edge filters (GPU): the table path against the float64 oracle
 and the network evaluation at sizes on both sides of its receiver groups
-(1, 2 and 4 receivers; table read from memory or staged in shared memory),
+(1 and 2 receivers; table read from memory or staged in shared memory),
 for open and periodic batches, atoms without neighbours and ragged last
 groups; the accuracy class of tables of sharp and of many-basis filters; and
 the fallback when the table does not serve the weights.
@@ -53,7 +53,7 @@ def system(name):
     return systems.concat([far, s, far])
 
 
-# group shapes change at 1,500 and 4,096 atoms
+# group shapes change at 1,500 atoms, staging at 400 (training) and 750
 SIZES = ["isolated", "molecules1", "molecules7", "molecules30", "water64", "box1499", "box1500", "box1503",
          "box4095", "box4097", "molecules120"]
 
