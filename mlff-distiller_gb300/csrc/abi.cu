@@ -193,7 +193,8 @@ WsLayout ws_layout(const mlff_dims& d, int32_t n_atoms, int32_t n_mol, int64_t c
         L.uh = take(fs * N * H);
         L.abar = take(fs * N * H3);
     }
-    if (path == MLFF_PATH_PLAIN_FP32 || path == MLFF_PATH_TRAIN || path == MLFF_PATH_TRAIN_TABLE) {
+    // filters by pair of atoms (plain.cu): every path that run_plain evaluates, and the table path's training
+    if (path == MLFF_PATH_PLAIN_FP32 || path == MLFF_PATH_TRAIN || dual || train_table) {
         L.pbase = take(4 * ((size_t)N + 1));
         L.pidx = take(4 * cap);
         L.pedge = take(4 * ((size_t)cap / 2 + 1));
