@@ -480,30 +480,39 @@ class StudentForceField(nn.Module):
         return base if self._engine is None else self._engine.route(base)
 
     def _slots(self, check: bool = False):
-        """(parameters, all, buffers, modules): (tensor dict, name, full name)
-        of every parameter, (tensor dict, name) of every parameter and
-        buffer, the first form of every buffer, and the modules' state: the
-        modules' own dicts, looked up once (walking the module tree by name
-        costs 0.1 ms, several times a training step) and, with ``check``,
-        again when a module, parameter or buffer was added or replaced by
-        another object."""
+        """(parameters, all, buffers, modules, children): (tensor dict, name,
+        full name) of every parameter, (tensor dict, name) of every parameter
+        and buffer, the first form of every buffer, the modules' state, and
+        the child dicts with the children in them: the modules' own dicts,
+        looked up once (walking the module tree by name costs 0.1 ms, several
+        times a training step) and, with ``check``, again when a module,
+        parameter or buffer was added or replaced by another object."""
         if check and self._weight_slots is not None and any(
                 len(par) != n_par or len(buf) != n_buf or tuple(sub.values()) != kids
                 for par, n_par, buf, n_buf, sub, kids in self._weight_slots[3]):
             self._weight_slots = None
         if self._weight_slots is None:
+            self._packed_version = None
             mods = list(self.named_modules())
             named = [[(d(m), n, f"{prefix}.{n}" if prefix else n) for prefix, m in mods for n in d(m)]
                      for d in (lambda m: m._parameters, lambda m: m._buffers)]
+            subs = [m._modules for _, m in mods if m._modules]
             self._weight_slots = (named[0], [(d, n) for d, n, _ in named[0] + named[1]], named[1],
                                   # (the dicts, not the modules: this one would keep itself alive)
                                   [(m._parameters, len(m._parameters), m._buffers, len(m._buffers), m._modules,
-                                    tuple(m._modules.values())) for _, m in mods])
+                                    tuple(m._modules.values())) for _, m in mods],
+                                  (subs, [k for sub in subs for k in sub.values()]))
         return self._weight_slots
 
     def _weights_version(self):
         """(address, in-place version) of every parameter and buffer: changes
-        when a weight is updated in place, reassigned or moved."""
+        when a weight is updated in place, reassigned or moved, or a module
+        is replaced (the weights lie in the modules below those that had
+        children, so these children are compared on every call: 2 us)."""
+        if self._weight_slots is not None:
+            subs, kids = self._weight_slots[4]
+            if [k for sub in subs for k in sub.values()] != kids:
+                self._weight_slots = None
         return tuple((t.data_ptr(), t._version) if t is not None else None
                      for t in (d[n] for d, n in self._slots()[1]))
 
@@ -517,7 +526,7 @@ class StudentForceField(nn.Module):
             self._packed_version = None
         v = self._weights_version()
         if v != self._packed_version:
-            params, _, buffers, _ = self._slots()
+            params, _, buffers = self._slots()[:3]
             self._engine.pack({full: d[n] for d, n, full in params + buffers if d[n] is not None})
             self._packed_version = v
         return self._engine
