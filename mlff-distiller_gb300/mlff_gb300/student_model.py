@@ -493,7 +493,8 @@ class StudentForceField(nn.Module):
             self._weight_slots = None
         if self._weight_slots is None:
             self._packed_version = None
-            mods = list(self.named_modules())
+            # (a shared module under each of its names, as state_dict() lists it)
+            mods = list(self.named_modules(remove_duplicate=False))
             named = [[(d(m), n, f"{prefix}.{n}" if prefix else n) for prefix, m in mods for n in d(m)]
                      for d in (lambda m: m._parameters, lambda m: m._buffers)]
             subs = [m._modules for _, m in mods if m._modules]

@@ -74,3 +74,30 @@ def test_energies_follow_a_replaced_submodule():
     other.load_state_dict(m.state_dict())
     got = energies(m)
     assert not torch.equal(got, e) and torch.equal(got, energies(other))
+
+
+def test_shared_blocks_are_packed_under_both_names(model):
+    model.interactions[1] = model.interactions[0]
+    assert_packed(model, 1)
+    with torch.no_grad():
+        model.interactions[1].update.mixing_matrix.add_(1.0)
+    assert_packed(model, 2)
+
+
+def test_shared_blocks_train_once():
+    """named_parameters() lists a shared parameter once."""
+    from mlff_gb300.student_model import StudentForceField, _trainable
+    m = StudentForceField()
+    m.interactions[2] = m.interactions[0]
+    assert [(n, id(p)) for n, p in _trainable(m, True)] == [(n, id(p)) for n, p in m.named_parameters()]
+
+
+@pytest.mark.gpu
+def test_shared_blocks_evaluate_as_equal_blocks():
+    from mlff_gb300.student_model import StudentForceField
+    torch.manual_seed(3)
+    m = StudentForceField().cuda().eval()
+    other = StudentForceField().cuda().eval()
+    m.interactions[1] = m.interactions[0]
+    other.load_state_dict(m.state_dict())
+    assert torch.equal(energies(m), energies(other))
