@@ -248,7 +248,6 @@ class VelocityVerletGPU:
 
     # one library call of n steps on the current stream
     def _call(self, n_steps: int, cap: int, e_trace: Optional[torch.Tensor], k_trace: Optional[torch.Tensor]):
-        self.path = self.engine._checked_path(self.path)
         ws = self.engine.workspace_for(self.N, self.B, cap, self.path)
         st = _lib.MDState()
         st.pos, st.vel = self.pos.data_ptr(), self.vel.data_ptr()
@@ -289,6 +288,15 @@ class VelocityVerletGPU:
                                                     ctypes.c_double(th["kT"]), ctypes.c_uint64(th["seed"]), n_steps,
                                                     ws.data_ptr(), ws.numel(), _stream_handle()))
 
+    def _select_path(self):
+        """Weights packed since the last run may need another path than the
+        one chosen for the earlier weights; the edges are the same."""
+        path = self.engine._checked_path(self.path)
+        if path != self.path:
+            cap = self.engine.edge_capacity
+            cap[path] = max(cap.get(path, 0), cap.get(self.path, 0))
+            self.path = path
+
     def _capacity(self) -> int:
         return max(self.engine.capacity(self.N, self.path),
                    int(self.engine.edge_capacity.get(self.path, 0) * self.headroom) + 1024)
@@ -298,6 +306,7 @@ class VelocityVerletGPU:
         """Advance n_steps.  Returns per-step potential / kinetic energy per
         structure, shape [n_steps, B] (eV), when record is set -- as device
         tensors with to_host=False (e.g. for energy_metrics.replica_energy_stats)."""
+        self._select_path()
         if not self._forces_valid:
             self.compute_forces()
         cap = self._capacity()
@@ -337,7 +346,7 @@ class VelocityVerletGPU:
     def _graph(self, k: int, cap: int, record: bool):
         ws = self.engine.workspace_for(self.N, self.B, cap, self.path)
         th = self.thermostat
-        key = (k, cap, record, ws.data_ptr(), None if th is None else (th["friction"], th["kT"], th["seed"]),
+        key = (k, cap, record, ws.data_ptr(), self.path, None if th is None else (th["friction"], th["kT"], th["seed"]),
                None if self.npt is None else tuple(sorted(self.npt.items())))
         if key in self._graphs:
             return self._graphs[key]
