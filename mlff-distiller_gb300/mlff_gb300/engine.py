@@ -363,16 +363,34 @@ class Engine:
 
     def capture(self, batch: Batch, path: int = _lib.PATH_TUNED_TC, forces: bool = True):
         """One energy_forces call captured in a CUDA graph, for repeated
-        evaluation of a fixed batch (the edge capacity must already be known:
-        call energy_forces once first).  Returns (replay, E, F): replay()
-        launches the graph on the current stream and refreshes E and F."""
-        self.energy_forces(batch, path, forces=forces, graph=False)   # sizes capacity and workspace
-        torch.cuda.synchronize()
-        g = torch.cuda.CUDAGraph()
-        with torch.cuda.graph(g):
-            E, F, _ = self.energy_forces(batch, path, forces=forces, check=False, graph=False)
-        self._graph_keep = g
-        return g.replay, E, F
+        evaluation of a fixed batch.  Returns (replay, E, F): replay()
+        launches the graph on the current stream and refreshes E and F; when
+        weights packed since need another path (route), it captures the call
+        again first."""
+        E = F = graph = used = ws = None
+
+        def record():
+            nonlocal E, F, graph, used, ws
+            self.energy_forces(batch, path, forces=forces, graph=False)   # sizes capacity and workspace
+            torch.cuda.synchronize()
+            graph, used = torch.cuda.CUDAGraph(), self._checked_path(path)
+            with torch.cuda.graph(graph):
+                e, f, _ = self.energy_forces(batch, path, forces=forces, check=False, graph=False)
+                if E is None:
+                    E, F = e, f
+                else:
+                    E.copy_(e)
+                    if forces:
+                        F.copy_(f)
+            ws = self.workspace   # the graph holds its address
+
+        def replay():
+            if self._checked_path(path) != used:
+                record()
+            graph.replay()
+
+        record()
+        return replay, E, F
 
     def neighbors(self, batch: Batch):
         """CSR (row_ptr, col) of the radius graph, for tests and tools."""

@@ -5,7 +5,7 @@ import numpy as np
 import pytest
 import torch
 
-from test_gpu_table_path import model
+from test_gpu_table_path import batch_of, model
 
 pytestmark = pytest.mark.gpu
 
@@ -35,3 +35,27 @@ def test_md_goes_on_with_weights_the_tables_do_not_serve(weights_bias, precision
         np.testing.assert_array_equal(a["potential_energy"], b["potential_energy"])
     np.testing.assert_array_equal(runs[0].positions(), runs[1].positions())
     assert not np.array_equal(first[0]["potential_energy"][-1], second[0]["potential_energy"][0])
+
+
+@pytest.mark.parametrize("precision", ["fp16x3", "tuned_fp32"])
+def test_captured_call_follows_the_weights(weights_bias, precision):
+    """Engine.capture's replay refreshes the same two tensors with the
+    results of the weights packed last."""
+    from mlff_gb300 import _lib, systems
+    s = systems.molecule_batch(3, 20, 40, seed=6)
+    b = batch_of(s)
+    m = model(weights_bias, precision)
+    eng = m.engine()
+    path, network = ((_lib.PATH_TABLE, _lib.PATH_TUNED_TC) if precision == "fp16x3" else
+                     (_lib.PATH_TABLE_FP32, _lib.PATH_TUNED_FP32))
+    assert m.path == path
+    replay, E, F = eng.capture(b, path)
+    old = {k: v.clone() for k, v in m.state_dict().items()}
+    for change, now in ((None, path), (sharpen, network), (lambda m: m.load_state_dict(old), path)):
+        if change is not None:
+            change(m)
+            m.engine()
+        replay()
+        replay()
+        E0, F0, _ = eng.energy_forces(b, now, graph=False)
+        assert torch.equal(E, E0) and torch.equal(F, F0)
