@@ -412,7 +412,8 @@ int mlff_profile_end(double *ms_by_kind, int64_t *launches_by_kind, int32_t n_ki
  * (0 removes the entry; the bucket's update tile is kept), _query_shape
  * reads both shapes (f, update_atoms) and _set_shape pins both (f = 0
  * removes the entry), _reset empties the cache.  Untuned buckets use f = 1
- * and 64-atom update tiles. */
+ * and 64-atom update tiles; path 5 takes path 1's entry of the bucket while
+ * it has none of its own. */
 int mlff_autotune(const mlff_dims *dims, const void *packed, const mlff_system *sys, int64_t edge_capacity,
                   int32_t path, const mlff_outputs *out, void *workspace, size_t workspace_bytes,
                   mlff_stream_t stream, int32_t repeats, int32_t *chosen, double *ms_per_candidate);

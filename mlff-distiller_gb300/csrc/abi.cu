@@ -94,14 +94,21 @@ int ceil_log2(int64_t x) {
 std::tuple<int, int, int> tune_key(int32_t path, int32_t n_atoms, int32_t n_mol) {
     return {path, ceil_log2(std::max(n_atoms, 1)), ceil_log2(std::max(n_mol, 1))};
 }
+// the bucket's shape (g_tune_mu held): the table form of path 1 takes path 1's
+// shape until it has one of its own, so that a shape set for path 1 reaches
+// the calls that the tables serve
+TunedShape cached_shape(int32_t path, int32_t n_atoms, int32_t n_mol) {
+    auto it = g_tune.find(tune_key(path, n_atoms, n_mol));
+    if (it == g_tune.end() && path == MLFF_PATH_TABLE) it = g_tune.find(tune_key(MLFF_PATH_TUNED_TC, n_atoms, n_mol));
+    return it == g_tune.end() ? DEFAULT_SHAPE : it->second;
+}
 }  // namespace
 
 TunedShape tuned_shape(int32_t path, int32_t n_atoms, int32_t n_mol) {
     if (!has_tc_edges(path)) return DEFAULT_SHAPE;
     if (g_tune_override.factor) return g_tune_override;
     std::lock_guard<std::mutex> lk(g_tune_mu);
-    auto it = g_tune.find(tune_key(path, n_atoms, n_mol));
-    return it == g_tune.end() ? DEFAULT_SHAPE : it->second;
+    return cached_shape(path, n_atoms, n_mol);
 }
 
 WsLayout ws_layout(const mlff_dims& d, int32_t n_atoms, int32_t n_mol, int64_t cap, int32_t path) {
@@ -482,13 +489,9 @@ int mlff_autotune_set(int32_t path, int32_t n_atoms, int32_t n_mol, int32_t fact
     }
     if (!has_tc_edges(path)) { set_error("only the tensor-core paths have a tunable shape"); return MLFF_ERR_INVALID; }
     std::lock_guard<std::mutex> lk(g_tune_mu);
-    const auto key = tune_key(path, n_atoms, n_mol);
-    if (factor == 0) {
-        g_tune.erase(key);
-    } else {
-        auto it = g_tune.find(key);   // the bucket's update tile stays as it was
-        g_tune[key] = TunedShape{factor, it == g_tune.end() ? DEFAULT_SHAPE.update_atoms : it->second.update_atoms};
-    }
+    const TunedShape sh{factor, cached_shape(path, n_atoms, n_mol).update_atoms};   // the bucket's update tile stays
+    if (factor == 0) g_tune.erase(tune_key(path, n_atoms, n_mol));
+    else g_tune[tune_key(path, n_atoms, n_mol)] = sh;
     return MLFF_OK;
 }
 

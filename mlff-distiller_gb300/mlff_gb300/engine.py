@@ -260,7 +260,7 @@ class Engine:
             if self.auto_tune and path in (_lib.PATH_TUNED_TC, _lib.PATH_TABLE) and _bucket(path, N, B) not in _tuned_buckets:
                 db = batch if not to_host else Batch(batch.Z.to(self.device), batch.pos.to(self.device),
                                                      batch.mol_ptr, batch.box, batch.pbc)
-                self.autotune(db, path)
+                self._autotune(db, path)
             if to_host:
                 dev = self.device
                 db = Batch(batch.Z.to(dev), batch.pos.to(dev), batch.mol_ptr, batch.box, batch.pbc)
@@ -339,7 +339,15 @@ class Engine:
         size bucket (mlff_autotune: a few timed calls per candidate, then
         cached by the library for every call of the bucket).  Returns the
         choices and the milliseconds per call of each partition factor.
-        Synchronises the stream; not for use during stream capture."""
+        A shape tuned for path 1 also serves its table form (path 5), which
+        is then not tuned by itself.  Synchronises the stream; not for use
+        during stream capture."""
+        res = self._autotune(batch, path, repeats)
+        if path == _lib.PATH_TUNED_TC:
+            _tuned_buckets.add(_bucket(_lib.PATH_TABLE, batch.n_atoms, batch.n_mol))
+        return res
+
+    def _autotune(self, batch: Batch, path: int, repeats: int = AUTOTUNE_REPEATS) -> dict:
         path = self._checked_path(path)
         self.energy_forces(batch, path, graph=False)       # sizes the edge capacity and workspace
         N, B = batch.n_atoms, batch.n_mol
