@@ -60,6 +60,9 @@ typedef struct CUstream_st *mlff_stream_t; /* same type as cudaStream_t */
  * tables (class 2); the workspace also serves mlff_param_grads_table and its
  * force term */
 #define MLFF_PATH_TRAIN_TABLE 7
+/* path 7's energies and forces, bit for bit, without the space of the
+ * gradient passes (100,000 atoms, 6.4 M edge slots: 10.4 against 19.1 GB) */
+#define MLFF_PATH_TRAIN_TABLE_FORWARD 8
 
 #define MLFF_MAX_LAYERS 8
 

@@ -118,7 +118,8 @@ WsLayout ws_layout(const mlff_dims& d, int32_t n_atoms, int32_t n_mol, int64_t c
     L.L = d.n_layers;
     const bool tc = has_tc_edges(path);
     const bool train_table = path == MLFF_PATH_TRAIN_TABLE;
-    const bool table = path == MLFF_PATH_TABLE || path == MLFF_PATH_TABLE_FP32 || train_table;
+    const bool train_fwd = path == MLFF_PATH_TRAIN_TABLE_FORWARD;
+    const bool table = path == MLFF_PATH_TABLE || path == MLFF_PATH_TABLE_FP32 || train_table || train_fwd;
     // arrays sized for the largest partition factor, so that tuning never changes the size
     const int64_t P_max = (int64_t)persistent_ctas(path) * (tc ? TUNE_FACTOR_MAX : 1);
     const TunedShape shape = tuned_shape(path, n_atoms, n_mol);
@@ -201,7 +202,7 @@ WsLayout ws_layout(const mlff_dims& d, int32_t n_atoms, int32_t n_mol, int64_t c
         L.abar = take(fs * N * H3);
     }
     // filters by pair of atoms (plain.cu): every path that run_plain evaluates, and the table path's training
-    if (path == MLFF_PATH_PLAIN_FP32 || path == MLFF_PATH_TRAIN || dual || train_table) {
+    if (path == MLFF_PATH_PLAIN_FP32 || path == MLFF_PATH_TRAIN || dual || train_table || train_fwd) {
         L.pbase = take(4 * ((size_t)N + 1));
         L.pidx = take(4 * cap);
         L.pedge = take(4 * ((size_t)cap / 2 + 1));
@@ -212,6 +213,7 @@ WsLayout ws_layout(const mlff_dims& d, int32_t n_atoms, int32_t n_mol, int64_t c
         L.gpart = take(fs * GRAD_SPLIT * H3 * H);
         L.gmix = take(fs * GRAD_MIX_BLOCKS * 9);
     }
+    if (train_table || train_fwd) p = train_forward_workspace(L, p);
     if (train_table) p = train_table_workspace(L, d, p);
     L.total = p;
     return L;
@@ -248,7 +250,7 @@ static int check_sys(const mlff_system* s, int64_t cap) {
 static int check_path(int32_t path) {
     if (path != MLFF_PATH_PLAIN_FP32 && path != MLFF_PATH_TUNED_TC && path != MLFF_PATH_TUNED_FP32 &&
         path != MLFF_PATH_TRAIN && path != MLFF_PATH_TRAIN_FORCES && path != MLFF_PATH_TABLE &&
-        path != MLFF_PATH_TABLE_FP32 && path != MLFF_PATH_TRAIN_TABLE) {
+        path != MLFF_PATH_TABLE_FP32 && path != MLFF_PATH_TRAIN_TABLE && path != MLFF_PATH_TRAIN_TABLE_FORWARD) {
         set_error("unknown path %d", path);
         return MLFF_ERR_INVALID;
     }
@@ -273,7 +275,7 @@ int energy_forces_impl(const mlff_dims& d, const void* packed, const mlff_system
     const float* P = static_cast<const float*>(packed);
     if (path == MLFF_PATH_PLAIN_FP32 || path == MLFF_PATH_TRAIN || path == MLFF_PATH_TRAIN_FORCES)
         return run_plain(d, P, po, sys, L, ws, out, st, nullptr, vf);
-    if (path == MLFF_PATH_TABLE_FP32 || path == MLFF_PATH_TRAIN_TABLE) return run_table(d, P, po, sys, L, ws, out, path, st, vf);
+    if (path == MLFF_PATH_TABLE_FP32 || is_train_table(path)) return run_table(d, P, po, sys, L, ws, out, path, st, vf);
     return run_tuned(d, P, po, sys, L, ws, out, path, st, vf);
 }
 int md_kick_drift(const WsLayout& L, void* ws, mlff_md_state* s, double dt, cudaStream_t st);

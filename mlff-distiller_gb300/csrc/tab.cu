@@ -817,12 +817,12 @@ int table_forward(const mlff_dims& d, const float* P, const PackedOffsets& po, c
     return MLFF_OK;
 }
 
-// The FP32 path with tabulated filters (MLFF_PATH_TABLE_FP32; MLFF_PATH_TRAIN_TABLE:
-// its reverse pass).
+// The FP32 path with tabulated filters (MLFF_PATH_TABLE_FP32; the training
+// paths: its reverse pass).
 int run_table(const mlff_dims& d, const float* P, const PackedOffsets& po, const mlff_system& sys, const WsLayout& L,
               void* ws, const mlff_outputs& out, int path, cudaStream_t st, const VerletFuse* vf) {
     int r;
-    if (path == MLFF_PATH_TRAIN_TABLE) {
+    if (is_train_table(path)) {
         // A training step's energies and forces: the fused FP32 path's forward
         // pass, bit for bit.  The loss divides by |F| and the gradients by |v|,
         // so another forward pass, as exact, moves them by up to 5e-5.

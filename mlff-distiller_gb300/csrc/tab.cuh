@@ -67,7 +67,13 @@ int fused_fp32_forward(const mlff_dims& d, const float* P, const PackedOffsets& 
 // forward pass with the tables: records, X, Xt, uz, ua of every layer
 int table_forward(const mlff_dims& d, const float* P, const PackedOffsets& po, const mlff_system& sys,
                   const WsLayout& L, void* ws, int path, cudaStream_t st);
-// training (train_tab.cu): offsets of its arrays from p on; returns the end
+// a training step's energies and forces (8: in a workspace without the gradient passes' arrays)
+inline bool is_train_table(int path) {
+    return path == MLFF_PATH_TRAIN_TABLE || path == MLFF_PATH_TRAIN_TABLE_FORWARD;
+}
+// training (train_tab.cu): offsets from p on, returns the end: the arrays of
+// the forward pass by pairs, and those that the gradient passes add
+size_t train_forward_workspace(WsLayout& L, size_t p);
 size_t train_table_workspace(WsLayout& L, const mlff_dims& d, size_t p);
 struct GradCtx;
 int run_train_table(const mlff_dims& d, const float* P, const PackedOffsets& po, const mlff_system& sys,

@@ -265,7 +265,7 @@ struct TabShape {
     bool smem;
 };
 inline TabShape tab_shape(int n_atoms, int path) {
-    if (path == MLFF_PATH_TRAIN_TABLE) return {1, n_atoms >= 400};
+    if (is_train_table(path)) return {1, n_atoms >= 400};
     if (n_atoms >= 1500) return {2, true};
     return {1, path == MLFF_PATH_TABLE || n_atoms >= 750};
 }

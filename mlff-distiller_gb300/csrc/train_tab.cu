@@ -1076,12 +1076,23 @@ int run_train(const mlff_dims& d, const float* P, const PackedOffsets& po, const
 
 }  // namespace
 
+static size_t take_bytes(size_t& p, size_t bytes) {
+    const size_t q = p;
+    p += (bytes + 255) & ~size_t(255);
+    return q;
+}
+
+size_t train_forward_workspace(WsLayout& L, size_t p) {
+    const int64_t pairs = L.cap / 2 + 1;   // filters by pair of atoms
+    L.erbf = take_bytes(p, sizeof(float) * pairs * RMAX);
+    L.fh = take_bytes(p, sizeof(float) * pairs * H);
+    L.ff = take_bytes(p, sizeof(float) * pairs * H3);
+    L.pgeo = take_bytes(p, sizeof(float4) * L.cap);
+    return p;
+}
+
 size_t train_table_workspace(WsLayout& L, const mlff_dims& d, size_t p) {
-    auto take = [&](size_t bytes) {
-        size_t q = p;
-        p += (bytes + 255) & ~size_t(255);
-        return q;
-    };
+    auto take = [&](size_t bytes) { return take_bytes(p, bytes); };
     const int64_t N = L.N, nseg = (L.cap + SEG - 1) / SEG;
     const int64_t nscan = (int64_t)TAB_NI * nseg + 1;
     L.txtbar = take(sizeof(float4) * 2 * N * H);
@@ -1103,14 +1114,9 @@ size_t train_table_workspace(WsLayout& L, const mlff_dims& d, size_t p) {
     L.tcst = take(4 * (TAB_NI + 1));
     L.thead = take(sizeof(float) * N * (2 * 64 * 3 + 2 * 32 * 2 + 32 + 1));
     L.tadj = take(sizeof(float) * (L.cap / CHUNK + TAB_NI + 1) * 6 * TAB_NC * H);
-    // the forward passes, filters by pair of atoms
-    const int64_t pairs = L.cap / 2 + 1;
+    // the value forward pass
     L.prows = take(sizeof(float) * (L.L + 1) * N * 4 * H);
-    L.erbf = take(sizeof(float) * pairs * RMAX);
-    L.fz = take(sizeof(float) * pairs * H);
-    L.fh = take(sizeof(float) * pairs * H);
-    L.ff = take(sizeof(float) * pairs * H3);
-    L.pgeo = take(sizeof(float4) * L.cap);
+    L.fz = take(sizeof(float) * (L.cap / 2 + 1) * H);
     L.tnode = take(sizeof(float) * 2 * NODES * (H3 + H));
     L.temb = take(sizeof(float) * EMB_SPLIT * (size_t)d.n_species * H);
     return p;

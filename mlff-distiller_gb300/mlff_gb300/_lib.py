@@ -32,6 +32,7 @@ PATH_TRAIN_FORCES = 4
 PATH_TABLE = 5
 PATH_TABLE_FP32 = 6
 PATH_TRAIN_TABLE = 7
+PATH_TRAIN_TABLE_FORWARD = 8
 
 PATHS = {"plain": PATH_PLAIN_FP32, "fp32": PATH_PLAIN_FP32, "plain_fp32": PATH_PLAIN_FP32,
          "fp16x3": PATH_TUNED_TC, "tc": PATH_TUNED_TC, "tuned": PATH_TUNED_TC,

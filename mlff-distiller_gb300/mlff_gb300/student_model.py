@@ -272,10 +272,10 @@ def _trainable(model, check: bool = False):
 
 class _EnergyTrain(torch.autograd.Function):
     """Training-mode E = model(positions), differentiable in the parameters
-    to second order.  The forward value and forces come from the fused FP32
-    path (no per-edge activations are stored, so a forward-only call stays
-    small); the parameter gradients from the plain FP32 path's reverse
-    passes, recomputed in backward.  backward(g): the position gradient
+    to second order.  The forward value and forces come from
+    Engine.train_energy_forces, whose workspace a forward-only call holds; the
+    parameter gradients from the reverse passes of training.param_grads and
+    force_term_grads, recomputed in backward.  backward(g): the position gradient
     sum_b g_b dE_b/dpos and
     the parameter gradients sum_b g_b dE_b/dtheta (mlff_param_grads).  When
     the backward itself is recorded (torch.autograd.grad(E, pos,
@@ -287,12 +287,7 @@ class _EnergyTrain(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, positions, model, batch, mol_index, *params):
-        from . import _lib
-        eng = model.engine()
-        path = eng.route(_lib.PATH_TUNED_FP32)
-        if path == _lib.PATH_TABLE_FP32:
-            path = _lib.PATH_TRAIN_TABLE   # path 2's forward pass, reverse pass through the tables
-        E, F, _ = eng.energy_forces(batch, path, forces=True)
+        E, F, _ = model.engine().train_energy_forces(batch)
         ctx.model, ctx.batch = model, batch
         ctx.save_for_backward(F, mol_index, *params)
         return E.to(positions.dtype)
