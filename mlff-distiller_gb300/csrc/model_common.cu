@@ -702,7 +702,7 @@ __global__ void __launch_bounds__(128) update_bwd_kernel(const float* __restrict
                                                          const float* __restrict__ Xt, const float* __restrict__ uz,
                                                          const float* __restrict__ ua,
                                                          const float* __restrict__ xbar_out, int32_t n_atoms,
-                                                         float* __restrict__ xtbar, int out_quads, const Status* st) {
+                                                         float* __restrict__ xtbar, const Status* st) {
     __shared__ float abar[UPD_ATOMS][H3];
     __shared__ float zbar[UPD_ATOMS][H];
     __shared__ float mix[9];
@@ -793,14 +793,9 @@ __global__ void __launch_bounds__(128) update_bwd_kernel(const float* __restrict
             float n = pair_distance(vt[0][q], vt[1][q], vt[2][q]);
             float sc = n > 0.0f ? cn[q] / n : 0.0f;     // d|v|/dv = v/|v|, 0 at v = 0
             float* o = xtbar + (int64_t)a * 4 * H;
-            if (out_quads) {
-                reinterpret_cast<float4*>(o)[c] = make_float4(sb[q] + cs[q], vb[0][q] + sc * vt[0][q],
-                                                              vb[1][q] + sc * vt[1][q], vb[2][q] + sc * vt[2][q]);
-            } else {
-                o[c] = sb[q] + cs[q];
+            o[c] = sb[q] + cs[q];
 #pragma unroll
-                for (int i = 0; i < 3; ++i) o[(1 + i) * H + c] = vb[i][q] + sc * vt[i][q];
-            }
+            for (int i = 0; i < 3; ++i) o[(1 + i) * H + c] = vb[i][q] + sc * vt[i][q];
         }
         __syncthreads();
     }
@@ -833,7 +828,7 @@ int launch_update_bwd(const mlff_dims& d, const float* packed, const LayerOffset
     const float* ua = ws_ptr<float>(ws, L.ua) + (int64_t)layer * L.N * H3;
     int blocks = (int)std::min<int64_t>((L.N + UPD_ATOMS - 1) / UPD_ATOMS, 152 * 4);
     update_bwd_kernel<<<std::max(blocks, 1), 128, 0, st>>>(packed, lo, Xt, uz, ua, xbar_out, L.N, xtbar,
-                                                           L.gather_bar == GATHER_QUADS, ws_ptr<Status>(ws, L.status));
+                                                           ws_ptr<Status>(ws, L.status));
     MLFF_LAUNCH_CHECK("update_bwd");
     return MLFF_OK;
 }

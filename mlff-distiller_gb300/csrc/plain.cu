@@ -207,13 +207,16 @@ __global__ void __launch_bounds__(256) sgemm_kernel(const T* __restrict__ A, con
 template <int MODE, class T>
 static int sgemm(const T* A, const float* B, const float* bias, T* C, T* C2, const T* Z,
                  int64_t M, const int32_t* m_dev, int N, int K, const Status* st, cudaStream_t s) {
-    if constexpr (!is_dual_v<T>) return gemm_nn(MODE, A, B, bias, C, C2, Z, M, m_dev, N, K, st, s);
-    const int64_t tiles = ((M + SG_BM - 1) / SG_BM) * ((N + SG_BN - 1) / SG_BN);
-    const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>(tiles, 152 * 8));
-    ProfScope prof(PK_PLAIN_GEMM, s);
-    sgemm_kernel<MODE, T><<<blocks, 256, 0, s>>>(A, B, bias, C, C2, Z, M, m_dev, N, K, st);
-    MLFF_LAUNCH_CHECK("sgemm");
-    return MLFF_OK;
+    if constexpr (!is_dual_v<T>) {
+        return gemm_nn(MODE, A, B, bias, C, C2, Z, M, m_dev, N, K, st, s);
+    } else {
+        const int64_t tiles = ((M + SG_BM - 1) / SG_BM) * ((N + SG_BN - 1) / SG_BN);
+        const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>(tiles, 152 * 8));
+        ProfScope prof(PK_PLAIN_GEMM, s);
+        sgemm_kernel<MODE, T><<<blocks, 256, 0, s>>>(A, B, bias, C, C2, Z, M, m_dev, N, K, st);
+        MLFF_LAUNCH_CHECK("sgemm");
+        return MLFF_OK;
+    }
 }
 
 // ------------------------------------------------------------- message

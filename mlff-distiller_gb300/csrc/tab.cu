@@ -759,9 +759,9 @@ int launch_fwd(const TabShape& s, const TabArgs& a, cudaStream_t st) {
 template <bool L0, bool PAIRS>
 int launch_bwd(const TabShape& s, const TabArgs& a, float scale, cudaStream_t st) {
     if (s.G == 2) return launch_bwd_t<2, true, L0, PAIRS>(a, scale, st);
-    if (s.smem) return launch_bwd_t<1, true, L0, PAIRS>(a, scale, st);
-    if constexpr (!PAIRS) return launch_bwd_t<1, false, L0, PAIRS>(a, scale, st);
-    else return launch_bwd_t<1, true, L0, PAIRS>(a, scale, st);   // (always staged)
+    if constexpr (!PAIRS)   // (after the tensor-core forward pass tab_shape always stages)
+        if (!s.smem) return launch_bwd_t<1, false, L0, PAIRS>(a, scale, st);
+    return launch_bwd_t<1, true, L0, PAIRS>(a, scale, st);
 }
 
 }  // namespace
