@@ -382,10 +382,12 @@ def training_throughput(sysm, n_structures, steps=5, warmup=2):
     reference's loss defaults: energy weight 1, force weight 100): forward
     and forces on the plain FP32 path, the loss derivatives, the parameter
     gradients of the energy and force terms from the hand-written reverse
-    pass and its forward-mode derivative, gradient clipping and AdamW.
+    pass and its forward-mode derivative (through the filter tables where
+    they serve the weights), gradient clipping and AdamW.
     Timed (CUDA events, after warm-up) on the first n_structures structures
     of the workload, targets = the untrained network's own outputs plus
-    seeded noise (the cost of a step does not depend on the values)."""
+    seeded noise (the values move the cost of a step only through the
+    accuracy class of the weights' filter tables, reported with it)."""
     from mlff_gb300 import _lib
     from mlff_gb300.engine import make_batch
     from mlff_gb300.training import ForceFieldTrainer
@@ -413,8 +415,9 @@ def training_throughput(sysm, n_structures, steps=5, warmup=2):
     med = statistics.median(ms)
     return {"structures": sub.n_mol, "atoms": sub.n_atoms, "steps": steps, "ms_per_step": round(med, 3),
             "atom_steps_per_s": round(sub.n_atoms / (med * 1e-3), 1),
+            "filter_table_class": model.engine().table_class,
             "step": "ForceFieldTrainer.step: energy + force loss (weights 1, 100), second-order parameter "
-                    "gradients on the plain FP32 path, grad-norm clip 1.0, AdamW"}
+                    "gradients through the filter tables (class 2) or the plain FP32 path, grad-norm clip 1.0, AdamW"}
 
 
 def time_replays(step, steps, flush):

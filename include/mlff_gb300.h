@@ -53,7 +53,8 @@ typedef struct CUstream_st *mlff_stream_t; /* same type as cudaStream_t */
  * function of the distance alone, evaluated in FP32 from the piecewise
  * polynomials that mlff_pack_weights builds.  A call whose weights' tables
  * miss the path's accuracy class ends with MLFF_ERR_UNSUPPORTED in the status
- * word; mlff_filter_table_class tells beforehand. */
+ * word; mlff_filter_table_class tells beforehand.  (A call of path 5 for
+ * energies alone reads no table and serves any weights.) */
 #define MLFF_PATH_TABLE 5         /* path 1's forward pass, reverse pass from the tables (class 1 or 2) */
 #define MLFF_PATH_TABLE_FP32 6    /* path 2 from the tables, both passes (class 2) */
 /* a training step: path 2's forward pass bit for bit, reverse pass from the
@@ -366,7 +367,8 @@ int mlff_param_grads_forces(const mlff_dims *dims, const void *packed, const mlf
  * 2 (mlff_filter_table_class; otherwise MLFF_ERR_UNSUPPORTED in the status
  * word).  A filter value is linear in the network's values at the table's
  * 576 nodes, so the filter's weight gradients need the network's reverse
- * pass at those nodes only; everything else is evaluated as in path 6.
+ * pass at those nodes only; the forward pass is path 0's, the other edge
+ * passes read the tables.
  * energy: double [B].  Fixed-order sums: the same bits on every call.
  * Workspace of both: mlff_workspace_size(..., MLFF_PATH_TRAIN_TABLE). */
 int mlff_param_grads_table(const mlff_dims *dims, const void *packed, const mlff_system *sys,

@@ -20,13 +20,7 @@ namespace mlff {
 
 constexpr float PI_F = 3.14159265358979f;
 
-// ------------------------------------------------------------- geometry
-// u = r / (d + 1e-8), d = |r| (:709-715); e = rbf(d) * fc(d) (:718-722) and
-// de/dd for the reverse pass.  Dual: the edge vector's tangent is
-// -(pos_t[b] - pos_t[a]) (positions moved along -G, G = pos_t [N][3],
-// optional; F = -dE/dpos) plus S_m r for a strain direction S_m [B][3][3]
-// (optional; positions and image shifts scale with the cell, so every
-// edge vector r becomes (I + eps S_m) r).
+// ---------------------------------------------------------------- pairs
 // Filter rows by pair of atoms.  The two directed edges of a pair have the
 // same distance, bit for bit, and so the same filter: the passes without
 // parameter gradients evaluate it once, at the edge whose sender has the lower
@@ -58,6 +52,13 @@ __global__ void pl_pair_count_kernel(const int32_t* __restrict__ row_ptr, const 
     }
 }
 
+// ------------------------------------------------------------- geometry
+// u = r / (d + 1e-8), d = |r| (:709-715); e = rbf(d) * fc(d) (:718-722) and
+// de/dd for the reverse pass.  Dual: the edge vector's tangent is
+// -(pos_t[b] - pos_t[a]) (positions moved along -G, G = pos_t [N][3],
+// optional; F = -dE/dpos) plus S_m r for a strain direction S_m [B][3][3]
+// (optional; positions and image shifts scale with the cell, so every
+// edge vector r becomes (I + eps S_m) r).
 template <class T>
 __global__ void pl_geom_kernel(const float4* __restrict__ pos4, const float* __restrict__ pos_t,
                                const double* __restrict__ strain_t,

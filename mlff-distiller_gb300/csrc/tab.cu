@@ -11,7 +11,7 @@
 // functions than the table resolves keep the network kernels).
 //
 // Measured (GB300): a reverse launch on 256 molecules (16,900 atoms, 0.85 M
-// edges) 0.47 ms against 0.72 + 0.07 ms of the tensor-core network kernels;
+// edges) 0.41 ms against 0.72 + 0.07 ms of the tensor-core network kernels;
 // the FP32 path on 64 molecules 11.2 -> 1.2 ms per call.
 #include <algorithm>
 #include <cmath>

@@ -26,8 +26,8 @@ constexpr int64_t TAB_SLICE = (int64_t)TAB_NI * TAB_ROW;    // floats of a slice
 constexpr int64_t TAB_LAYER = TAB_SLICES * TAB_SLICE;       // floats of a layer
 // Accuracy of the table where it is worst (the ends of the intervals),
 // relative 2-norms over all intervals and channels of (filter, derivative).
-// TAB_FP32: as accurate as the FP32 evaluation; TAB_TC: as the split-FP16
-// evaluation (its filter derivative is off by about 1e-5).
+// TAB_TOL_D_FP32: as accurate as the FP32 evaluation; TAB_TOL_D_TC: as the
+// split-FP16 evaluation (its filter derivative is off by about 1e-5).
 constexpr double TAB_TOL_F = 2e-7, TAB_TOL_D_FP32 = 4e-6, TAB_TOL_D_TC = 1.2e-5;
 constexpr int TAB_OK_TC = 1, TAB_OK_FP32 = 2;       // flag values (0: the table is not used)
 

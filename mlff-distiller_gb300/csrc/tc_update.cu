@@ -6,20 +6,21 @@
 // Transposed GEMMs, D[channel][atom] = W[channel][k] X[atom][k]^T: a TMEM
 // lane is an output channel, a column an atom, so the epilogue thread that
 // owns channel c touches channel c of consecutive atoms -- coalesced rows of
-// the [N][4][H] feature arrays.  64-atom tiles (MMA N = 64, so that a
-// 3,000-atom system still spreads over 47 SMs), persistent CTAs of 8 warps,
-// two per SM (one CTA's epilogues overlap the other's weight stream and MMAs):
-// in the epilogues warp w reads TMEM lane quarter w % 4 for atoms
-// 32 (w / 4) .. +31; the B tiles are built one atom row per warp (lane l:
-// channels 4l..4l+3, coalesced 512-byte rows).
+// the [N][4][H] feature arrays.  Tiles of 64 or 32 atoms (MMA N; 32 spread a
+// small system over more SMs), persistent CTAs of 8 warps, two per SM (one
+// CTA's epilogues overlap the other's weight stream and MMAs), or of 16 warps
+// where one 32-atom tile per SM is all there is: in the epilogues warp w reads
+// TMEM lane quarter w % 4 for the atoms of group w / 4; the B tiles are built
+// one atom row per warp (lane l: channels 4l..4l+3, coalesced 512-byte rows).
 //
 // The weights (split-FP16 A-operand tile pairs, 8 KB per 128 x 16 block)
-// stream through a ring of bulk copies (5 slots forward, 2 reverse: what
-// two CTAs per SM leave of shared memory) in the order the MMAs use
-// them: one thread issues the MMAs and commits each slot, another refills
-// the slots (during a GEMM, and ahead of the next GEMM while the epilogue
-// runs).  The forward accumulators are pre-filled with the bias, so every
-// MMA accumulates.  Every wait is bounded (MLFF_ERR_TIMEOUT).
+// stream through a ring of bulk copies in units of one pair (16 warps: two),
+// 6 slots forward, 2 (64 atoms), 8 (32) or 6 (16 warps) in the reverse kernel:
+// what the CTAs per SM leave of shared memory.  One thread per accumulator
+// tile of a GEMM issues its MMAs and commits the slots, another refills them
+// (during a GEMM, and ahead of the next GEMM while the epilogue runs).  The
+// forward accumulators are pre-filled with the bias, so every MMA
+// accumulates.  Every wait is bounded (MLFF_ERR_TIMEOUT).
 #include <cuda_fp16.h>
 #include <mutex>
 #include "common.cuh"
@@ -235,8 +236,9 @@ __device__ __forceinline__ void uwait_mma(UCtl& c, int w, int where) {
 }
 
 // ------------------------------------------------------- forward kernel
-// smem: B tile [s, |v|] (K = 256: 4 K-blocks; hi half then lo half, 64 KB),
-// the H tile (K = 128, 32 KB) aliased into it after GEMM1, the ring (48 KB).
+// smem: B tile [s, |v|] (K = 256: 4 K-blocks; hi half then lo half, 64 KB; for
+// 32 atoms 32 KB in a region of 48, epilogue 2's rows), the H tile (K = 128,
+// half as large) aliased into it after GEMM1, the ring (48 KB; 512 threads: 96).
 // TMEM: D1 = z (cols 0..UN-1), D2 chunk g = (ds, g1, g2)[g] (UN + UN g).
 // UN-atom tiles, UN = 64 or 32 (the autotuner's update tile: small systems
 // spread over more SMs with 32); the ring takes what two CTAs per SM leave.
@@ -522,7 +524,8 @@ int launch_update_fwd_tc(const float* packed, const LayerOffsets& lo, const WsLa
 // abar = dE/d(ds, g1, g2) [atom][3H] -> zbar = (U2^T abar) silu'(uz) ->
 // cb = U1^T zbar = dE/d[s, |v|]; xtbar = (sb + cs, vb + cn v / |v|).
 // smem: abar B tile (K = 384: 6 K-blocks, hi then lo, 96 KB), the zbar tile
-// (K = 128, 32 KB) aliased into it after GEMM3, the ring (16 KB).
+// (K = 128, 32 KB) aliased into it after GEMM3 (both for 64 atoms, half for
+// 32), the ring (16 KB for 64 atoms, 64 KB for 32, 96 KB with 512 threads).
 // TMEM: D3 = zbar pre-activation (cols 0..UN-1), D4 = (cs, cn) (UN + UN g).
 template <int UN, int NT>
 struct UBwd {

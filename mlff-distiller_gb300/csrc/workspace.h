@@ -70,9 +70,10 @@ struct WsLayout {
     size_t toffs, tscan;       // int32 [intervals][segments] offsets of the sort; scan scratch
     size_t tcst;               // int32 [intervals + 1] first partial sum of each interval
     size_t thead;              // float: activations and adjoints of the energy head
-    size_t tadj;               // float [partial sums][18][H]
-    size_t prows, pgeo;        // plain forward pass of the force term: X rows, geometry
-    size_t tnode;              // float [nodes][3H], [nodes][H]
+    size_t tadj;               // float [partial sums][18 (force term: 36)][H]
+    size_t prows;              // float [L + 1][N][4][H] X rows of the gradient passes' value forward pass
+    size_t pgeo;               // float4 [cap] (u, d) of the forward passes by pairs
+    size_t tnode;              // float [2][nodes][3H], [2][nodes][H]
     size_t temb;               // float: partial embedding gradients
     size_t erbf;               // float [cap][RMAX]
     size_t erbf_d;             // float [cap][RMAX]

@@ -9,7 +9,10 @@ path forward, hand-written reverse pass with the weight-gradient
 reductions) and, for a loss on forces, G_i = dL/dF_i (one call of
 ``mlff_param_grads_forces``: the same path in forward mode over the reverse
 pass, which adds sum_i G_i . dF_i/dtheta -- what the reference gets by
-taking forces with create_graph=True and differentiating again).
+taking forces with create_graph=True and differentiating again).  Where the
+filter tables serve the weights, ``mlff_param_grads_table`` and
+``mlff_param_grads_forces_table`` give the same from the plain path's forward
+pass and the tables.
 
 ``ForceFieldLoss`` restates the reference's loss (training/losses.py:15-
 246: energy, force, angular and stress terms with mse / mae / huber
@@ -321,7 +324,8 @@ class ForceFieldTrainer:
     """One optimisation step per call on energies and forces: forward and
     forces on the plain FP32 path, the loss and its derivatives w = dL/dE,
     G = dL/dF (``ForceFieldLoss``), parameter gradients from the CUDA
-    reverse pass and its forward-mode derivative (``param_grads``),
+    reverse pass and its forward-mode derivative (``param_grads``; through
+    the filter tables where they serve the weights),
     gradient clipping and AdamW."""
 
     def __init__(self, model, loss: Optional[ForceFieldLoss] = None, lr: float = 1e-3, weight_decay: float = 1e-5,
