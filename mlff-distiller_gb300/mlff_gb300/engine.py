@@ -197,6 +197,16 @@ class Engine:
         ``to_host``: the batch's Z and positions may live in host memory and
         the results are returned in host memory."""
         path = self._checked_path(path)
+        try:
+            return self._energy_forces(batch, path, forces, virial, atom_energy, check, graph, to_host)
+        except torch.OutOfMemoryError:
+            if path != _lib.PATH_TABLE_FP32:
+                raise
+        # the tables' edge records take 100 bytes per edge slot (10 million atoms: 329 against 265 GB)
+        return self._energy_forces(batch, _lib.PATH_TUNED_FP32, forces, virial, atom_energy, check, graph, to_host)
+
+    def _energy_forces(self, batch: Batch, path: int, forces: bool, virial: bool, atom_energy: bool, check: bool,
+                       graph: Optional[bool], to_host: bool):
         use_graph = self.use_graphs if graph is None else graph
         if use_graph and check and not torch.cuda.is_current_stream_capturing():
             res = self._graph_call(batch, path, forces, virial, atom_energy, to_host)

@@ -291,7 +291,9 @@ class VelocityVerletGPU:
     def _select_path(self):
         """Weights packed since the last run may need another path than the
         one chosen for the earlier weights; the edges are the same."""
-        path = self.engine._checked_path(self.path)
+        self._set_path(self.engine._checked_path(self.path))
+
+    def _set_path(self, path: int):
         if path != self.path:
             cap = self.engine.edge_capacity
             cap[path] = max(cap.get(path, 0), cap.get(self.path, 0))
@@ -310,11 +312,18 @@ class VelocityVerletGPU:
         if not self._forces_valid:
             self.compute_forces()
         cap = self._capacity()
+        try:
+            self.engine.workspace_for(self.N, self.B, cap, self.path)
+        except torch.OutOfMemoryError:   # (as Engine.energy_forces)
+            if self.path != _lib.PATH_TABLE_FP32:
+                raise
+            self._set_path(_lib.PATH_TUNED_FP32)
+            cap = self._capacity()
+            self.engine.workspace_for(self.N, self.B, cap, self.path)
         # the library reads the float32 positions of its own buffer; the
         # batch descriptor only carries Z, mol_ptr, box and pbc
         self._pos32 = self.pos.to(torch.float32)
         self._batch_sys = Batch(self.Z, self._pos32, self.mol_ptr, self.box, self.pbc).system()
-        self.engine.workspace_for(self.N, self.B, cap, self.path)
         epot = torch.zeros(n_steps, self.B, dtype=torch.float64, device=self.dev) if record else None
         ekin = torch.zeros_like(epot) if record else None
         done = 0

@@ -84,3 +84,27 @@ def test_forward_only_call_of_a_large_system(weights_bias):
     m(torch.tensor(s.Z, device="cuda"), pos, cell=torch.tensor(np.diag(s.box[0])), pbc=torch.tensor([True] * 3))
     eng = m.engine()
     assert eng.workspace.numel() == sizes(24_000, eng.capacity(24_000, ALONE), (ALONE,))[0] < 3e9
+
+
+def test_fp32_call_whose_records_do_not_fit(engine):
+    """The table path's workspace is larger than the network kernels'; where
+    only theirs fits they run, other paths' shortage is the caller's."""
+    del engine.energy_forces
+    engine.use_graphs, engine.short = False, True
+    table = _lib.PATH_TABLE_FP32
+    calls = []
+
+    def eager(b, path, *args):
+        calls.append(path)
+        if engine.short and path != NETWORK:
+            raise torch.OutOfMemoryError("no room")
+        return path
+
+    engine._eager_call = eager
+    assert engine.energy_forces(batch(5), table) == NETWORK and calls == [table, NETWORK]
+    with pytest.raises(torch.OutOfMemoryError):
+        engine.energy_forces(batch(5), _lib.PATH_TABLE)
+    engine.short = False
+    assert engine.energy_forces(batch(5), table) == table
+    network, records = sizes(100_000, 6_400_000, (NETWORK, table))
+    assert 0 < records - network < 101 * 6_400_000
