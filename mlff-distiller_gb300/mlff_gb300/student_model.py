@@ -509,8 +509,7 @@ class StudentForceField(nn.Module):
             subs, kids = self._weight_slots[4]
             if [k for sub in subs for k in sub.values()] != kids:
                 self._weight_slots = None
-        return tuple((t.data_ptr(), t._version) if t is not None else None
-                     for t in (d[n] for d, n in self._slots()[1]))
+        return [(t.data_ptr(), t._version) if (t := d[n]) is not None else None for d, n in self._slots()[1]]
 
     def engine(self) -> Engine:
         dev = self.embedding.weight.device
